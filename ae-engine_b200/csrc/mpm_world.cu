@@ -1731,13 +1731,16 @@ __device__ __forceinline__ WarpStage<T> warp_stage(unsigned char* smem, int warp
 // guarantees.  Every lane of the warp calls it; has = false lanes contribute nothing.  x is the
 // position, mv = m v, A = m C - k tau.  The cell key is the global index of the stencil's base
 // node, unique across scenes.  kMixed: lanes may belong to different scenes (each run looks its
-// scene up from its base node's block); otherwise every lane belongs to scene sc.
+// scene up from its base node's block); otherwise every lane belongs to scene sc.  write_keys: the
+// next substep sorts, so each particle's key goes to its slot and, with dense grouping, each group
+// of equal keys is counted in its cell with one atomic (the grouping is needed here anyway).
 // runs of at most this many particles are summed one node per lane; longer ones by the column lanes
 constexpr int kShortRun = 6;
 
 template <class T, bool kMixed>
 __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const SceneDev<T>& sc, bool has, const T* x,
-                                                 T m, const T* mv, const T* A, const WarpStage<T>& st) {
+                                                 T m, const T* mv, const T* A, const WarpStage<T>& st, uint32_t slot,
+                                                 int write_keys) {
   using V4 = typename V4T<T>::type;
   const int lane = threadIdx.x & 31;
   int g[3] = {0, 0, 0};
@@ -1760,6 +1763,10 @@ __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const Sce
   // within a group in lane order; pos is this particle's slot in that grouped order
   const uint32_t peers = __match_any_sync(0xffffffffu, key);
   const int leader = __ffs(peers) - 1;
+  if (write_keys && has) {
+    w.keys[slot] = key;
+    if (w.bins && lane == leader) atomicAdd(w.bins + key, uint32_t(__popc(peers)));
+  }
   const uint32_t lead_cnt = lane == leader ? uint32_t(__popc(peers)) : 0u;
   uint32_t incl = lead_cnt;
 #pragma unroll
@@ -1995,11 +2002,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
     w.out[4][j] = mk4(o.v[0], o.v[1], o.v[2], o.C[0]);
     w.out[5][j] = mk4(o.C[1], o.C[2], o.C[3], o.C[4]);
     w.out[6][j] = mk4(o.C[5], o.C[6], o.C[7], o.C[8]);
-    if (write_keys) w.keys[j] = cell_key(sc, AE_MPM_MODE_PHYSICS, o.x[0], o.x[1], o.x[2]);
     err = o.err;
     cl = o.clamped;
     need = o.needs_clamp;
-    has = !need;
+    has = !need;  // the particles that need the clamp are scattered (and keyed) by its kernel
     m = a0.w;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -2008,7 +2014,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
     }
 #pragma unroll
     for (int k = 0; k < 9; ++k) A[k] = o.C[k];
-  } else if (j < ch.w && write_keys) {
+  } else if (j < ch.w && write_keys && !w.bins) {
     w.keys[j] = sc.dead_key;
   }
   const uint32_t e = __reduce_or_sync(0xffffffffu, err);
@@ -2023,14 +2029,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
   qbase = __shfl_sync(0xffffffffu, qbase, 0);
   if (need) w.clamp_queue[qbase + __popc(qmask & ((1u << lane) - 1u))] = make_uint2(uint32_t(j), uint32_t(ch.x));
   __syncwarp();  // every lane has read its F, J and material: the scatter may reuse the region
-  p2g_warp_scatter<T, false>(w, sc, has, xs, m, mv, A, st);
+  p2g_warp_scatter<T, false>(w, sc, has, xs, m, mv, A, st, uint32_t(j), write_keys);
 }
 
 // The snow return mapping of snow_clamp_kernel for the particles the fused kernel queued, each
 // then scattered into the next substep's accumulator with its final A.  A warp takes 32
 // consecutive queue entries (possibly of several scenes of a world).
 template <class T>
-__global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> w) {
+__global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> w, int write_keys) {
   using V4 = typename V4T<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
@@ -2083,7 +2089,7 @@ __global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> 
       mv[0] = m * a4.x, mv[1] = m * a4.y, mv[2] = m * a4.z;
     }
     __syncwarp();  // prefetched data consumed: the scatter may reuse the region
-    p2g_warp_scatter<T, true>(w, sc, valid, xs, m, mv, A, st);
+    p2g_warp_scatter<T, true>(w, sc, valid, xs, m, mv, A, st, q.x, write_keys);
   }
 }
 
@@ -2205,17 +2211,163 @@ __global__ void det_reset_kernel(const uint32_t* __restrict__ seg_start, const u
 // ============================================================================================
 // keys, pack/unpack, totals, grid export
 // ============================================================================================
+// Cell keys of the current positions; with dense grouping also the live particles per cell (one
+// atomic per cell and warp), and no keys for the dead slots, which that grouping never reads.
 template <class T, int MODE>
 __global__ void init_keys_kernel(WorldDev<T> w) {
   const int4 ch = cta_chunk(w);
   const SceneDev<T>& sc = w.scenes[ch.x];
   const int j = ch.y + threadIdx.x;
-  if (j < ch.z) {
+  const bool live = j < ch.z;
+  uint32_t key = sc.dead_key;
+  if (live) {
     auto a0 = ld4(w.in[0] + j);
-    w.keys[j] = cell_key(sc, MODE, a0.x, a0.y, a0.z);
-  } else if (j < ch.w) {
-    w.keys[j] = sc.dead_key;
+    key = cell_key(sc, MODE, a0.x, a0.y, a0.z);
   }
+  if (!w.bins) {
+    if (j < ch.w) w.keys[j] = key;
+    return;
+  }
+  const uint32_t peers = __match_any_sync(0xffffffffu, live ? key : 0xffffffffu);
+  if (live) {
+    w.keys[j] = key;
+    if (int(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(w.bins + key, uint32_t(__popc(peers)));
+  }
+}
+
+// ============================================================================================
+// dense grouping: particles in ascending cell order through one counter per grid node
+// ============================================================================================
+// The kernels that write the keys count the live particles of every cell (w.bins).  bin_scan turns
+// the counts into offsets and bin_scatter claims a place per particle with them: two launches and
+// 12 bytes per node + 12 per particle, where the radix sort takes 3 launches and 20 bytes per key
+// for each 8 bits of key.  Equal keys land in no defined order, so only the modes whose results do
+// not depend on it (anything but deterministic) use it.  Sorted places of a scene are its slot
+// range: the dead key's cell holds the off-grid particles of the reference modes first and then,
+// without entries, the scene's empty slots.
+//
+// One CTA scans 4096 nodes (64 blocks) and zeroes the counts it read, so the array is clean for
+// the next count; offsets are written only where a count is not zero.  The CTA that finishes last
+// scans the segment totals (no CTA waits for another).
+constexpr int kBinSeg = 4096;
+constexpr int kBinThreads = 256;
+
+__device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  return x;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, uint64_t nodes,
+                                                               const uint32_t* __restrict__ dead_blk,
+                                                               uint32_t* seg_total, uint32_t* done) {
+  __shared__ uint32_t wsum[kBinThreads / 32];
+  __shared__ uint32_t s_last, s_carry;
+  const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
+  const uint64_t base = uint64_t(blockIdx.x) * kBinSeg + uint64_t(wi) * 512u;
+  uint4* bins4 = reinterpret_cast<uint4*>(w.bins);
+  uint4* off4 = reinterpret_cast<uint4*>(w.bin_off);
+  uint4 c[4];
+  uint32_t pad[4], any[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const uint64_t i = base + r * 128 + lane * 4;
+    c[r] = make_uint4(0u, 0u, 0u, 0u);
+    pad[r] = 0u;
+    if (i < nodes) {
+      c[r] = bins4[i >> 2];
+      if ((i & 63u) == 0 && dead_blk[i >> 6]) {  // the scene's empty slots follow the dead key's particles
+        const SceneDev<T>& sc = w.scenes[w.blk_scene[i >> 6]];
+        pad[r] = sc.p_cap - sc.p_count;
+      }
+    }
+  }
+  uint32_t ex[4], run = 0;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    any[r] = c[r].x | c[r].y | c[r].z | c[r].w;
+    const uint32_t t = c[r].x + c[r].y + c[r].z + c[r].w + pad[r];
+    const uint32_t incl = warp_scan_incl(t, lane);
+    ex[r] = run + incl - t;
+    run += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) wsum[wi] = run;
+  __syncthreads();
+  uint32_t off = 0, total = 0;
+#pragma unroll
+  for (int k = 0; k < kBinThreads / 32; ++k) {
+    const uint32_t v = wsum[k];
+    if (k < wi) off += v;
+    total += v;
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    if (!any[r]) continue;
+    const uint64_t q = (base + r * 128 + lane * 4) >> 2;
+    uint4 o;
+    o.x = off + ex[r];
+    o.y = o.x + c[r].x + pad[r];
+    o.z = o.y + c[r].y;
+    o.w = o.z + c[r].z;
+    off4[q] = o;
+    bins4[q] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (tid == 0) {
+    seg_total[blockIdx.x] = total;
+    __threadfence();
+    s_last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    s_carry = 0u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (uint32_t s0 = 0; s0 < gridDim.x; s0 += kBinThreads * 4) {
+    uint32_t v[4], t = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t i = s0 + tid * 4 + k;
+      v[k] = i < gridDim.x ? __ldcg(seg_total + i) : 0u;
+      t += v[k];
+    }
+    const uint32_t incl = warp_scan_incl(t, lane);
+    __syncthreads();  // the previous round's wsum and carry have been read
+    if (lane == 31) wsum[wi] = incl;
+    __syncthreads();
+    uint32_t o = s_carry + incl - t, sum = 0;
+#pragma unroll
+    for (int k = 0; k < kBinThreads / 32; ++k) {
+      if (k < wi) o += wsum[k];
+      sum += wsum[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t i = s0 + tid * 4 + k;
+      if (i < gridDim.x) w.seg_off[i] = o;
+      o += v[k];
+    }
+    __syncthreads();
+    if (tid == 0) s_carry += sum;
+  }
+  if (tid == 0) *done = 0u;
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) bin_scatter_kernel(WorldDev<T> w, uint32_t* __restrict__ perm,
+                                                          uint32_t n_slots) {
+  const int4 ch = cta_chunk(w);
+  const int j = ch.y + threadIdx.x, lane = threadIdx.x & 31;
+  const bool live = j < ch.z;
+  const uint32_t key = live ? w.keys[j] : 0xffffffffu;
+  const uint32_t peers = __match_any_sync(0xffffffffu, key);
+  const int leader = __ffs(peers) - 1;
+  uint32_t pos = 0;
+  if (live && lane == leader) pos = atomicAdd(w.bin_off + key, uint32_t(__popc(peers))) + w.seg_off[key / kBinSeg];
+  pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+  if (live && pos < n_slots) perm[pos] = uint32_t(j);
 }
 
 // staging layout (elements of T): pos 3n | vel 3n | F 9n | J n | C 9n | mass n | then u16 mat n
@@ -2544,7 +2696,21 @@ class World final : public WorldBase {
     AE_TRY(cudaMemcpy(d_ptrA_, bufA_, sizeof(V4*) * 7, cudaMemcpyHostToDevice));
     AE_TRY(cudaMemcpy(d_ptrB_, bufB_, sizeof(V4*) * 7, cudaMemcpyHostToDevice));
     AE_TRY(dmalloc(&keys_, sizeof(uint32_t) * pc));
-    AE_TRY(sort_scratch_alloc(sort_, pc, alloc_ ? &World::sort_alloc : nullptr, alloc_));
+    // Dense grouping reads every node's counter; the radix sort moves 20 bytes per key and pass.
+    // The grid decides: up to 16 nodes per particle slot (or 8 M nodes, 5 us of scan) the dense
+    // grouping wins, a huge grid with few particles in it keeps the radix sort.
+    dense_sort_ = !opts_.deterministic && blk * 64 <= 16 * cap + (uint64_t(8) << 20);
+    if (dense_sort_) {
+      n_segs_ = uint32_t((blk * 64 + kBinSeg - 1) / kBinSeg);
+      AE_TRY(dmalloc(&bins_, sizeof(uint32_t) * blk * 64));
+      AE_TRY(cudaMemset(bins_, 0, sizeof(uint32_t) * blk * 64));
+      AE_TRY(dmalloc(&bin_off_, sizeof(uint32_t) * blk * 64));
+      AE_TRY(dmalloc(&seg_, sizeof(uint32_t) * 2 * n_segs_));
+      AE_TRY(dmalloc(&bin_perm_, sizeof(uint32_t) * pc));
+      AE_TRY(cudaMemset(bin_perm_, 0, sizeof(uint32_t) * pc));
+    } else {
+      AE_TRY(sort_scratch_alloc(sort_, pc, alloc_ ? &World::sort_alloc : nullptr, alloc_));
+    }
     // grid
     const uint64_t nodes = blk * 64;
     AE_TRY(dmalloc(&acc_, sizeof(V4) * nodes));
@@ -2917,35 +3083,25 @@ class World final : public WorldBase {
     int rc = prepare();
     if (rc) return rc;
     if (n == 0) return AE_MPM_OK;
+    if ((rc = settle_order())) return rc;
     if ((rc = sync_scatter())) return rc;
-    if (keys_stale_) {
-      WorldDev<T> w = dev(false);
-      launch_init_keys(w);
-      keys_stale_ = false;
-      keys_fresh_ = true;
-    }
-    const int interval = opts_.deterministic ? 1 : opts_.sort_interval;
-    const uint64_t period = (interval % 2 == 0) ? uint64_t(interval) : uint64_t(2 * interval);
+    const uint32_t interval = sort_interval();
+    const uint32_t period = (interval % 2 == 0) ? interval : 2 * interval;
     uint32_t left = n;
-    if (opts_.use_graph) {
-      while (left > 0 && substep_ % period != 0) {
+    while (left > 0) {
+      if (opts_.use_graph && phase_ == 0 && left >= period && n_chunks_ > 0) {
+        if (!sorted_) sort_particles();
+        rc = ensure_graph(period);
+        if (rc) return rc;
+        Graph& g = graphs_[substep_ & 1];
+        AE_TRY(cudaGraphLaunch(g.exec, stream_));
+        launches_ += g.launches;
+        substep_ += period;
+        left -= period;
+      } else {
         substep_eager();
         --left;
       }
-      if (left >= period) {
-        rc = ensure_graph(period);
-        if (rc) return rc;
-        while (left >= period) {
-          AE_TRY(cudaGraphLaunch(graph_, stream_));
-          launches_ += graph_launches_;
-          substep_ += period;
-          left -= uint32_t(period);
-        }
-      }
-    }
-    while (left > 0) {
-      substep_eager();
-      --left;
     }
     AE_TRY(cudaGetLastError());
     return AE_MPM_OK;
@@ -3070,10 +3226,7 @@ class World final : public WorldBase {
   }
   cudaStream_t stream() const override { return stream_; }
   int set_stream_priority(int priority) override {
-    if (graph_) {
-      cudaGraphExecDestroy(graph_);
-      graph_ = nullptr;
-    }
+    drop_graphs();
     AE_TRY(cudaStreamSynchronize(stream_));
     cudaStream_t s = nullptr;
     AE_TRY(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority));
@@ -3083,8 +3236,7 @@ class World final : public WorldBase {
   }
   ae_mpm_exec_opts& opts() override { return opts_; }
   void invalidate_graph() override {
-    if (graph_) cudaGraphExecDestroy(graph_);
-    graph_ = nullptr;
+    drop_graphs();
     chunks_dirty_ = true;
   }
   uint64_t device_bytes() const override { return device_bytes_; }
@@ -3199,13 +3351,7 @@ class World final : public WorldBase {
     int rc = prepare();
     if (rc) return rc;
     if (n == 0 || n_chunks_ == 0) return AE_MPM_OK;
-    if ((rc = sync_scatter())) return rc;
-    if (keys_stale_) {
-      WorldDev<T> w = dev(false);
-      launch_init_keys(w);
-      keys_stale_ = false;
-      keys_fresh_ = true;
-    }
+    if ((rc = settle_order()) || (rc = sync_scatter())) return rc;
     // all substeps are queued before the one wait, so that (past the first) the stream is never
     // idle waiting for the host and the events measure device time, not launch latency
     // per substep: start, after the sort, after P2G, after the grid update, end, and after the
@@ -3314,10 +3460,7 @@ class World final : public WorldBase {
       }
       if (n_chunks_ > 0)
         AE_TRY(cudaMemcpyAsync(d_chunks_, h_chunks_.data(), sizeof(int4) * n_chunks_, cudaMemcpyHostToDevice, stream_));
-      if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-      }
+      drop_graphs();
       chunks_dirty_ = false;
     } else if (any_count_dirty_) {
       // particle counts changed, the chunk layout (by capacity) did not: rewrite those scenes'
@@ -3337,10 +3480,7 @@ class World final : public WorldBase {
         count_dirty_[s] = 0;
       }
       any_count_dirty_ = false;
-      if (graph_) {  // a one-scene world's graph carries the count in its launch parameters
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-      }
+      drop_graphs();  // a one-scene world's graphs carry the count in their launch parameters
     }
     int rc = sync_tables();
     if (rc) return rc;
@@ -3389,6 +3529,9 @@ class World final : public WorldBase {
     }
     w.perm = sorted ? perm_ : nullptr;
     w.keys = keys_;
+    w.bins = bins_;
+    w.bin_off = bin_off_;
+    w.seg_off = seg_ ? seg_ + n_segs_ : nullptr;
     w.acc = acc_;
     w.vel = vel_;
     w.blk_flag = blk_flag_;
@@ -3568,84 +3711,120 @@ class World final : public WorldBase {
     launches_ += 2;
     mark(5);  // the fused kernel alone ends here
     if (has_snow_) {
-      snow_clamp_scatter_kernel<T><<<sms * 8, 128, fused_smem(128), stream_>>>(wf);
+      snow_clamp_scatter_kernel<T><<<sms * 8, 128, fused_smem(128), stream_>>>(wf, write_keys ? 1 : 0);
       ++launches_;
     }
     mark(4);
   }
 
+  uint32_t sort_interval() const { return opts_.deterministic ? 1u : uint32_t(opts_.sort_interval); }
+
+  // The particles changed since their order was established (upload, scene change, ...): the next
+  // substep sorts, and the sort interval counts from there, so a run never starts on particles in
+  // the caller's order.
+  int settle_order() {
+    if (phase_ >= sort_interval()) phase_ = 0;  // the interval was shortened
+    if (!keys_stale_) return AE_MPM_OK;
+    // cells counted for the dropped state
+    if (dense_sort_ && keys_fresh_) AE_TRY(cudaMemsetAsync(bins_, 0, sizeof(uint32_t) * 64 * total_blocks_, stream_));
+    keys_stale_ = keys_fresh_ = sorted_ = false;
+    phase_ = 0;
+    return AE_MPM_OK;
+  }
+
+  // perm_: sorted position -> storage slot of the current particle state
+  void sort_particles() {
+    if (!keys_fresh_) {
+      WorldDev<T> wk = dev(false);
+      launch_init_keys(wk);
+    }
+    if (dense_sort_) {
+      WorldDev<T> w = dev(false);
+      bin_scan_kernel<T><<<n_segs_, kBinThreads, 0, stream_>>>(w, total_blocks_ * 64, dead_blk_, seg_, counters_ + 5);
+      bin_scatter_kernel<T><<<n_chunks_, chunk_threads_, 0, stream_>>>(w, bin_perm_, uint32_t(total_cap_));
+      perm_ = bin_perm_;
+      launches_ += 2;
+    } else {
+      launches_ += radix_sort_pairs(keys_, total_cap_, key_bits_, sort_, stream_, &sorted_keys_, &perm_);
+    }
+    keys_fresh_ = false;  // the counts (or the keys) are used up
+    sorted_ = true;
+  }
+
   void substep_eager() {
-    const int interval = opts_.deterministic ? 1 : opts_.sort_interval;
-    const bool do_sort = (substep_ % uint64_t(interval)) == 0;
-    // G2P writes the cell keys only for a substep that sorts next; a sort whose keys were not
-    // written by the G2P just before it (sort interval changed, first substep) computes them first
-    const bool next_sorts = ((substep_ + 1) % uint64_t(interval)) == 0;
+    // the keys of the next sort are written by the G2P just before it; a sort without them (first
+    // substep, changed interval) computes them first.  Only the fused G2P counts cells too.
+    const uint32_t next = phase_ + 1 >= sort_interval() ? 0u : phase_ + 1;
+    const bool write_keys = next == 0 && (!dense_sort_ || fused());
     if (n_chunks_ > 0) {
       mark(0);
-      if (do_sort) {
-        if (!keys_fresh_) {
-          WorldDev<T> wk = dev(false);
-          launch_init_keys(wk);
-        }
-        // keys of a small grid in a mode whose results do not depend on the order of equal keys:
-        // one counting pass instead of two radix passes
-        if (!opts_.deterministic && key_bits_ <= kCountingSortBits && total_cap_ > uint64_t(kSmallSortMax))
-          launches_ += counting_sort_pairs(keys_, total_cap_, key_bits_, sort_, stream_, &sorted_keys_, &perm_);
-        else
-          launches_ += radix_sort_pairs(keys_, total_cap_, key_bits_, sort_, stream_, &sorted_keys_, &perm_);
-      }
+      if (phase_ == 0 && !sorted_) sort_particles();
       mark(1);
-      WorldDev<T> w = dev(do_sort);
+      WorldDev<T> w = dev(sorted_);
       switch (mode_) {
         case AE_MPM_MODE_PHYSICS:
           if (fused())
-            substep_fused(w, next_sorts);
+            substep_fused(w, write_keys);
           else
-            substep_mode<AE_MPM_MODE_PHYSICS>(w, next_sorts);
+            substep_mode<AE_MPM_MODE_PHYSICS>(w, write_keys);
           break;
-        case AE_MPM_MODE_REFERENCE: substep_mode<AE_MPM_MODE_REFERENCE>(w, next_sorts); break;
-        default: substep_mode<AE_MPM_MODE_VELOCITY_ONLY>(w, next_sorts); break;
+        case AE_MPM_MODE_REFERENCE: substep_mode<AE_MPM_MODE_REFERENCE>(w, write_keys); break;
+        default: substep_mode<AE_MPM_MODE_VELOCITY_ONLY>(w, write_keys); break;
       }
-      keys_fresh_ = next_sorts || opts_.deterministic;
+      keys_fresh_ = write_keys;
+      sorted_ = false;
       a_in_ = !a_in_;
     }
+    phase_ = next;
     ++substep_;
   }
 
-  int ensure_graph(uint64_t period) {
-    if (graph_ && graph_period_ == period && graph_variant_ == opts_.p2g_variant) return AE_MPM_OK;
-    if (graph_) {
-      cudaGraphExecDestroy(graph_);
-      graph_ = nullptr;
+  // A graph holds one period of substeps from sorted particles to sorted particles: lcm(2, sort
+  // interval), since buffers and touched lists alternate.  A period may start on either parity (the
+  // interval counts from the last upload), so there is one graph for each.
+  int ensure_graph(uint32_t period) {
+    Graph& gr = graphs_[substep_ & 1];
+    if (gr.exec && gr.period == period && gr.variant == opts_.p2g_variant && gr.a_in == a_in_) return AE_MPM_OK;
+    if (gr.exec) {
+      cudaGraphExecDestroy(gr.exec);
+      gr.exec = nullptr;
     }
     const bool a_in0 = a_in_;
     const uint64_t sub0 = substep_, l0 = launches_;
     AE_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    for (uint64_t k = 0; k < period; ++k) substep_eager();
+    for (uint32_t k = 0; k < period; ++k) substep_eager();
+    if (!sorted_) sort_particles();
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     a_in_ = a_in0;
     substep_ = sub0;
-    graph_launches_ = launches_ - l0;
+    gr.launches = launches_ - l0;
     launches_ = l0;
     if (e != cudaSuccess) {
       err = std::string("stream capture failed: ") + cudaGetErrorString(e);
       return AE_MPM_ECUDA;
     }
-    e = cudaGraphInstantiate(&graph_, g, 0);
+    e = cudaGraphInstantiate(&gr.exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
       err = std::string("graph instantiation failed: ") + cudaGetErrorString(e);
-      graph_ = nullptr;
+      gr.exec = nullptr;
       return AE_MPM_ECUDA;
     }
-    graph_period_ = period;
-    graph_variant_ = opts_.p2g_variant;
+    gr.period = period;
+    gr.variant = opts_.p2g_variant;
+    gr.a_in = a_in0;
     return AE_MPM_OK;
+  }
+  void drop_graphs() {
+    for (Graph& g : graphs_) {
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+      g.exec = nullptr;
+    }
   }
 
   void release() {
-    if (graph_) cudaGraphExecDestroy(graph_);
+    drop_graphs();
     if (stream_) cudaStreamSynchronize(stream_);
     if (xfer_ev_) cudaEventDestroy(xfer_ev_);
     for (int k = 0; k < 7; ++k) {
@@ -3657,6 +3836,10 @@ class World final : public WorldBase {
     dfree(d_ptrB_);
     dfree(keys_);
     sort_scratch_free(sort_, alloc_ ? &World::sort_free : nullptr, alloc_);
+    dfree(bins_);
+    dfree(bin_off_);
+    dfree(seg_);
+    dfree(bin_perm_);
     dfree(acc_);
     dfree(vel_);
     dfree(blk_flag_);
@@ -3702,6 +3885,9 @@ class World final : public WorldBase {
   bool a_in_ = true;
   uint32_t* keys_ = nullptr;
   SortScratch sort_;
+  bool dense_sort_ = false;  // particles are grouped by counting (bins_), not by the radix sort
+  uint32_t *bins_ = nullptr, *bin_off_ = nullptr, *seg_ = nullptr, *bin_perm_ = nullptr;
+  uint32_t n_segs_ = 0;
   const uint32_t* perm_ = nullptr;
   const uint32_t* sorted_keys_ = nullptr;
   V4* acc_ = nullptr;
@@ -3717,9 +3903,14 @@ class World final : public WorldBase {
   size_t stage_bytes_ = 0;
   double* partial_ = nullptr;
   cudaStream_t stream_ = nullptr;
-  cudaGraphExec_t graph_ = nullptr;
-  uint64_t graph_period_ = 0, graph_launches_ = 0;
-  int graph_variant_ = -1;
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    uint32_t period = 0;
+    uint64_t launches = 0;
+    int variant = -1;
+    bool a_in = true;
+  };
+  Graph graphs_[2];  // by the parity of the period's first substep
   bool lanes_smem_set_ = false, fused_smem_set_ = false, ref_lanes_smem_set_ = false;
   bool scatter_pending_ = false;  // the accumulator holds the P2G of the current particle state
   bool scatter_invalid_ = false;  // the particles changed since that scatter
@@ -3731,7 +3922,9 @@ class World final : public WorldBase {
   bool keys_stale_ = true, chunks_dirty_ = true, scenes_dirty_ = true, mats_dirty_ = false;
   size_t scene_lo_ = 0, scene_hi_ = SIZE_MAX;  // dirty range of the scene table (all of it at first)
   size_t mat_lo_ = SIZE_MAX, mat_hi_ = 0;       // dirty range of the material table
-  bool keys_fresh_ = false;  // keys_ hold the cell keys of the current positions
+  bool keys_fresh_ = false;  // keys_ (and the cell counts) are those of the current positions
+  bool sorted_ = false;      // perm_ orders the current particle state
+  uint32_t phase_ = 0;       // substeps since the last sort was due
 };
 
 WorldBase* make_world(const ae_mpm_scene_desc* scenes, uint32_t n_scenes, const ae_mpm_exec_opts& opts, std::string& why,

@@ -64,6 +64,11 @@ struct WorldDev {
   V4* out[7];
   const uint32_t* perm;  // sorted position -> storage slot; nullptr = identity
   uint32_t* keys;        // keys for the next sort, written by G2P in the new slot order
+  // dense grouping (bin_scan_kernel): live particles per cell of the next sort, the offset of each
+  // cell within its scan segment, and each segment's offset; bins is null when the world radix-sorts
+  uint32_t* bins;
+  uint32_t* bin_off;
+  uint32_t* seg_off;
   V4* acc;
   V4* vel;
   uint32_t* blk_flag;

@@ -1,0 +1,97 @@
+"""GPU tests of the particle grouping a non-deterministic world does before its substeps: dense
+counting per grid node, the radix sort where the grid is huge for its particles.
+
+Tolerances: trajectories that differ only in the order of atomic sums agree to 1e-6 of the largest
+coordinate (a few tens of substeps); the reference modes against the f32 oracle to 2e-5.
+"""
+import numpy as np
+import pytest
+
+import ae_mpm as M
+import ae_mpm_scenes as S
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.abs(a.astype(np.float64) - b).max() / np.abs(b).max())
+
+
+@pytest.mark.parametrize("interval,threads,graph", [(1, 128, 1), (3, 256, 1), (16, 128, 1), (5, 256, 0)])
+def test_uneven_scenes_with_empty_slots_match_scenes_alone(ctx, interval, threads, graph):
+    # counts below, at and far below the capacity, an empty scene, one-block grids next to large
+    # ones: every scene's sorted places must be its own slot range
+    pairs = [S.tiny_scene(n, g, mat, seed=0xB0 + n, v=(0.4, -0.3, 0.2)) for n, g, mat in
+             ((1, 4, S.water()), (1000, 16, S.jelly()), (2, 8, S.jelly()), (4097, 36, S.snow()), (33, 7, S.water()),
+              (6001, 64, S.jelly()))]
+    caps = (7, 1000, 300, 5000, 257, 6001)
+    scenes = []
+    for (sc, _), cap in zip(pairs, caps):
+        sc.wall_margin = 1
+        sc.max_particles = cap
+        scenes.append(sc)
+    opts = dict(sort_interval=interval, block_threads=threads, use_graph=graph)
+    w = M.World(ctx, scenes, M.exec_opts(**opts))
+    empty = 2
+    for i, (_, p) in enumerate(pairs):
+        if i != empty:
+            w.upload(i, p)
+    for k in (7, 34):  # odd first run: later periods start on the other parity
+        w.step(k)
+    w.upload(3, pairs[3][1])  # one scene restarts: the order starts anew for the whole world
+    w.step(10)
+    assert w.sync(raise_on_error=False) in (M.OK, M.EDOMAIN)
+    for i, (sc, p) in enumerate(pairs):
+        if i == empty:
+            continue
+        alone = M.World(ctx, [sc], M.exec_opts(sort_interval=1, use_graph=0))
+        alone.upload(0, p)
+        alone.step(10 if i == 3 else 51)
+        alone.sync(raise_on_error=False)
+        a, b = w.download(i, p.n), alone.download(0, p.n)
+        assert rel(a.pos, b.pos) <= 1e-6, i
+        assert np.array_equal(a.mass, b.mass), i
+        alone.close()
+    w.close()
+
+
+def test_huge_grid_with_few_particles_matches_small_grid_order(ctx):
+    # 256^3 nodes for 2 000 particles: the radix sort is kept; held to the FP64 oracle
+    sc, p = S.tiny_scene(2000, 256, S.snow(), v=(0.5, 0.0, -0.5), box=(0.45, 0.48))
+    ref = p.astype(np.float64)
+    O.run(sc, ref, 20)
+    for interval in (1, 4):
+        w = M.World(ctx, [sc], M.exec_opts(sort_interval=interval))
+        w.upload(0, p)
+        w.step(20)
+        w.sync()
+        assert rel(w.download(0, p.n).pos, ref.pos) <= 1e-5, interval
+        w.close()
+
+
+@pytest.mark.parametrize("n", [33, 5000, 70001])
+def test_off_grid_particles_of_the_reference_modes_match_the_oracle(ctx, n):
+    # a tenth of the particles lies beyond the grid's upper faces and shares the dead key with the
+    # world's empty slots (the capacity is the power of two above n)
+    rng = np.random.default_rng(n)
+    g, dx = 24, 0.5
+    p = M.Particles.empty(n)
+    p.pos[:] = (0.5 + rng.random((n, 3)) * (g - 4)) * dx
+    out = rng.random(n) < 0.1
+    p.pos[out, rng.integers(0, 3)] += g * dx
+    p.vel[:] = rng.normal(0, 0.3, (n, 3))
+    p.mass[:] = 0.01
+    p.J[:] = 1.0
+    cfg = M.Config(grid_dx=dx, grid_size=(g, g, g), substeps=3, gravity=(0, -9.81, 0), damping=0.995)
+    grid = M.Grid(g, g, g, dx, (0.0, 0.0, 0.0))
+    mats = [M.material(young_modulus=1e4, poisson_ratio=0.25, density=1000.0)]
+    idx = np.arange(n, dtype=np.uint64)
+    a, b = p.copy(), p.copy()
+    ctx.step_parallel_with_grid(a, grid, cfg, mats, [M.NEO_HOOKEAN], 0.016, idx)
+    assert O.step_parallel_with_grid(b, grid, cfg, mats, [M.NEO_HOOKEAN], 0.016, idx) == 0
+    assert rel(a.pos, b.pos) <= 2e-5
+    a, b = p.copy(), p.copy()
+    ctx.step_velocity_only_parallel(a, grid, cfg, 0.1, idx)
+    assert O.step_velocity_only_parallel(b, grid, cfg, 0.1, idx) == 0
+    assert rel(a.pos, b.pos) <= 2e-5
