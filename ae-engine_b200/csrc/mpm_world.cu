@@ -3315,20 +3315,10 @@ class World final : public WorldBase {
     if (rc || !keep_queued) return rc;
     scatter_invalid_ = false;
     // the slot's blocks may hold the last scatter of the scene that vacated it: zero them (their
-    // flags stay set, so the touched list keeps each block once) and scatter the new particles
+    // flags stay set, so the touched list keeps each block once); the next step() scatters the new
+    // particles once it has put them in cell order
     AE_TRY(cudaMemsetAsync(acc_ + uint64_t(h.blk_off) * 64u, 0, sizeof(V4) * 64 * blocks_of(descs_[s]), stream_));
-    if ((rc = prepare())) return rc;
-    if (n == 0) return AE_MPM_OK;
-    WorldDev<T> w = with_list(dev(false), int(substep_ & 1));
-    const int c0 = chunk_first_[s], c1 = chunk_first_[s + 1];
-    if (!w.one_scene) w.chunks = d_chunks_ + c0;
-    const size_t per = sizeof(V4) * kLaneVecs + sizeof(int4);
-    if (!lanes_smem_set_) {
-      AE_TRY(cudaFuncSetAttribute(p2g_lanes_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * 256)));
-      lanes_smem_set_ = true;
-    }
-    p2g_lanes_kernel<T><<<unsigned(c1 - c0), chunk_threads_, per * chunk_threads_, stream_>>>(w);
-    AE_TRY(cudaGetLastError());
+    if (std::find(late_slots_.begin(), late_slots_.end(), s) == late_slots_.end()) late_slots_.push_back(s);
     return AE_MPM_OK;
   }
 
@@ -3563,17 +3553,20 @@ class World final : public WorldBase {
     ++launches_;
   }
 
+  void launch_p2g_lanes(WorldDev<T>& w, int chunks) {
+    const size_t per = sizeof(V4) * kLaneVecs + sizeof(int4);
+    if (!lanes_smem_set_) {  // sized for the largest block (256 threads) the world accepts
+      cudaFuncSetAttribute(p2g_lanes_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * 256));
+      lanes_smem_set_ = true;
+    }
+    p2g_lanes_kernel<T><<<chunks, chunk_threads_, per * chunk_threads_, stream_>>>(w);
+  }
+
   template <int MODE>
   void launch_p2g(WorldDev<T>& w) {
     const size_t sm = sizeof(V4) * max_tile_nodes();
     if (MODE == AE_MPM_MODE_PHYSICS && opts_.p2g_variant == kVarLanes) {
-      const size_t per = sizeof(V4) * kLaneVecs + sizeof(int4);
-      const size_t sm2 = per * chunk_threads_;
-      if (!lanes_smem_set_) {  // sized for the largest block (256 threads) the world accepts
-        cudaFuncSetAttribute(p2g_lanes_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * 256));
-        lanes_smem_set_ = true;
-      }
-      p2g_lanes_kernel<T><<<n_chunks_, chunk_threads_, sm2, stream_>>>(w);
+      launch_p2g_lanes(w, n_chunks_);
       return;
     }
     if (MODE == AE_MPM_MODE_REFERENCE && opts_.p2g_variant == kVarLanes) {
@@ -3686,13 +3679,28 @@ class World final : public WorldBase {
       scatter_pending_ = false;
     }
     scatter_invalid_ = false;
+    // In cell order: particles as the caller stored them would each be a run of their own, 27 vector
+    // reductions per particle instead of per cell and warp (dam break, 8.4 M particles in random
+    // order: 7.3 ms of P2G against 0.8 with the sort the first substep does anyway).
     if (fused() && !scatter_pending_ && n_chunks_ > 0) {
+      if (phase_ == 0 && !sorted_) sort_particles();
       AE_TRY(cudaMemsetAsync(touched_count(par), 0, sizeof(uint32_t), stream_));
-      WorldDev<T> w = with_list(dev(false), par);
+      WorldDev<T> w = with_list(dev(sorted_), par);
       launch_p2g<AE_MPM_MODE_PHYSICS>(w);
       ++launches_;
       scatter_pending_ = true;
+    } else if (fused() && !late_slots_.empty()) {  // only the slots assigned since the last step
+      if (phase_ == 0 && !sorted_) sort_particles();
+      for (uint32_t s : late_slots_) {
+        const int c0 = chunk_first_[s], c1 = chunk_first_[s + 1];
+        if (c1 == c0 || h_scenes_[s].p_count == 0) continue;
+        WorldDev<T> w = with_list(dev(sorted_), par);
+        if (!w.one_scene) w.chunks = d_chunks_ + c0;
+        launch_p2g_lanes(w, c1 - c0);
+        ++launches_;
+      }
     }
+    late_slots_.clear();
     AE_TRY(cudaGetLastError());
     return AE_MPM_OK;
   }
@@ -3914,6 +3922,7 @@ class World final : public WorldBase {
   bool lanes_smem_set_ = false, fused_smem_set_ = false, ref_lanes_smem_set_ = false;
   bool scatter_pending_ = false;  // the accumulator holds the P2G of the current particle state
   bool scatter_invalid_ = false;  // the particles changed since that scatter
+  std::vector<uint32_t> late_slots_;  // slots assigned into a queued scatter, not scattered themselves yet
   uint64_t substep_ = 0, snap_substep_ = 0, launches_ = 0;
   cudaEvent_t* stage_events_ = nullptr;
   cudaEvent_t xfer_ev_ = nullptr;  // orders copy streams against the world's stream
