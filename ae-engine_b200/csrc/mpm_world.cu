@@ -2370,35 +2370,54 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(WorldDev<T> w, uint32_
   if (live && pos < n_slots) perm[pos] = uint32_t(j);
 }
 
-// staging layout (elements of T): pos 3n | vel 3n | F 9n | J n | C 9n | mass n | then u16 mat n
+// One scene's particles in the caller's layout: arrays of the caller on this device, or a staging
+// area (pos 3n | vel 3n | F 9n | J n | C 9n | mass n, then n u16 material indices).
 template <class T>
-__global__ void pack_kernel(typename V4T<T>::type* const* dst, const T* __restrict__ st, uint64_t n, uint32_t p_off,
-                            const SceneDev<T>* scp, const MatDev* mats) {
-  uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const T* pos = st;
-  const T* vel = st + 3 * n;
-  const T* F = st + 6 * n;
-  const T* J = st + 15 * n;
-  const T* C = st + 16 * n;
-  const T* mass = st + 25 * n;
-  const uint16_t* mat = reinterpret_cast<const uint16_t*>(st + 26 * n);
-  uint64_t s = p_off + i;
-  dst[0][s] = mk4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], mass[i]);
-  dst[1][s] = mk4(F[9 * i], F[9 * i + 1], F[9 * i + 2], F[9 * i + 3]);
-  dst[2][s] = mk4(F[9 * i + 4], F[9 * i + 5], F[9 * i + 6], F[9 * i + 7]);
-  dst[3][s] = mk4(F[9 * i + 8], J[i], Bits<T>::pack(uint32_t(mat[i])), Bits<T>::pack(uint32_t(i)));
-  T c[9];
+struct XferDev {
+  T* f[6];  // pos, vel, F, J, C, mass
+  uint16_t* mat;
+  uint32_t n, pad;
+};
+// The scenes of one transfer: a single one by value, or a table over the scenes s0, s0 + 1, ... (n = 0
+// for scenes that do not take part).
+template <class T>
+struct XferSet {
+  const XferDev<T>* tab;
+  uint32_t s0;
+  XferDev<T> one;
+  __device__ __forceinline__ XferDev<T> of(uint32_t s) const { return tab ? tab[s - s0] : one; }
+};
+
+// Caller's layout -> slots, one launch for all scenes of a transfer (a launch per scene, 4.6 us each
+// for 19 000 particles, took 2.4 ms for 512 scenes against 0.4 together).  Bound by memory: 106 bytes
+// read and 112 written per particle run at the copy rate.
+template <class T>
+__global__ void __launch_bounds__(256) pack_kernel(WorldDev<T> w, XferSet<T> xs) {
+  using V4 = typename V4T<T>::type;
+  const int4 ch = cta_chunk(w);
+  const SceneDev<T>& sc = w.scenes[ch.x];
+  const XferDev<T> d = xs.of(uint32_t(ch.x));
+  const uint32_t s = uint32_t(ch.y) + threadIdx.x;
+  const uint64_t i = s - sc.p_off;
+  if (i >= d.n) return;
+  V4* const* dst = const_cast<V4* const*>(w.in);
+  const T *pos = d.f[0], *vel = d.f[1], *F = d.f[2], *C = d.f[4];
+  const T J = d.f[3][i], m = d.f[5][i];
+  const uint32_t mi = d.mat[i];
+  T f[9], c[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) c[k] = C[9 * i + k];
-  const SceneDev<T>& sc = *scp;
+  for (int k = 0; k < 9; ++k) {
+    f[k] = F[9 * i + k];
+    c[k] = C[9 * i + k];
+  }
+  dst[0][s] = mk4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], m);
+  dst[1][s] = mk4(f[0], f[1], f[2], f[3]);
+  dst[2][s] = mk4(f[4], f[5], f[6], f[7]);
+  dst[3][s] = mk4(f[8], J, Bits<T>::pack(mi), Bits<T>::pack(uint32_t(i)));
   if (sc.mode == AE_MPM_MODE_PHYSICS) {  // the C slot holds A = m C - k tau on the device
-    const uint32_t mi = mat[i];
-    const MatDev& md = mats[sc.mat_off + (mi < sc.n_mat ? mi : sc.n_mat)];
-    T f[9], a[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) f[k] = F[9 * i + k];
-    affine_from_c(sc, md, mass[i], c, f, J[i], a);
+    const MatDev& md = w.mats[sc.mat_off + (mi < sc.n_mat ? mi : sc.n_mat)];
+    T a[9];
+    affine_from_c(sc, md, m, c, f, J, a);
 #pragma unroll
     for (int k = 0; k < 9; ++k) c[k] = a[k];
   }
@@ -2407,49 +2426,83 @@ __global__ void pack_kernel(typename V4T<T>::type* const* dst, const T* __restri
   dst[6][s] = mk4(c[5], c[6], c[7], c[8]);
 }
 
+// Slots -> caller's layout in two launches: the slot of each original index (inv), then a gather
+// that writes every array in order.  Scattering from the slots instead (one launch) sends each
+// particle's 12- and 36-byte rows to lines of their own: 3.46 ms for 8.4 M particles whose order is
+// not the caller's, 0.14 for 1 M that nearly kept it.
 template <class T>
-__global__ void unpack_kernel(const typename V4T<T>::type* const* src, T* __restrict__ st, uint64_t n, uint32_t p_off,
-                              const SceneDev<T>* scp, const MatDev* mats) {
+__global__ void __launch_bounds__(256) unpack_index_kernel(WorldDev<T> w, XferSet<T> xs, uint32_t* __restrict__ inv) {
+  const int4 ch = cta_chunk(w);
+  const SceneDev<T>& sc = w.scenes[ch.x];
+  const uint32_t n = xs.of(uint32_t(ch.x)).n;
+  const uint32_t s = uint32_t(ch.y) + threadIdx.x;
+  if (s - sc.p_off >= n) return;
+  const uint32_t o = Bits<T>::unpack(w.in[3][s].w);
+  if (o < n) inv[sc.p_off + o] = s;
+}
+
+// rows of K values per lane -> K consecutive values per particle at dst[i0 * K], through the warp's
+// shared row buffer, so that each store instruction writes consecutive values
+template <int K, class T>
+__device__ __forceinline__ void store_rows(T* dst, uint64_t i0, uint64_t n, const T* v, T* buf, bool has, int lane) {
+  if (has) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) buf[lane * K + k] = v[k];
+  }
+  __syncwarp();
+  const uint64_t end = n * K;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const uint64_t q = i0 * K + uint64_t(k * 32 + lane);
+    if (q < end) dst[q] = buf[k * 32 + lane];
+  }
+  __syncwarp();
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) unpack_kernel(WorldDev<T> w, XferSet<T> xs, const uint32_t* __restrict__ inv) {
   using V4 = typename V4T<T>::type;
-  uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t s = p_off + i;
-  V4 a0 = src[0][s], a1 = src[1][s], a2 = src[2][s], a3 = src[3][s], a4 = src[4][s], a5 = src[5][s], a6 = src[6][s];
-  uint64_t o = Bits<T>::unpack(a3.w);
-  if (o >= n) return;
-  T* pos = st;
-  T* vel = st + 3 * n;
-  T* F = st + 6 * n;
-  T* J = st + 15 * n;
-  T* C = st + 16 * n;
-  T* mass = st + 25 * n;
-  uint16_t* mat = reinterpret_cast<uint16_t*>(st + 26 * n);
-  pos[3 * o] = a0.x;
-  pos[3 * o + 1] = a0.y;
-  pos[3 * o + 2] = a0.z;
-  mass[o] = a0.w;
-  const T f[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
-  T c[9] = {a4.w, a5.x, a5.y, a5.z, a5.w, a6.x, a6.y, a6.z, a6.w};
-  const SceneDev<T>& sc = *scp;
-  if (sc.mode == AE_MPM_MODE_PHYSICS) {  // C = (A + k tau) / m
-    const uint32_t mi = Bits<T>::unpack(a3.z) & 0xffffu;
-    const MatDev& md = mats[sc.mat_off + (mi < sc.n_mat ? mi : sc.n_mat)];
-    T tau[9];
-    phys_tau(md, f, a3.y, tau);
-    const T k = affine_k(sc, md, a0.w);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) c[q] = (c[q] + k * tau[q]) / a0.w;
+  __shared__ T rows[8][32 * 9];
+  const int4 ch = cta_chunk(w);
+  const SceneDev<T>& sc = w.scenes[ch.x];
+  const XferDev<T> d = xs.of(uint32_t(ch.x));
+  const int lane = threadIdx.x & 31;
+  T* buf = rows[threadIdx.x >> 5];
+  const uint64_t i = uint32_t(ch.y) + threadIdx.x - sc.p_off, i0 = i - lane;
+  if (i0 >= d.n) return;  // warp-uniform
+  bool has = i < d.n;
+  uint32_t s = 0;
+  if (has) {
+    s = inv[sc.p_off + i];
+    has = s - sc.p_off < d.n;
   }
+  T f[9], c[9], x[3], v[3], J = T(0), m = T(0);
+  uint32_t mi = 0;
+  if (has) {
+    const V4 a0 = ld4(w.in[0] + s), a1 = ld4(w.in[1] + s), a2 = ld4(w.in[2] + s), a3 = ld4(w.in[3] + s);
+    const V4 a4 = ld4(w.in[4] + s), a5 = ld4(w.in[5] + s), a6 = ld4(w.in[6] + s);
+    x[0] = a0.x, x[1] = a0.y, x[2] = a0.z, m = a0.w;
+    v[0] = a4.x, v[1] = a4.y, v[2] = a4.z;
+    J = a3.y;
+    mi = Bits<T>::unpack(a3.z) & 0xffffu;
+    f[0] = a1.x, f[1] = a1.y, f[2] = a1.z, f[3] = a1.w, f[4] = a2.x, f[5] = a2.y, f[6] = a2.z, f[7] = a2.w, f[8] = a3.x;
+    c[0] = a4.w, c[1] = a5.x, c[2] = a5.y, c[3] = a5.z, c[4] = a5.w, c[5] = a6.x, c[6] = a6.y, c[7] = a6.z, c[8] = a6.w;
+    if (sc.mode == AE_MPM_MODE_PHYSICS) {  // C = (A + k tau) / m
+      const MatDev& md = w.mats[sc.mat_off + (mi < sc.n_mat ? mi : sc.n_mat)];
+      T tau[9];
+      phys_tau(md, f, J, tau);
+      const T k = affine_k(sc, md, m);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    F[9 * o + k] = f[k];
-    C[9 * o + k] = c[k];
+      for (int q = 0; q < 9; ++q) c[q] = (c[q] + k * tau[q]) / m;
+    }
+    d.f[3][i] = J;
+    d.f[5][i] = m;
+    d.mat[i] = uint16_t(mi);
   }
-  J[o] = a3.y;
-  vel[3 * o] = a4.x;
-  vel[3 * o + 1] = a4.y;
-  vel[3 * o + 2] = a4.z;
-  mat[o] = uint16_t(Bits<T>::unpack(a3.z) & 0xffffu);
+  store_rows<3>(d.f[0], i0, d.n, x, buf, has, lane);
+  store_rows<3>(d.f[1], i0, d.n, v, buf, has, lane);
+  store_rows<9>(d.f[2], i0, d.n, f, buf, has, lane);
+  store_rows<9>(d.f[4], i0, d.n, c, buf, has, lane);
 }
 
 // per-chunk FP64 partial sums [mass, px, py, pz, ke]; fixed reduction order (deterministic)
@@ -2691,10 +2744,6 @@ class World final : public WorldBase {
       AE_TRY(dmalloc(&bufA_[k], sizeof(V4) * pc));
       AE_TRY(dmalloc(&bufB_[k], sizeof(V4) * pc));
     }
-    AE_TRY(dmalloc(&d_ptrA_, sizeof(V4*) * 7));
-    AE_TRY(dmalloc(&d_ptrB_, sizeof(V4*) * 7));
-    AE_TRY(cudaMemcpy(d_ptrA_, bufA_, sizeof(V4*) * 7, cudaMemcpyHostToDevice));
-    AE_TRY(cudaMemcpy(d_ptrB_, bufB_, sizeof(V4*) * 7, cudaMemcpyHostToDevice));
     AE_TRY(dmalloc(&keys_, sizeof(uint32_t) * pc));
     // Dense grouping reads every node's counter; the radix sort moves 20 bytes per key and pass.
     // The grid decides: up to 16 nodes per particle slot (or 8 M nodes, 5 us of scan) the dense
@@ -2778,10 +2827,8 @@ class World final : public WorldBase {
     if (rebase) {
       int rc = ensure_stage(cnt);
       if (rc) return rc;
-      if ((rc = sync_tables())) return rc;
-      unpack_kernel<T><<<unsigned((cnt + 255) / 256), 256, 0, stream_>>>(in_ptrs_dev(), stage_, cnt, h_scenes_[s].p_off,
-                                                                          d_scenes_ + s, d_mats_);
-      AE_TRY(cudaGetLastError());
+      const XferDev<T> x = stage_xfer(stage_, cnt);
+      if ((rc = launch_unpack(1, &s, &x))) return rc;
     }
     fill_scene_params(h_scenes_[s], d);
     for (uint32_t k = 0; k < d.n_materials; ++k) {
@@ -2798,13 +2845,120 @@ class World final : public WorldBase {
     keys_stale_ = true;  // dx or origin may have moved the cells
     scatter_invalid_ = true;
     if (rebase) {
-      int rc = sync_tables();
+      const XferDev<T> x = stage_xfer(stage_, cnt);
+      const int rc = launch_pack(1, &s, &x);
       if (rc) return rc;
-      pack_kernel<T><<<unsigned((cnt + 255) / 256), 256, 0, stream_>>>(in_ptrs_dev(), stage_, cnt, h_scenes_[s].p_off,
-                                                                        d_scenes_ + s, d_mats_);
-      AE_TRY(cudaGetLastError());
       keys_stale_ = true;
     }
+    return AE_MPM_OK;
+  }
+
+  static XferDev<T> stage_xfer(T* st, uint64_t n) {
+    return XferDev<T>{{st, st + 3 * n, st + 6 * n, st + 15 * n, st + 16 * n, st + 25 * n},
+                      reinterpret_cast<uint16_t*>(st + 26 * n), uint32_t(n), 0u};
+  }
+  static XferDev<T> view_xfer(const HostView<T>& hv, uint64_t n) {
+    return XferDev<T>{{hv.f[0], hv.f[1], hv.f[2], hv.f[3], hv.f[4], hv.f[5]}, hv.mat, uint32_t(n), 0u};
+  }
+
+  // Whether the kernels may use the caller's arrays in place: every one of them ordinary memory of
+  // the world's device, aligned for its type.  Anything else (host, managed or another device's
+  // memory, odd addresses) travels through the staging area.
+  static bool direct_view(const HostView<T>& hv) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (int k = 0; k < 7; ++k) {
+      const void* p = k < 6 ? static_cast<const void*>(hv.f[k]) : hv.mat;
+      if (reinterpret_cast<uintptr_t>(p) % (k < 6 ? sizeof(T) : sizeof(uint16_t)) != 0) return false;
+      cudaPointerAttributes a{};
+      if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      if (a.type != cudaMemoryTypeDevice || a.device != dev) return false;
+    }
+    return true;
+  }
+
+  // Launch range and description of a transfer of k scenes (x[i] describes scene scenes[i]); false
+  // when no particle moves.  A single scene travels as a launch parameter, several as a table.
+  int xfer_range(uint32_t k, const uint32_t* scenes, const XferDev<T>* x, WorldDev<T>& w, XferSet<T>& xs, int& blocks) {
+    blocks = 0;
+    int rc = prepare();
+    if (rc) return rc;
+    w = dev(false);
+    xs = XferSet<T>{};
+    int c0 = 0;
+    if (k == 1) {
+      xs.one = x[0];
+      c0 = chunk_first_[scenes[0]];
+      blocks = int((x[0].n + uint32_t(chunk_threads_) - 1) / uint32_t(chunk_threads_));
+    } else {
+      uint32_t lo = scenes[0], hi = scenes[0];
+      for (uint32_t i = 1; i < k; ++i) {
+        lo = std::min(lo, scenes[i]);
+        hi = std::max(hi, scenes[i]);
+      }
+      h_xfer_.assign(hi - lo + 1, XferDev<T>{});
+      for (uint32_t i = 0; i < k; ++i) h_xfer_[scenes[i] - lo] = x[i];
+      if (h_xfer_.size() > xfer_cap_) {
+        AE_TRY(cudaStreamSynchronize(stream_));  // queued transfers may still read the old table
+        dfree(d_xfer_);
+        d_xfer_ = nullptr;
+        xfer_cap_ = 0;
+        AE_TRY(dmalloc(&d_xfer_, sizeof(XferDev<T>) * h_xfer_.size()));
+        xfer_cap_ = h_xfer_.size();
+      }
+      AE_TRY(cudaMemcpyAsync(d_xfer_, h_xfer_.data(), sizeof(XferDev<T>) * h_xfer_.size(), cudaMemcpyHostToDevice,
+                             stream_));
+      xs.tab = d_xfer_;
+      xs.s0 = lo;
+      c0 = chunk_first_[lo];
+      blocks = chunk_first_[hi + 1] - c0;
+    }
+    if (!w.one_scene) w.chunks = d_chunks_ + c0;
+    return AE_MPM_OK;
+  }
+
+  // a scene named twice in one call is transferred twice, in order
+  static bool has_repeats(uint32_t k, const uint32_t* scenes) {
+    std::vector<uint32_t> v(scenes, scenes + k);
+    std::sort(v.begin(), v.end());
+    return std::adjacent_find(v.begin(), v.end()) != v.end();
+  }
+
+  int launch_pack(uint32_t k, const uint32_t* scenes, const XferDev<T>* x) {
+    if (k > 1 && has_repeats(k, scenes)) {
+      int rc = AE_MPM_OK;
+      for (uint32_t i = 0; i < k && rc == AE_MPM_OK; ++i) rc = launch_pack(1, scenes + i, x + i);
+      return rc;
+    }
+    WorldDev<T> w{};
+    XferSet<T> xs{};
+    int blocks = 0;
+    const int rc = xfer_range(k, scenes, x, w, xs, blocks);
+    if (rc || blocks == 0) return rc;
+    pack_kernel<T><<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs);
+    AE_TRY(cudaGetLastError());
+    return AE_MPM_OK;
+  }
+
+  // the slot index lives in the clamp queue, which is empty between substeps
+  int launch_unpack(uint32_t k, const uint32_t* scenes, const XferDev<T>* x) {
+    if (k > 1 && has_repeats(k, scenes)) {
+      int rc = AE_MPM_OK;
+      for (uint32_t i = 0; i < k && rc == AE_MPM_OK; ++i) rc = launch_unpack(1, scenes + i, x + i);
+      return rc;
+    }
+    WorldDev<T> w{};
+    XferSet<T> xs{};
+    int blocks = 0;
+    const int rc = xfer_range(k, scenes, x, w, xs, blocks);
+    if (rc || blocks == 0) return rc;
+    uint32_t* inv = reinterpret_cast<uint32_t*>(clamp_queue_);
+    unpack_index_kernel<T><<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs, inv);
+    unpack_kernel<T><<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs, inv);
+    AE_TRY(cudaGetLastError());
     return AE_MPM_OK;
   }
 
@@ -2832,33 +2986,23 @@ class World final : public WorldBase {
             std::to_string(h_scenes_[s].p_cap);
       return AE_MPM_EINVAL;
     }
-    HostView<T> hv = host_view<T>(host);
+    const HostView<T> hv = host_view<T>(host);
     const T* const* f = hv.f;
     if (n > 0 && (!f[0] || !f[1] || !f[2] || !f[3] || !f[4] || !f[5] || !hv.mat)) {
       err = "particle view has a null array";
       return AE_MPM_EINVAL;
     }
-    int rc = ensure_stage(n);
-    if (rc) return rc;
     if (n > 0) {
-      // the view's arrays may be host or device memory (unified addressing picks the direction);
-      // a view laid out as the staging itself travels in one copy
-      if (staging_layout(hv, n)) {
-        AE_TRY(cudaMemcpyAsync(stage_, f[0], sizeof(T) * 26 * n + sizeof(uint16_t) * n, cudaMemcpyDefault, stream_));
-      } else {
-        AE_TRY(cudaMemcpyAsync(stage_, f[0], sizeof(T) * 3 * n, cudaMemcpyDefault, stream_));
-        AE_TRY(cudaMemcpyAsync(stage_ + 3 * n, f[1], sizeof(T) * 3 * n, cudaMemcpyDefault, stream_));
-        AE_TRY(cudaMemcpyAsync(stage_ + 6 * n, f[2], sizeof(T) * 9 * n, cudaMemcpyDefault, stream_));
-        AE_TRY(cudaMemcpyAsync(stage_ + 15 * n, f[3], sizeof(T) * n, cudaMemcpyDefault, stream_));
-        AE_TRY(cudaMemcpyAsync(stage_ + 16 * n, f[4], sizeof(T) * 9 * n, cudaMemcpyDefault, stream_));
-        AE_TRY(cudaMemcpyAsync(stage_ + 25 * n, f[5], sizeof(T) * n, cudaMemcpyDefault, stream_));
-        AE_TRY(cudaMemcpyAsync(stage_ + 26 * n, hv.mat, sizeof(uint16_t) * n, cudaMemcpyDefault, stream_));
+      XferDev<T> x = view_xfer(hv, n);
+      if (!direct_view(hv)) {
+        const int rs = ensure_stage(n);
+        if (rs) return rs;
+        const int rc = stage_in(stage_, hv, n, stream_);
+        if (rc) return rc;
+        x = stage_xfer(stage_, n);
       }
-      rc = sync_tables();
+      const int rc = launch_pack(1, &s, &x);
       if (rc) return rc;
-      pack_kernel<T><<<unsigned((n + 255) / 256), 256, 0, stream_>>>(in_ptrs_dev(), stage_, n, h_scenes_[s].p_off,
-                                                                      d_scenes_ + s, d_mats_);
-      AE_TRY(cudaGetLastError());
     }
     scatter_invalid_ = true;
     // the same count keeps the scene table, the chunks and the captured graph (which replays from
@@ -2888,25 +3032,42 @@ class World final : public WorldBase {
       err = "particle view has a null array";
       return AE_MPM_EINVAL;
     }
-    int rc = ensure_stage(n);
-    if (rc) return rc;
-    rc = sync_tables();
-    if (rc) return rc;
-    unpack_kernel<T><<<unsigned((n + 255) / 256), 256, 0, stream_>>>(in_ptrs_dev(), stage_, n, h_scenes_[s].p_off,
-                                                                      d_scenes_ + s, d_mats_);
-    AE_TRY(cudaGetLastError());
-    if (staging_layout(hv, n)) {
-      AE_TRY(cudaMemcpyAsync(f[0], stage_, sizeof(T) * 26 * n + sizeof(uint16_t) * n, cudaMemcpyDefault, stream_));
-    } else {
-      AE_TRY(cudaMemcpyAsync(f[0], stage_, sizeof(T) * 3 * n, cudaMemcpyDefault, stream_));
-      AE_TRY(cudaMemcpyAsync(f[1], stage_ + 3 * n, sizeof(T) * 3 * n, cudaMemcpyDefault, stream_));
-      AE_TRY(cudaMemcpyAsync(f[2], stage_ + 6 * n, sizeof(T) * 9 * n, cudaMemcpyDefault, stream_));
-      AE_TRY(cudaMemcpyAsync(f[3], stage_ + 15 * n, sizeof(T) * n, cudaMemcpyDefault, stream_));
-      AE_TRY(cudaMemcpyAsync(f[4], stage_ + 16 * n, sizeof(T) * 9 * n, cudaMemcpyDefault, stream_));
-      AE_TRY(cudaMemcpyAsync(f[5], stage_ + 25 * n, sizeof(T) * n, cudaMemcpyDefault, stream_));
-      AE_TRY(cudaMemcpyAsync(hv.mat, stage_ + 26 * n, sizeof(uint16_t) * n, cudaMemcpyDefault, stream_));
+    const bool direct = direct_view(hv);
+    XferDev<T> x = view_xfer(hv, n);
+    if (!direct) {
+      const int rs = ensure_stage(n);
+      if (rs) return rs;
+      x = stage_xfer(stage_, n);
     }
+    int rc = launch_unpack(1, &s, &x);
+    if (rc) return rc;
+    if (!direct && (rc = stage_out(stage_, hv, n, stream_))) return rc;
     AE_TRY(cudaStreamSynchronize(stream_));
+    return AE_MPM_OK;
+  }
+
+  // a view's arrays into a staging area and back (unified addressing picks the direction); a view
+  // laid out as the staging itself travels in one copy
+  int stage_in(T* st, const HostView<T>& hv, uint64_t n, cudaStream_t cs) {
+    if (staging_layout(hv, n)) {
+      AE_TRY(cudaMemcpyAsync(st, hv.f[0], sizeof(T) * 26 * n + sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
+      return AE_MPM_OK;
+    }
+    const uint64_t at[6] = {0, 3, 6, 15, 16, 25}, len[6] = {3, 3, 9, 1, 9, 1};
+    for (int f = 0; f < 6; ++f)
+      AE_TRY(cudaMemcpyAsync(st + at[f] * n, hv.f[f], sizeof(T) * len[f] * n, cudaMemcpyDefault, cs));
+    AE_TRY(cudaMemcpyAsync(st + 26 * n, hv.mat, sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
+    return AE_MPM_OK;
+  }
+  int stage_out(const T* st, const HostView<T>& hv, uint64_t n, cudaStream_t cs) {
+    if (staging_layout(hv, n)) {
+      AE_TRY(cudaMemcpyAsync(hv.f[0], st, sizeof(T) * 26 * n + sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
+      return AE_MPM_OK;
+    }
+    const uint64_t at[6] = {0, 3, 6, 15, 16, 25}, len[6] = {3, 3, 9, 1, 9, 1};
+    for (int f = 0; f < 6; ++f)
+      AE_TRY(cudaMemcpyAsync(hv.f[f], st + at[f] * n, sizeof(T) * len[f] * n, cudaMemcpyDefault, cs));
+    AE_TRY(cudaMemcpyAsync(hv.mat, st + 26 * n, sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
     return AE_MPM_OK;
   }
 
@@ -2950,38 +3111,38 @@ class World final : public WorldBase {
         err = "particle view has a null array";
         return AE_MPM_EINVAL;
       }
-      total += stage_region(counts[i]);
     }
-    {
+    // views in device memory are read in place; the others get a region of the staging area each
+    std::vector<XferDev<T>> x(k);
+    std::vector<uint8_t> staged(k, 0);
+    for (uint32_t i = 0; i < k; ++i) {
+      const HostView<T> hv = host_view<T>(&views[i]);
+      x[i] = view_xfer(hv, counts[i]);
+      staged[i] = counts[i] > 0 && !direct_view(hv);
+      if (staged[i]) total += stage_region(counts[i]);
+    }
+    if (total > 0) {
       const int rs = ensure_stage_bytes(total);
       if (rs) return rs;
-    }
-    // all copies first, back to back on the copy stream (the world's own by default), then the packs
-    const cudaStream_t cs = copy ? copy : stream_;
-    if (copy) {  // the staging area is free once the world's queued work is done with it
-      const int r = stream_after(cs, stream_);
-      if (r) return r;
-    }
-    uint64_t off = 0;
-    for (uint32_t i = 0; i < k; ++i) {
-      const uint64_t n = counts[i];
-      T* st = reinterpret_cast<T*>(reinterpret_cast<char*>(stage_) + off);
-      HostView<T> hv = host_view<T>(&views[i]);
-      if (n > 0) {
-        if (staging_layout(hv, n)) {
-          AE_TRY(cudaMemcpyAsync(st, hv.f[0], sizeof(T) * 26 * n + sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
-        } else {
-          const uint64_t at[6] = {0, 3, 6, 15, 16, 25}, len[6] = {3, 3, 9, 1, 9, 1};
-          for (int f = 0; f < 6; ++f)
-            AE_TRY(cudaMemcpyAsync(st + at[f] * n, hv.f[f], sizeof(T) * len[f] * n, cudaMemcpyDefault, cs));
-          AE_TRY(cudaMemcpyAsync(st + 26 * n, hv.mat, sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
-        }
+      // all copies first, back to back on the copy stream (the world's own by default), then the pack
+      const cudaStream_t cs = copy ? copy : stream_;
+      if (copy) {  // the staging area is free once the world's queued work is done with it
+        const int r = stream_after(cs, stream_);
+        if (r) return r;
       }
-      off += stage_region(n);
-    }
-    if (copy) {
-      const int r = stream_after(stream_, cs);
-      if (r) return r;
+      uint64_t off = 0;
+      for (uint32_t i = 0; i < k; ++i) {
+        if (!staged[i]) continue;
+        T* st = reinterpret_cast<T*>(reinterpret_cast<char*>(stage_) + off);
+        const int r = stage_in(st, host_view<T>(&views[i]), counts[i], cs);
+        if (r) return r;
+        x[i] = stage_xfer(st, counts[i]);
+        off += stage_region(counts[i]);
+      }
+      if (copy) {
+        const int r = stream_after(stream_, cs);
+        if (r) return r;
+      }
     }
     for (uint32_t i = 0; i < k; ++i) {
       const uint32_t s = scenes[i];
@@ -2990,18 +3151,8 @@ class World final : public WorldBase {
         count_changed(s);
       }
     }
-    int rc = sync_tables();
+    const int rc = launch_pack(k, scenes, x.data());
     if (rc) return rc;
-    off = 0;
-    for (uint32_t i = 0; i < k; ++i) {
-      const uint64_t n = counts[i];
-      const T* st = reinterpret_cast<const T*>(reinterpret_cast<const char*>(stage_) + off);
-      if (n > 0)
-        pack_kernel<T><<<unsigned((n + 255) / 256), 256, 0, stream_>>>(in_ptrs_dev(), st, n, h_scenes_[scenes[i]].p_off,
-                                                                        d_scenes_ + scenes[i], d_mats_);
-      off += stage_region(n);
-    }
-    AE_TRY(cudaGetLastError());
     keys_stale_ = true;
     scatter_invalid_ = true;
     return AE_MPM_OK;
@@ -3029,45 +3180,35 @@ class World final : public WorldBase {
         err = "particle view has a null array";
         return AE_MPM_EINVAL;
       }
-      total += stage_region(h_scenes_[scenes[i]].p_count);
     }
-    {
+    std::vector<XferDev<T>> x(k);
+    std::vector<uint64_t> at(k, UINT64_MAX);  // offset of a staged scene's region
+    for (uint32_t i = 0; i < k; ++i) {
+      const uint64_t n = h_scenes_[scenes[i]].p_count;
+      const HostView<T> hv = host_view<T>(&views[i]);
+      x[i] = view_xfer(hv, n);
+      if (n == 0 || direct_view(hv)) continue;
+      at[i] = total;
+      total += stage_region(n);
+    }
+    if (total > 0) {
       const int rs = ensure_stage_bytes(total);
       if (rs) return rs;
     }
-    int rc = sync_tables();
+    for (uint32_t i = 0; i < k; ++i)
+      if (at[i] != UINT64_MAX)
+        x[i] = stage_xfer(reinterpret_cast<T*>(reinterpret_cast<char*>(stage_) + at[i]), x[i].n);
+    const int rc = launch_unpack(k, scenes, x.data());
     if (rc) return rc;
-    uint64_t off = 0;
-    for (uint32_t i = 0; i < k; ++i) {
-      const SceneDev<T>& h = h_scenes_[scenes[i]];
-      T* st = reinterpret_cast<T*>(reinterpret_cast<char*>(stage_) + off);
-      if (h.p_count > 0)
-        unpack_kernel<T><<<unsigned((h.p_count + 255) / 256), 256, 0, stream_>>>(in_ptrs_dev(), st, h.p_count, h.p_off,
-                                                                                 d_scenes_ + scenes[i], d_mats_);
-      off += stage_region(h.p_count);
-    }
-    AE_TRY(cudaGetLastError());
     const cudaStream_t cs = copy ? copy : stream_;
     if (copy) {
       const int r = stream_after(cs, stream_);
       if (r) return r;
     }
-    off = 0;
     for (uint32_t i = 0; i < k; ++i) {
-      const uint64_t n = h_scenes_[scenes[i]].p_count;
-      const T* st = reinterpret_cast<const T*>(reinterpret_cast<const char*>(stage_) + off);
-      HostView<T> hv = host_view<T>(&views[i]);
-      if (n > 0) {
-        if (staging_layout(hv, n)) {
-          AE_TRY(cudaMemcpyAsync(hv.f[0], st, sizeof(T) * 26 * n + sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
-        } else {
-          const uint64_t at[6] = {0, 3, 6, 15, 16, 25}, len[6] = {3, 3, 9, 1, 9, 1};
-          for (int f = 0; f < 6; ++f)
-            AE_TRY(cudaMemcpyAsync(hv.f[f], st + at[f] * n, sizeof(T) * len[f] * n, cudaMemcpyDefault, cs));
-          AE_TRY(cudaMemcpyAsync(hv.mat, st + 26 * n, sizeof(uint16_t) * n, cudaMemcpyDefault, cs));
-        }
-      }
-      off += stage_region(n);
+      if (at[i] == UINT64_MAX) continue;
+      const int r = stage_out(x[i].f[0], host_view<T>(&views[i]), x[i].n, cs);
+      if (r) return r;
     }
     if (copy) {  // the next use of the staging area on the world's stream waits for these reads
       const int r = stream_after(stream_, cs);
@@ -3403,7 +3544,6 @@ class World final : public WorldBase {
 
   V4** in_buf() { return a_in_ ? bufA_ : bufB_; }
   V4** out_buf() { return a_in_ ? bufB_ : bufA_; }
-  V4* const* in_ptrs_dev() { return a_in_ ? d_ptrA_ : d_ptrB_; }
 
   int ensure_stage(uint64_t n) { return ensure_stage_bytes(sizeof(T) * 26 * n + sizeof(uint16_t) * n + 64); }
   int ensure_stage_bytes(size_t need) {
@@ -3840,8 +3980,6 @@ class World final : public WorldBase {
       dfree(bufB_[k]);
       dfree(snap_[k]);
     }
-    dfree(d_ptrA_);
-    dfree(d_ptrB_);
     dfree(keys_);
     sort_scratch_free(sort_, alloc_ ? &World::sort_free : nullptr, alloc_);
     dfree(bins_);
@@ -3866,6 +4004,7 @@ class World final : public WorldBase {
     dfree(d_chunks_);
     dfree(partial_);
     dfree(stage_);
+    dfree(d_xfer_);
     if (stream_) cudaStreamDestroy(stream_);
   }
 
@@ -3888,8 +4027,6 @@ class World final : public WorldBase {
   V4* bufA_[7] = {};
   V4* bufB_[7] = {};
   V4* snap_[7] = {};
-  V4** d_ptrA_ = nullptr;
-  V4** d_ptrB_ = nullptr;
   bool a_in_ = true;
   uint32_t* keys_ = nullptr;
   SortScratch sort_;
@@ -3909,6 +4046,9 @@ class World final : public WorldBase {
   bool has_snow_ = false;
   T* stage_ = nullptr;
   size_t stage_bytes_ = 0;
+  std::vector<XferDev<T>> h_xfer_;  // many-scene transfer table
+  XferDev<T>* d_xfer_ = nullptr;
+  size_t xfer_cap_ = 0;
   double* partial_ = nullptr;
   cudaStream_t stream_ = nullptr;
   struct Graph {
