@@ -447,11 +447,10 @@ AE_HD bool clamp_is_identity(const T* F, T lo, T hi) {
          det3(F) > T(0);
 }
 
-// FP32 SVD, redone in FP64 when a near-degenerate pair straddles a clamp threshold
+// Whether a near-degenerate pair of singular values straddles a clamp threshold: the one case where
+// the clamped F depends on individual FP32 singular vectors, and the SVD is redone in FP64
 template <class T>
-AE_HD bool svd3_fallback(const T* F, T* U, T* s, T* V, bool allow, T lo, T hi) {
-  svd3(F, U, s, V);
-  if (!allow || sizeof(T) == sizeof(double)) return false;
+AE_HD bool svd3_straddles(const T* s, T lo, T hi) {
   T smax = t_max(t_abs(s[0]), T(1e-30));
   bool need = false;
 #pragma unroll
@@ -460,19 +459,7 @@ AE_HD bool svd3_fallback(const T* F, T* U, T* s, T* V, bool allow, T lo, T hi) {
     for (int j = i + 1; j < 3; ++j)
       if (t_abs(s[i] - s[j]) < T(kSvdGapTol) * smax && ((s[i] < lo) != (s[j] < lo) || (s[i] > hi) != (s[j] > hi)))
         need = true;
-  if (!need) return false;
-  double Fd[9], Ud[9], sd[3], Vd[9];
-#pragma unroll
-  for (int i = 0; i < 9; ++i) Fd[i] = double(F[i]);
-  svd3(Fd, Ud, sd, Vd);
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    U[i] = T(Ud[i]);
-    V[i] = T(Vd[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i) s[i] = T(sd[i]);
-  return true;
+  return need;
 }
 
 }  // namespace aemp

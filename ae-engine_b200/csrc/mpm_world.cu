@@ -1241,10 +1241,11 @@ __device__ __forceinline__ void g2p_physics_gather(const VelTile<T>& vt, const S
   for (int k = 0; k < 9; ++k) C[k] = cs * B[k];
 }
 
-// update half of the physics G2P: advection, F update and the material's return mapping
+// update half of the physics G2P: advection and the F or J update.  Snow whose F left the elastic
+// region (needs_clamp) has its trial F and old J_p here; everything else is final.  o.C keeps C.
 template <class T>
-__device__ __forceinline__ void g2p_physics_update(const SceneDev<T>& sc, const MatDev& md, const T* x0, const T* v,
-                                                   const T* F, T J, T m, G2POut<T>& o) {
+__device__ __forceinline__ void g2p_physics_move(const SceneDev<T>& sc, const MatDev& md, const T* x0, const T* v,
+                                                 const T* F, T J, G2POut<T>& o) {
   bool nan = false, clamped = false;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -1264,10 +1265,6 @@ __device__ __forceinline__ void g2p_physics_update(const SceneDev<T>& sc, const 
     o.J = t_max(Jn, T(0.01));
 #pragma unroll
     for (int k = 0; k < 9; ++k) o.F[k] = F[k];
-    T A[9];
-    affine_from_c(sc, md, m, o.C, o.F, o.J, A);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) o.C[k] = A[k];
     return;
   }
   T G[9];
@@ -1275,19 +1272,68 @@ __device__ __forceinline__ void g2p_physics_update(const SceneDev<T>& sc, const 
   for (int k = 0; k < 9; ++k) G[k] = ((k % 4 == 0) ? T(1) : T(0)) + sc.dt * o.C[k];
   mm3(G, F, o.F);
   if (md.model == kPhysSnow) {
-    // elastic region (every singular value provably inside the clamp interval): F_E and J_p
-    // are final; otherwise the clamp kernel does the SVD, the return mapping and A
+    // elastic region: every singular value provably inside the clamp interval, F_E and J_p are final
     o.J = J;
     o.needs_clamp = !clamp_is_identity(o.F, T(1) - T(md.theta_c), T(1) + T(md.theta_s));
   } else {
     o.J = det3(o.F);
   }
-  if (!o.needs_clamp) {  // the C slot carries A from here on
-    T A[9];
-    affine_from_c(sc, md, m, o.C, o.F, o.J, A);
+}
+
+// the C slot carries A = m C - k tau from here on (not for particles that still need the clamp)
+template <class T>
+__device__ __forceinline__ void g2p_physics_affine(const SceneDev<T>& sc, const MatDev& md, T m, G2POut<T>& o) {
+  T A[9];
+  affine_from_c(sc, md, m, o.C, o.F, o.J, A);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) o.C[k] = A[k];
+  for (int k = 0; k < 9; ++k) o.C[k] = A[k];
+}
+
+// The FP64 redo of the snow return mapping's SVD, taken by few particles: a call of its own, so that
+// its registers and stack stay out of the FP32 path.
+__device__ __noinline__ void svd3_fp64(const float* F, float* U, float* s, float* V) {
+  double Fd[9], Ud[9], sd[3], Vd[9];
+  for (int i = 0; i < 9; ++i) Fd[i] = double(F[i]);
+  svd3(Fd, Ud, sd, Vd);
+  for (int i = 0; i < 9; ++i) {
+    U[i] = float(Ud[i]);
+    V[i] = float(Vd[i]);
   }
+  for (int i = 0; i < 3; ++i) s[i] = float(sd[i]);
+}
+
+// Snow return mapping: F = U S V^T, singular values clamped to [1-theta_c, 1+theta_s],
+// J_p *= prod(S)/prod(S_clamped) (ae_physics/src/mpm.rs:565-606 plus Stomakhin's J_p), with the FP64
+// SVD redo where a near-degenerate pair straddles a threshold.  Returns whether it was redone.
+template <class T>
+__device__ __forceinline__ bool snow_return(const MatDev& md, bool redo, T* F, T& J) {
+  const T lo = T(1) - T(md.theta_c), hi = T(1) + T(md.theta_s);
+  T U[9], sg[3], V[9];
+  svd3(F, U, sg, V);
+  bool fb = false;
+  if constexpr (sizeof(T) == 4) {
+    if (redo && svd3_straddles(sg, lo, hi)) {
+      float tF[9], tU[9], ts[3], tV[9];
+      for (int i = 0; i < 9; ++i) tF[i] = F[i];
+      svd3_fp64(tF, tU, ts, tV);
+      for (int i = 0; i < 9; ++i) {
+        U[i] = tU[i];
+        V[i] = tV[i];
+      }
+      for (int i = 0; i < 3; ++i) sg[i] = ts[i];
+      fb = true;
+    }
+  }
+  T scl[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) scl[k] = t_min(t_max(sg[k], lo), hi);
+  J = J * ((sg[0] * sg[1] * sg[2]) / (scl[0] * scl[1] * scl[2]));
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      F[r * 3 + c] = U[r * 3 + 0] * scl[0] * V[c * 3 + 0] + U[r * 3 + 1] * scl[1] * V[c * 3 + 1] + U[r * 3 + 2] * scl[2] * V[c * 3 + 2];
+  return fb;
 }
 
 // mpm_substep_serial_active / parallel_with_indices G2P (mpm_solver.rs:914-1053, 1206-1325)
@@ -1589,7 +1635,8 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
     const T F[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
     if (MODE == AE_MPM_MODE_PHYSICS) {
       const MatDev& md = mat_of(w, sc, Bits<T>::unpack(a3.z) & 0xffffu);
-      g2p_physics_update<T>(sc, md, x0, pv, F, a3.y, a0.w, o);
+      g2p_physics_move<T>(sc, md, x0, pv, F, a3.y, o);
+      if (!o.needs_clamp) g2p_physics_affine<T>(sc, md, a0.w, o);
     } else if (MODE == AE_MPM_MODE_REFERENCE) {
       g2p_reference<T>(vt, sc, x0, F, o);
     } else {
@@ -1637,11 +1684,8 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
   if (need) w.clamp_queue[qbase + __popc(qmask & ((1u << lane) - 1u))] = make_uint2(uint32_t(j), uint32_t(ch.x));
 }
 
-// Snow return mapping for the particles G2P queued: F = U S V^T, singular values clamped to
-// [1-theta_c, 1+theta_s], J_p *= prod(S)/prod(S_clamped) (ae_physics/src/mpm.rs:565-606 plus
-// Stomakhin's J_p), with the FP64 SVD redo where a near-degenerate pair straddles a threshold.
-// 64 registers, 8 blocks of 128 per SM: the FP64 redo, taken by few particles, would otherwise set
-// the register count (94) and leave three quarters of the SM's warp slots empty.
+// Snow return mapping for the particles G2P queued, then A from the returned F.
+// 64 registers, 8 blocks of 128 per SM.
 template <class T>
 __global__ void __launch_bounds__(128, 8) snow_clamp_kernel(WorldDev<T> w) {
   using V4 = typename V4T<T>::type;
@@ -1659,20 +1703,8 @@ __global__ void __launch_bounds__(128, 8) snow_clamp_kernel(WorldDev<T> w) {
     const SceneDev<T>& sc = w.scenes[q.y];
     V4 a1 = w.out[1][q.x], a2 = w.out[2][q.x], a3 = w.out[3][q.x];
     const MatDev& md = mat_of(w, sc, Bits<T>::unpack(a3.z) & 0xffffu);
-    const T F[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
-    const T lo = T(1) - T(md.theta_c), hi = T(1) + T(md.theta_s);
-    T U[9], sg[3], V[9];
-    const bool fb = svd3_fallback(F, U, sg, V, w.svd_fallback != 0, lo, hi);
-    T scl[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) scl[k] = t_min(t_max(sg[k], lo), hi);
-    const T J = a3.y * ((sg[0] * sg[1] * sg[2]) / (scl[0] * scl[1] * scl[2]));
-    T nF[9];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        nF[r * 3 + c] = U[r * 3 + 0] * scl[0] * V[c * 3 + 0] + U[r * 3 + 1] * scl[1] * V[c * 3 + 1] + U[r * 3 + 2] * scl[2] * V[c * 3 + 2];
+    T nF[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x}, J = a3.y;
+    const bool fb = snow_return<T>(md, w.svd_fallback != 0, nF, J);
     w.out[1][q.x] = mk4(nF[0], nF[1], nF[2], nF[3]);
     w.out[2][q.x] = mk4(nF[4], nF[5], nF[6], nF[7]);
     w.out[3][q.x] = mk4(nF[8], J, a3.z, a3.w);
@@ -1708,7 +1740,7 @@ struct WarpStage {
   V4* col;   // col[pos * 9 + column]
   V4* wxm;   // wxm[pos] = (wx0, wx1, wx2, m)
   V4* acol;  // acol[pos] = dx * A[.][0]
-  int4* gk;  // gk[pos] = (stencil base, cell key)
+  int4* gk;  // gk[pos] = (cell key, block row pitch and plane pitch of its scene, -)
 };
 template <class T>
 __host__ __device__ constexpr size_t warp_stage_bytes() {
@@ -1730,8 +1762,8 @@ __device__ __forceinline__ WarpStage<T> warp_stage(unsigned char* smem, int warp
 // for particles whose 27 stencil nodes all lie inside their scene's grid, which G2P's domain clamp
 // guarantees.  Every lane of the warp calls it; has = false lanes contribute nothing.  x is the
 // position, mv = m v, A = m C - k tau.  The cell key is the global index of the stencil's base
-// node, unique across scenes.  kMixed: lanes may belong to different scenes (each run looks its
-// scene up from its base node's block); otherwise every lane belongs to scene sc.  write_keys: the
+// node, unique across scenes.  kMixed: lanes may belong to different scenes (sc is the lane's own);
+// otherwise every lane belongs to scene sc.  write_keys: the
 // next substep sorts, so each particle's key goes to its slot and, with dense grouping, each group
 // of equal keys is counted in its cell with one atomic (the grouping is needed here anyway).
 // runs of at most this many particles are summed one node per lane; longer ones by the column lanes
@@ -1801,7 +1833,23 @@ __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const Sce
     st.wxm[pos] = mk4(wt[0][0], wt[0][1], wt[0][2], m);
     st.acol[pos] = mk4(c0[0], c0[1], c0[2], T(0));
   }
-  st.gk[pos] = make_int4(g[0], g[1], g[2], int(key));
+  st.gk[pos] = make_int4(int(key), sc.nb[0], sc.nb[0] * sc.nb[1], 0);
+  if (kMixed && has) {
+    // the stencil's blocks (at most 2 per axis), every lane its own particle's at once: marked run by
+    // run, each run would wait for its flags in turn
+    uint32_t gb[8];
+    uint32_t set[8];
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int bx = (g[0] + 2 * (o & 1)) >> 2, by = (g[1] + (o & 2)) >> 2, bz = (g[2] + ((o >> 1) & 2)) >> 2;
+      gb[o] = sc.blk_off + (uint32_t(bz) * uint32_t(sc.nb[1]) + uint32_t(by)) * uint32_t(sc.nb[0]) + uint32_t(bx);
+    }
+#pragma unroll
+    for (int o = 0; o < 8; ++o) set[o] = *static_cast<volatile uint32_t*>(w.blk_flag + gb[o]);
+#pragma unroll
+    for (int o = 0; o < 8; ++o)
+      if (set[o] == 0u) mark_block(w, gb[o]);
+  }
   __syncwarp();
   // lanes 0..26 are 3 particle groups x 9 (y,z) columns; lanes 27..31 mirror lanes 22..26
   // (in-bounds reads, results never used)
@@ -1814,8 +1862,13 @@ __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const Sce
     starts &= starts - 1u;
     const int e0 = starts ? __ffs(starts) - 1 : 32;
     const int4 run = st.gk[s0];
-    if (uint32_t(run.w) == 0xffffffffu) continue;
-    const SceneDev<T>& rs = kMixed ? w.scenes[w.blk_scene[uint32_t(run.w) >> 6]] : sc;
+    const uint32_t rk = uint32_t(run.x);
+    if (rk == 0xffffffffu) continue;
+    // node index of the run's stencil node (X, Y, Z) = base + x part + y part + z part, each part the
+    // distance of that axis from the base node in the block-major order
+    const int r0 = int(rk & 3u), r1 = int((rk >> 2) & 3u), r2 = int((rk >> 4) & 3u);
+    const uint32_t row64 = uint32_t(run.y) << 6, plane64 = uint32_t(run.z) << 6;
+    const uint32_t rb = rk & ~63u;
     if (e0 - s0 <= kShortRun) {
       // a short run: one lane per stencil node (27 lanes), each summing every particle of the run
       // for its node; no combine across lane groups, one vector reduction per lane
@@ -1851,23 +1904,13 @@ __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const Sce
         }
       }
       if (lane < 27 && m != T(0)) {
-        const int Xn = run.x + xa, Yn = run.y + jn % 3, Zn = run.z + jn / 3;
-        const uint32_t node =
-            ((rs.blk_off + (uint32_t(Zn >> 2) * uint32_t(rs.nb[1]) + uint32_t(Yn >> 2)) * uint32_t(rs.nb[0]) +
-              uint32_t(Xn >> 2))
-             << 6) |
-            (uint32_t(Zn & 3) << 4) | (uint32_t(Yn & 3) << 2) | uint32_t(Xn & 3);
+        const uint32_t Xl = uint32_t(r0 + xa), Yl = uint32_t(r1 + jn % 3), Zl = uint32_t(r2 + jn / 3);
+        const uint32_t node = rb + ((Xl >> 2) << 6) + (Yl >> 2) * row64 + (Zl >> 2) * plane64 +
+                              ((Zl & 3u) << 4 | (Yl & 3u) << 2 | (Xl & 3u));
         atomic_add4(w.acc + node, m, px, py, pz);
-      }
-      if (kMixed && lane >= 27) {  // the run's stencil blocks (at most 2 per axis): lanes 27..31 and
-        for (int o = lane - 27; o < 8; o += 5) {  // 27..29 again
-          const int bx = (run.x + 2 * (o & 1)) >> 2, by = (run.y + (o & 2)) >> 2, bz = (run.z + ((o >> 1) & 2)) >> 2;
-          mark_block(w, rs.blk_off + (uint32_t(bz) * uint32_t(rs.nb[1]) + uint32_t(by)) * uint32_t(rs.nb[0]) + uint32_t(bx));
-        }
       }
       continue;
     }
-    const int X = run.x, Y = run.y + nb, Z = run.z + nc;
     T m0 = 0, x0 = 0, y0 = 0, z0 = 0, m1 = 0, x1 = 0, y1 = 0, z1 = 0, m2 = 0, x2 = 0, y2 = 0, z2 = 0;
     if constexpr (sizeof(T) == 4) {  // x and y of each node as one packed pair
       float2 q0 = make_float2(0.f, 0.f), q1 = q0, q2 = q0;
@@ -1919,17 +1962,12 @@ __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const Sce
       m2 = groups(m2), x2 = groups(x2), y2 = groups(y2), z2 = groups(z2);
     }
     if (lane < 9) {
-      const uint32_t row = ((rs.blk_off + (uint32_t(Z >> 2) * uint32_t(rs.nb[1]) + uint32_t(Y >> 2)) * uint32_t(rs.nb[0])) << 6) |
-                           (uint32_t(Z & 3) << 4) | (uint32_t(Y & 3) << 2);
-      auto node = [row](int xa) { return row + ((uint32_t(xa >> 2) << 6) | uint32_t(xa & 3)); };
-      if (m0 != T(0)) atomic_add4(w.acc + node(X), m0, x0, y0, z0);
-      if (m1 != T(0)) atomic_add4(w.acc + node(X + 1), m1, x1, y1, z1);
-      if (m2 != T(0)) atomic_add4(w.acc + node(X + 2), m2, x2, y2, z2);
-    }
-    if (kMixed && lane >= 9 && lane < 17) {  // the run's stencil blocks (at most 2 per axis)
-      const int o = lane - 9;
-      const int bx = (run.x + 2 * (o & 1)) >> 2, by = (run.y + (o & 2)) >> 2, bz = (run.z + ((o >> 1) & 2)) >> 2;
-      mark_block(w, rs.blk_off + (uint32_t(bz) * uint32_t(rs.nb[1]) + uint32_t(by)) * uint32_t(rs.nb[0]) + uint32_t(bx));
+      const uint32_t Yl = uint32_t(r1 + nb), Zl = uint32_t(r2 + nc);
+      const uint32_t row = rb + (Yl >> 2) * row64 + (Zl >> 2) * plane64 + ((Zl & 3u) << 4 | (Yl & 3u) << 2);
+      auto node = [row](uint32_t xl) { return row + ((xl >> 2) << 6 | (xl & 3u)); };
+      if (m0 != T(0)) atomic_add4(w.acc + node(uint32_t(r0)), m0, x0, y0, z0);
+      if (m1 != T(0)) atomic_add4(w.acc + node(uint32_t(r0 + 1)), m1, x1, y1, z1);
+      if (m2 != T(0)) atomic_add4(w.acc + node(uint32_t(r0 + 2)), m2, x2, y2, z2);
     }
   }
   if (!kMixed) {  // grid blocks of the warp's stencil bounding box (all inside the grid)
@@ -1950,6 +1988,23 @@ __device__ __forceinline__ void p2g_warp_scatter(const WorldDev<T>& w, const Sce
   __syncwarp();  // the staging region is free again
 }
 
+// snow_return on F (park[0..8]) and J_p (park[9]) at a stride of 32 in the warp's shared staging: a
+// call of its own, so that the fused kernel's other particles keep their registers
+template <class T>
+__device__ __noinline__ bool snow_return_parked(const MatDev* md, bool redo, T* park) {
+  T F[9], J = park[9 * 32];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) F[k] = park[k * 32];
+  const bool fb = snow_return<T>(*md, redo, F, J);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) park[k * 32] = F[k];
+  park[9 * 32] = J;
+  return fb;
+}
+
+// yielding snow particles of a warp from which on the fused kernel maps them back itself
+constexpr int kInlineClamp = 8;
+
 // G2P of substep s and P2G of substep s + 1 (physics mode).  The grid update of substep s ran
 // before; w.touched / w.touched_count are the touched-block list of substep s + 1.
 template <class T>
@@ -1968,6 +2023,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
   uint32_t err = 0;
   bool cl = false, need = false, has = false;
   T xs[3] = {0, 0, 0}, m = 0, mv[3] = {0, 0, 0}, A[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
   if (live) {
     const uint32_t src = w.perm ? w.perm[j] : uint32_t(j);
 #pragma unroll
@@ -1994,8 +2050,45 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
     const V4 a1 = pre[lane], a2 = pre[32 + lane], a3 = pre[64 + lane];
     const T F[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
     const MatDev& md = mat_of(w, sc, Bits<T>::unpack(a3.z) & 0xffffu);
-    g2p_physics_update<T>(sc, md, x0, pv, F, a3.y, a0.w, o);
-    w.out[0][j] = mk4(o.x[0], o.x[1], o.x[2], a0.w);
+    g2p_physics_move<T>(sc, md, x0, pv, F, a3.y, o);
+    need = o.needs_clamp;
+    // Yielding snow: a warp with many such particles maps them back here; a few are left to the
+    // clamp kernel, which packs 32 of them from all over into a warp.
+    const uint32_t yielding = __ballot_sync(live_mask, need);
+    m = a0.w;
+    if (__popc(yielding) >= kInlineClamp) {
+      // the particle waits in the warp's staging region (past the prefetched F) during the call
+      T* park = reinterpret_cast<T*>(pre + 96) + lane;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        park[k * 32] = o.F[k];
+        park[(10 + k) * 32] = o.C[k];
+      }
+      park[9 * 32] = o.J;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        park[(19 + a) * 32] = o.x[a];
+        park[(22 + a) * 32] = o.v[a];
+      }
+      park[25 * 32] = m;
+      if (need && snow_return_parked<T>(&md, w.svd_fallback != 0, park)) atomicAdd(w.err + 4 * ch.x + 1, 1u);
+      need = false;
+      const T volatile* back = park;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        o.F[k] = back[k * 32];
+        o.C[k] = back[(10 + k) * 32];
+      }
+      o.J = back[9 * 32];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        o.x[a] = back[(19 + a) * 32];
+        o.v[a] = back[(22 + a) * 32];
+      }
+      m = back[25 * 32];
+    }
+    if (!need) g2p_physics_affine<T>(sc, md, m, o);
+    w.out[0][j] = mk4(o.x[0], o.x[1], o.x[2], m);
     w.out[1][j] = mk4(o.F[0], o.F[1], o.F[2], o.F[3]);
     w.out[2][j] = mk4(o.F[4], o.F[5], o.F[6], o.F[7]);
     w.out[3][j] = mk4(o.F[8], o.J, a3.z, a3.w);
@@ -2004,9 +2097,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
     w.out[6][j] = mk4(o.C[5], o.C[6], o.C[7], o.C[8]);
     err = o.err;
     cl = o.clamped;
-    need = o.needs_clamp;
-    has = !need;  // the particles that need the clamp are scattered (and keyed) by its kernel
-    m = a0.w;
+    has = !need;  // the queued particles are scattered (and keyed) by the clamp kernel
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       xs[a] = o.x[a];
@@ -2033,8 +2124,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
 }
 
 // The snow return mapping of snow_clamp_kernel for the particles the fused kernel queued, each
-// then scattered into the next substep's accumulator with its final A.  A warp takes 32
-// consecutive queue entries (possibly of several scenes of a world).
+// then scattered into the next substep's accumulator with its final A.  A warp takes consecutive
+// queue entries (possibly of several scenes of a world): as many as spread the queue over all warps,
+// between 4 and 32, because scattered particles are runs of their own that a warp sums one after
+// another (a short queue took 16 us with 32 entries per warp).
 template <class T>
 __global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> w, int write_keys) {
   using V4 = typename V4T<T>::type;
@@ -2043,10 +2136,11 @@ __global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> 
   const WarpStage<T> st = warp_stage<T>(smem, threadIdx.x >> 5);
   V4* pre = st.col;  // position+mass, velocity+A of the queued particle: pre[k * 32 + lane], until the scatter
   const uint32_t count = launch_count(w.clamp_count);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < count; base += stride) {
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5), warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t per = min(32u, max(4u, (count + warps - 1) / warps));
+  for (uint32_t base = warp * per; base < count; base += warps * per) {
     const uint32_t i = base + lane;
-    const bool valid = i < count;
+    const bool valid = uint32_t(lane) < per && i < count;
     const uint2 q = valid ? w.clamp_queue[i] : make_uint2(0u, 0u);
     const SceneDev<T>& sc = w.scenes[q.y];
     T xs[3] = {0, 0, 0}, m = 0, mv[3] = {0, 0, 0}, A[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -2058,21 +2152,16 @@ __global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> 
       cp_async_commit();
       const V4 a1 = w.out[1][q.x], a2 = w.out[2][q.x], a3 = w.out[3][q.x];
       const MatDev& md = mat_of(w, sc, Bits<T>::unpack(a3.z) & 0xffffu);
-      const T F[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
-      const T lo = T(1) - T(md.theta_c), hi = T(1) + T(md.theta_s);
-      T U[9], sg[3], V[9];
-      const bool fb = svd3_fallback(F, U, sg, V, w.svd_fallback != 0, lo, hi);
-      T scl[3];
+      T nF[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x}, J = a3.y;
+      T* park = reinterpret_cast<T*>(pre + 128) + lane;
 #pragma unroll
-      for (int k = 0; k < 3; ++k) scl[k] = t_min(t_max(sg[k], lo), hi);
-      const T J = a3.y * ((sg[0] * sg[1] * sg[2]) / (scl[0] * scl[1] * scl[2]));
-      T nF[9];
+      for (int k = 0; k < 9; ++k) park[k * 32] = nF[k];
+      park[9 * 32] = J;
+      const bool fb = snow_return_parked<T>(&md, w.svd_fallback != 0, park);
+      const T volatile* back = park;
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          nF[r * 3 + c] = U[r * 3 + 0] * scl[0] * V[c * 3 + 0] + U[r * 3 + 1] * scl[1] * V[c * 3 + 1] +
-                          U[r * 3 + 2] * scl[2] * V[c * 3 + 2];
+      for (int k = 0; k < 9; ++k) nF[k] = back[k * 32];
+      J = back[9 * 32];
       w.out[1][q.x] = mk4(nF[0], nF[1], nF[2], nF[3]);
       w.out[2][q.x] = mk4(nF[4], nF[5], nF[6], nF[7]);
       w.out[3][q.x] = mk4(nF[8], J, a3.z, a3.w);
