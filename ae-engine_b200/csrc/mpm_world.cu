@@ -1621,13 +1621,18 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
   if (kTile) __syncthreads();
   uint32_t err = 0;
   bool cl = false, need = false;
+  const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
   if (live) {
     const T x0[3] = {a0.x, a0.y, a0.z};
     G2POut<T> o;
     T pv[3] = {0, 0, 0};
     if (MODE == AE_MPM_MODE_PHYSICS) {
-      const bool done = g2p_physics_gather_sep<T>(
-          GridRows<T>{w.vel, sc.blk_off, uint32_t(sc.nb[0]), uint32_t(sc.nb[1])}, sc, x0, pv, o.C);
+      bool done;
+      const GridRows<T> rows{w.vel, sc.blk_off, uint32_t(sc.nb[0]), uint32_t(sc.nb[1])};
+      if constexpr (sizeof(T) == 4)
+        done = g2p_physics_gather_sep_f2(rows, sc, x0, pv, o.C);
+      else
+        done = g2p_physics_gather_sep<T>(rows, sc, x0, pv, o.C);
       if (!done) g2p_physics_gather<T>(vt, sc, x0, pv, o.C);  // stencil partly outside the grid
     }
     cp_async_wait_all();
@@ -1662,12 +1667,20 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
     w.out[4][j] = mk4(o.v[0], o.v[1], o.v[2], o.C[0]);
     w.out[5][j] = mk4(o.C[1], o.C[2], o.C[3], o.C[4]);
     w.out[6][j] = mk4(o.C[5], o.C[6], o.C[7], o.C[8]);
-    // the next substep's cell key, only when the next substep sorts (the world tracks this)
-    if (write_keys) w.keys[j] = cell_key(sc, MODE, o.x[0], o.x[1], o.x[2]);
+    // the next substep's cell key, only when the next substep sorts (the world tracks this); with
+    // dense grouping counted in its cell too
+    if (write_keys) {
+      const uint32_t key = cell_key(sc, MODE, o.x[0], o.x[1], o.x[2]);
+      w.keys[j] = key;
+      if (w.bins) {
+        const uint32_t peers = __match_any_sync(live_mask, key);
+        if (lane == __ffs(peers) - 1) atomicAdd(w.bins + key, uint32_t(__popc(peers)));
+      }
+    }
     err = o.err;
     cl = o.clamped;
     need = o.needs_clamp;
-  } else if (j < ch.w && write_keys) {
+  } else if (j < ch.w && write_keys && !w.bins) {
     w.keys[j] = sc.dead_key;
   }
   // warp-aggregated error words, counters and clamp-queue appends
@@ -2195,6 +2208,10 @@ __global__ void discard_scatter_kernel(typename V4T<T>::type* acc, uint32_t* blk
   }
 }
 
+// dense grouping (bin_scan_kernel): nodes per scan CTA
+constexpr int kBinSeg = 4096;
+constexpr int kBinThreads = 256;
+
 // ============================================================================================
 // deterministic mode: per-cell fixed-order sums, per-node fixed-order gather
 // ============================================================================================
@@ -2271,8 +2288,16 @@ __global__ void __launch_bounds__(256) det_gather_kernel(WorldDev<T> w, uint32_t
         const int a = o % 3, b = (o / 3) % 3, c = o / 9;
         int X = i - a, Y = j - b, Z = k - c;
         if (X < 0 || Y < 0 || Z < 0) continue;
-        uint32_t s = w.cell_slot[node_index(sc, X, Y, Z)];
-        if (s == 0xffffffffu) continue;
+        const uint32_t ck = node_index(sc, X, Y, Z);
+        uint32_t s;
+        if (w.cells) {
+          const uint2 cell = w.cells[ck];
+          if (cell.y == 0u) continue;
+          s = cell.x + w.seg_off[ck / kBinSeg];
+        } else {
+          s = w.cell_slot[ck];
+          if (s == 0xffffffffu) continue;
+        }
         V4 r = w.cell_rec[uint64_t(s) * 27 + o];
         m += r.x;
         px += r.y;
@@ -2286,6 +2311,169 @@ __global__ void __launch_bounds__(256) det_gather_kernel(WorldDev<T> w, uint32_t
     if (l == 0) {
       w.blk_flag[gb] = 0u;
       blk_epoch[gb] = ep;
+    }
+  }
+}
+
+// ---- deterministic sums with dense grouping ----
+// After the grouping a cell's particles stand together but in no defined order.  The warp whose 32
+// sorted places hold a cell's first place puts them in slot order (as the stable radix sort does),
+// writes the final order and adds them up in it: lanes 0..26 are the 27 stencil nodes, every lane
+// adds its node's contributions particle by particle.  One thread per cell with 108 accumulators
+// (det_cellsum_kernel) left the chip to a few spilling warps: 211 us for 1 M particles at 8 per cell.
+//
+// Slot order: up to 32 particles rank each other by shuffles, up to kCellRankMax by comparing with
+// the whole cell; a larger cell (a collapsed scene) is collected in one pass over its scene's keys, so
+// that no cell costs the square of its size.
+constexpr uint32_t kCellRankMax = 512;
+
+template <class T>
+struct Wo {  // a weight and its node's offset from the particle
+  T w, o;
+};
+template <class T>
+struct PhysCellStage {
+  using V4 = typename V4T<T>::type;
+  V4 vm[32], a0[32], a1[32], a2[32];  // (m v, m), rows of A
+  Wo<T> wo[32 * 9];                   // wo[i * 9 + 3 axis + k]
+  int4 g[32];
+};
+template <class T, int MODE>
+struct CellStage {
+  P2GPart<T> p[32];
+};
+template <class T>
+struct CellStage<T, AE_MPM_MODE_PHYSICS> : PhysCellStage<T> {};
+
+template <class T>
+__device__ __forceinline__ void cell_stage_put(CellStage<T, AE_MPM_MODE_PHYSICS>& st, int i, const P2GPart<T>& p) {
+  st.vm[i] = mk4(p.v[0], p.v[1], p.v[2], p.m);
+  st.a0[i] = mk4(p.A[0], p.A[1], p.A[2], T(0));
+  st.a1[i] = mk4(p.A[3], p.A[4], p.A[5], T(0));
+  st.a2[i] = mk4(p.A[6], p.A[7], p.A[8], T(0));
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) st.wo[i * 9 + 3 * a + k] = Wo<T>{p.w[a][k], p.o[a][k]};
+  st.g[i] = make_int4(p.g[0], p.g[1], p.g[2], 0);
+}
+template <class T, int MODE>
+__device__ __forceinline__ void cell_stage_put(CellStage<T, MODE>& st, int i, const P2GPart<T>& p) {
+  st.p[i] = p;
+}
+// p2g_contrib of staged particle i at node offset (a, b, c); `inside`: every staged stencil is
+template <class T>
+__device__ __forceinline__ bool cell_contrib(const CellStage<T, AE_MPM_MODE_PHYSICS>& st, const SceneDev<T>& sc, int i,
+                                             int a, int b, int c, bool inside, T& cm, T& cx, T& cy, T& cz) {
+  if (!inside) {
+    const int4 g = st.g[i];
+    const int X = g.x + a, Y = g.y + b, Z = g.z + c;
+    if (X < 0 || Y < 0 || Z < 0 || X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) return false;
+  }
+  const Wo<T> x = st.wo[i * 9 + a], y = st.wo[i * 9 + 3 + b], z = st.wo[i * 9 + 6 + c];
+  const auto v = st.vm[i];
+  const auto r0 = st.a0[i], r1 = st.a1[i], r2 = st.a2[i];
+  const T ww = x.w * y.w * z.w;
+  cm = ww * v.w;
+  cx = ww * (v.x + r0.x * x.o + r0.y * y.o + r0.z * z.o);
+  cy = ww * (v.y + r1.x * x.o + r1.y * y.o + r1.z * z.o);
+  cz = ww * (v.z + r2.x * x.o + r2.y * y.o + r2.z * z.o);
+  return true;
+}
+template <class T, int MODE>
+__device__ __forceinline__ bool cell_contrib(const CellStage<T, MODE>& st, const SceneDev<T>& sc, int i, int a, int b,
+                                             int c, bool, T& cm, T& cx, T& cy, T& cz) {
+  return p2g_contrib<T, MODE>(sc, st.p[i], a, b, c, cm, cx, cy, cz);
+}
+
+template <class T, int MODE>
+__global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uint32_t* __restrict__ grouped,
+                                                        uint32_t* __restrict__ ordered) {
+  using V4 = typename V4T<T>::type;
+  extern __shared__ __align__(16) unsigned char smem[];
+  auto& st = reinterpret_cast<CellStage<T, MODE>*>(smem)[threadIdx.x >> 5];
+  const int4 ch = cta_chunk(w);
+  const SceneDev<T>& sc = w.scenes[ch.x];
+  const int lane = threadIdx.x & 31;
+  const uint32_t pos = uint32_t(ch.y) + threadIdx.x;
+  const bool live = int(pos) < ch.z;
+  const uint32_t key = live ? w.keys[grouped[pos]] : 0u;
+  uint32_t first = 0xffffffffu, cnt = 0;
+  if (live) {
+    const uint2 cell = w.cells[key];
+    first = cell.x + w.seg_off[key / kBinSeg];
+    cnt = cell.y;
+  }
+  const int na = lane % 3, nb = (lane / 3) % 3, nc = min(lane / 9, 2);
+  uint32_t heads = __ballot_sync(0xffffffffu, live && first == pos);
+  while (heads) {
+    const int h = __ffs(heads) - 1;
+    heads &= heads - 1u;
+    const uint32_t start = __shfl_sync(0xffffffffu, first, h), k = __shfl_sync(0xffffffffu, cnt, h);
+    const uint32_t ck = __shfl_sync(0xffffffffu, key, h);
+    const uint32_t* run = grouped + start;
+    uint32_t* out = ordered + start;
+    uint32_t slot = 0, rank = 0;
+    if (k <= 32u) {
+      slot = uint32_t(lane) < k ? run[lane] : 0xffffffffu;
+      for (uint32_t i = 0; i < k; ++i) rank += __shfl_sync(0xffffffffu, slot, int(i)) < slot ? 1u : 0u;
+      if (uint32_t(lane) < k) out[rank] = slot;
+    } else if (k <= kCellRankMax) {
+      for (uint32_t b0 = 0; b0 < k; b0 += 32) {
+        const uint32_t s = b0 + lane < k ? run[b0 + lane] : 0xffffffffu;
+        uint32_t r = 0;
+        for (uint32_t i = 0; i < k; ++i) r += run[i] < s ? 1u : 0u;
+        if (s != 0xffffffffu) out[r] = s;
+      }
+    } else {
+      uint32_t r = 0;
+      const uint32_t end = sc.p_off + sc.p_count;
+      for (uint32_t j0 = sc.p_off; j0 < end; j0 += 32) {
+        const bool hit = j0 + lane < end && w.keys[j0 + lane] == ck;
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        if (hit) out[r + __popc(m & ((1u << lane) - 1u))] = j0 + lane;
+        r += __popc(m);
+      }
+    }
+    __syncwarp();
+    if (ck == sc.dead_key) continue;  // off-grid particles of the reference modes: ordered, not summed
+    T am = T(0), ax = T(0), ay = T(0), az = T(0);
+    int g0 = 0, g1 = 0, g2 = 0;
+    for (uint32_t b0 = 0; b0 < k; b0 += 32) {
+      const uint32_t n = min(32u, k - b0);
+      bool in = true;
+      if (uint32_t(lane) < n) {
+        P2GPart<T> p;
+        if (k > 32u) {
+          slot = out[b0 + lane];
+          rank = uint32_t(lane);
+        }
+        p2g_setup<T, MODE>(w, sc, slot, p);
+        cell_stage_put(st, int(rank), p);
+        g0 = p.g[0], g1 = p.g[1], g2 = p.g[2];
+        in = g0 >= 0 && g1 >= 0 && g2 >= 0 && g0 + 2 < sc.n[0] && g1 + 2 < sc.n[1] && g2 + 2 < sc.n[2];
+      }
+      const bool inside = __all_sync(0xffffffffu, in);
+      __syncwarp();
+      for (uint32_t i = 0; i < n; ++i) {
+        T cm, cx, cy, cz;
+        if (cell_contrib(st, sc, int(i), na, nb, nc, inside, cm, cx, cy, cz)) {
+          am += cm;
+          ax += cx;
+          ay += cy;
+          az += cz;
+        }
+      }
+      __syncwarp();
+    }
+    if (lane < 27) w.cell_rec[uint64_t(start) * 27 + lane] = mk4(am, ax, ay, az);
+    // the cell's stencil spans at most two blocks per axis
+    g0 = __shfl_sync(0xffffffffu, g0, 0), g1 = __shfl_sync(0xffffffffu, g1, 0), g2 = __shfl_sync(0xffffffffu, g2, 0);
+    if (lane < 8) {
+      const int X = (lane & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
+      const int Y = (lane & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
+      const int Z = (lane & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
+      mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * sc.nb[1] + (Y >> 2)) * sc.nb[0] + (X >> 2));
     }
   }
 }
@@ -2338,8 +2526,6 @@ __global__ void init_keys_kernel(WorldDev<T> w) {
 // One CTA scans 4096 nodes (64 blocks) and zeroes the counts it read, so the array is clean for
 // the next count; offsets are written only where a count is not zero.  The CTA that finishes last
 // scans the segment totals (no CTA waits for another).
-constexpr int kBinSeg = 4096;
-constexpr int kBinThreads = 256;
 
 __device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
 #pragma unroll
@@ -2395,15 +2581,24 @@ __global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, ui
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    if (!any[r]) continue;
-    const uint64_t q = (base + r * 128 + lane * 4) >> 2;
+    const uint64_t i = base + r * 128 + lane * 4, q = i >> 2;
     uint4 o;
     o.x = off + ex[r];
     o.y = o.x + c[r].x + pad[r];
     o.z = o.y + c[r].y;
     o.w = o.z + c[r].z;
-    off4[q] = o;
-    bins4[q] = make_uint4(0u, 0u, 0u, 0u);
+    if (any[r]) {
+      off4[q] = o;
+      bins4[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (w.cells && i < nodes) {  // occupied now, or at the last sort
+      uint4* cq = reinterpret_cast<uint4*>(w.cells) + (i >> 1);
+      const uint4 a = cq[0], b = cq[1];
+      if (any[r] | a.y | a.w | b.y | b.w) {
+        cq[0] = make_uint4(o.x, c[r].x, o.y, c[r].y);
+        cq[1] = make_uint4(o.z, c[r].z, o.w, c[r].w);
+      }
+    }
   }
   if (tid == 0) {
     seg_total[blockIdx.x] = total;
@@ -2837,7 +3032,7 @@ class World final : public WorldBase {
     // Dense grouping reads every node's counter; the radix sort moves 20 bytes per key and pass.
     // The grid decides: up to 16 nodes per particle slot (or 8 M nodes, 5 us of scan) the dense
     // grouping wins, a huge grid with few particles in it keeps the radix sort.
-    dense_sort_ = !opts_.deterministic && blk * 64 <= 16 * cap + (uint64_t(8) << 20);
+    dense_sort_ = blk * 64 <= 16 * cap + (uint64_t(8) << 20);
     if (dense_sort_) {
       n_segs_ = uint32_t((blk * 64 + kBinSeg - 1) / kBinSeg);
       AE_TRY(dmalloc(&bins_, sizeof(uint32_t) * blk * 64));
@@ -2846,6 +3041,12 @@ class World final : public WorldBase {
       AE_TRY(dmalloc(&seg_, sizeof(uint32_t) * 2 * n_segs_));
       AE_TRY(dmalloc(&bin_perm_, sizeof(uint32_t) * pc));
       AE_TRY(cudaMemset(bin_perm_, 0, sizeof(uint32_t) * pc));
+      if (opts_.deterministic) {
+        AE_TRY(dmalloc(&cells_, sizeof(uint2) * blk * 64));
+        AE_TRY(cudaMemset(cells_, 0, sizeof(uint2) * blk * 64));
+        AE_TRY(dmalloc(&ordered_, sizeof(uint32_t) * pc));
+        AE_TRY(cudaMemset(ordered_, 0, sizeof(uint32_t) * pc));
+      }
     } else {
       AE_TRY(sort_scratch_alloc(sort_, pc, alloc_ ? &World::sort_alloc : nullptr, alloc_));
     }
@@ -2868,9 +3069,11 @@ class World final : public WorldBase {
     AE_TRY(dmalloc(&err_, sizeof(uint32_t) * 4 * n));
     AE_TRY(cudaMemset(err_, 0, sizeof(uint32_t) * 4 * n));
     if (opts_.deterministic) {
-      AE_TRY(dmalloc(&cell_slot_, sizeof(uint32_t) * nodes));
-      AE_TRY(cudaMemset(cell_slot_, 0xff, sizeof(uint32_t) * nodes));
-      AE_TRY(dmalloc(&seg_start_, sizeof(uint32_t) * pc));
+      if (!dense_sort_) {
+        AE_TRY(dmalloc(&cell_slot_, sizeof(uint32_t) * nodes));
+        AE_TRY(cudaMemset(cell_slot_, 0xff, sizeof(uint32_t) * nodes));
+        AE_TRY(dmalloc(&seg_start_, sizeof(uint32_t) * pc));
+      }
       AE_TRY(dmalloc(&cell_rec_, sizeof(V4) * 27 * pc));
     }
     return AE_MPM_OK;
@@ -3751,6 +3954,7 @@ class World final : public WorldBase {
     w.bins = bins_;
     w.bin_off = bin_off_;
     w.seg_off = seg_ ? seg_ + n_segs_ : nullptr;
+    w.cells = cells_;
     w.acc = acc_;
     w.vel = vel_;
     w.blk_flag = blk_flag_;
@@ -3821,7 +4025,18 @@ class World final : public WorldBase {
   template <int MODE>
   void substep_mode(WorldDev<T>& w, bool write_keys) {
     const int sms = device_sm_count();
-    if (opts_.deterministic) {
+    if (opts_.deterministic && dense_sort_) {
+      const size_t sm = sizeof(CellStage<T, MODE>) * size_t(chunk_threads_ / 32);
+      if (!det_smem_set_) {  // sized for the largest block (256 threads) the world accepts
+        cudaFuncSetAttribute(det_cells_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(sizeof(CellStage<T, MODE>) * 8));
+        det_smem_set_ = true;
+      }
+      det_cells_kernel<T, MODE><<<n_chunks_, chunk_threads_, sm, stream_>>>(w, bin_perm_, ordered_);
+      det_gather_kernel<T, MODE><<<sms * 8, 256, 0, stream_>>>(w, blk_epoch_, counters_ + 2);
+      mark(2);
+      launches_ += 2;
+    } else if (opts_.deterministic) {
       det_heads_kernel<<<unsigned((total_cap_ + 255) / 256), 256, 0, stream_>>>(w.sorted_keys, total_cap_, dead_blk_,
                                                                                  cell_slot_, seg_start_, counters_ + 1);
       det_cellsum_kernel<T, MODE><<<sms * 8, 128, 0, stream_>>>(w, total_cap_);
@@ -3979,7 +4194,8 @@ class World final : public WorldBase {
       WorldDev<T> w = dev(false);
       bin_scan_kernel<T><<<n_segs_, kBinThreads, 0, stream_>>>(w, total_blocks_ * 64, dead_blk_, seg_, counters_ + 5);
       bin_scatter_kernel<T><<<n_chunks_, chunk_threads_, 0, stream_>>>(w, bin_perm_, uint32_t(total_cap_));
-      perm_ = bin_perm_;
+      // a deterministic substep orders each cell (det_cells_kernel) before anything reads the order
+      perm_ = opts_.deterministic ? ordered_ : bin_perm_;
       launches_ += 2;
     } else {
       launches_ += radix_sort_pairs(keys_, total_cap_, key_bits_, sort_, stream_, &sorted_keys_, &perm_);
@@ -3992,7 +4208,7 @@ class World final : public WorldBase {
     // the keys of the next sort are written by the G2P just before it; a sort without them (first
     // substep, changed interval) computes them first.  Only the fused G2P counts cells too.
     const uint32_t next = phase_ + 1 >= sort_interval() ? 0u : phase_ + 1;
-    const bool write_keys = next == 0 && (!dense_sort_ || fused());
+    const bool write_keys = next == 0 && (!dense_sort_ || fused() || opts_.deterministic);
     if (n_chunks_ > 0) {
       mark(0);
       if (phase_ == 0 && !sorted_) sort_particles();
@@ -4075,6 +4291,8 @@ class World final : public WorldBase {
     dfree(bin_off_);
     dfree(seg_);
     dfree(bin_perm_);
+    dfree(cells_);
+    dfree(ordered_);
     dfree(acc_);
     dfree(vel_);
     dfree(blk_flag_);
@@ -4121,6 +4339,8 @@ class World final : public WorldBase {
   SortScratch sort_;
   bool dense_sort_ = false;  // particles are grouped by counting (bins_), not by the radix sort
   uint32_t *bins_ = nullptr, *bin_off_ = nullptr, *seg_ = nullptr, *bin_perm_ = nullptr;
+  uint2* cells_ = nullptr;        // deterministic dense grouping: each cell's places
+  uint32_t* ordered_ = nullptr;   // ... and the sorted places in slot order within each cell
   uint32_t n_segs_ = 0;
   const uint32_t* perm_ = nullptr;
   const uint32_t* sorted_keys_ = nullptr;
@@ -4148,7 +4368,7 @@ class World final : public WorldBase {
     bool a_in = true;
   };
   Graph graphs_[2];  // by the parity of the period's first substep
-  bool lanes_smem_set_ = false, fused_smem_set_ = false, ref_lanes_smem_set_ = false;
+  bool lanes_smem_set_ = false, fused_smem_set_ = false, ref_lanes_smem_set_ = false, det_smem_set_ = false;
   bool scatter_pending_ = false;  // the accumulator holds the P2G of the current particle state
   bool scatter_invalid_ = false;  // the particles changed since that scatter
   std::vector<uint32_t> late_slots_;  // slots assigned into a queued scatter, not scattered themselves yet

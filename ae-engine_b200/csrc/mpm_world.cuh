@@ -69,6 +69,9 @@ struct WorldDev {
   uint32_t* bins;
   uint32_t* bin_off;
   uint32_t* seg_off;
+  // deterministic worlds with dense grouping, per node: {first sorted place within its scan segment,
+  // particles} of the cell based there
+  uint2* cells;
   V4* acc;
   V4* vel;
   uint32_t* blk_flag;

@@ -95,3 +95,55 @@ def test_off_grid_particles_of_the_reference_modes_match_the_oracle(ctx, n):
     ctx.step_velocity_only_parallel(a, grid, cfg, 0.1, idx)
     assert O.step_velocity_only_parallel(b, grid, cfg, 0.1, idx) == 0
     assert rel(a.pos, b.pos) <= 2e-5
+
+
+@pytest.mark.parametrize("sizes", [(1, 31, 32, 33), (512, 64, 2), (513, 700, 40), (3000, 5)])
+def test_deterministic_sums_over_crowded_cells(ctx, sizes):
+    # cells of up to 32 particles, up to the rank limit and above it: the slot order of each cell, and
+    # with it every bit, repeats from run to run whatever order the grouping's atomics gave
+    rng = np.random.default_rng(sum(sizes))
+    g, dx = 16, 1.0 / 16
+    x = np.concatenate([(np.array([4.6 + 1.5 * i, 5.6, 6.6]) + 0.8 * rng.random((k, 3))) * dx
+                        for i, k in enumerate(sizes)])
+    x = x[rng.permutation(len(x))]
+    p = S.make_particles(x, (0.3, -0.2, 0.1), 1e-5, 0)
+    p.J[:] = 1.0
+    sc = M.Scene(n=(g, g, g), dx=dx, dt=1e-4, materials=[S.jelly(E=100.0)], max_particles=p.n + 9)
+    ref = p.astype(np.float64)
+    O.run(sc, ref, 7)
+    runs = []
+    for graph in (0, 1, 1):
+        w = M.World(ctx, [sc], M.exec_opts(deterministic=1, use_graph=graph))
+        w.upload(0, p)
+        w.step(7)
+        w.sync(raise_on_error=False)
+        runs.append(w.download(0, p.n))
+        w.close()
+    assert rel(runs[0].pos, ref.pos) <= 1e-5
+    for r in runs[1:]:
+        for f in ("pos", "vel", "F", "J", "C"):
+            assert np.array_equal(getattr(r, f), getattr(runs[0], f)), f
+
+
+@pytest.mark.parametrize("mode", [M.MODE_REFERENCE, M.MODE_VELOCITY_ONLY])
+def test_deterministic_reference_modes_with_off_grid_particles_repeat(ctx, mode):
+    rng = np.random.default_rng(7)
+    g, dx, n = 20, 0.5, 3001
+    p = M.Particles.empty(n)
+    p.pos[:] = rng.random((n, 3)) * (g + 2) * dx  # some beyond the upper faces
+    p.vel[:] = rng.normal(0, 0.3, (n, 3))
+    p.mass[:] = 0.01
+    p.J[:] = 1.0
+    sc = M.Scene(n=(g, g, g), dx=dx, dt=0.01, materials=[M.material(young_modulus=1e4, poisson_ratio=0.25)], mode=mode,
+                 gravity=(0, -9.81, 0), max_particles=n + 100)
+    out = []
+    for det in (1, 1, 0):
+        w = M.World(ctx, [sc], M.exec_opts(deterministic=det))
+        w.upload(0, p)
+        w.step(5)
+        w.sync(raise_on_error=False)
+        out.append(w.download(0, n))
+        w.close()
+    for f in ("pos", "vel", "F", "J", "C"):
+        assert np.array_equal(getattr(out[0], f), getattr(out[1], f)), f
+    assert rel(out[0].pos, out[2].pos) <= 2e-5
