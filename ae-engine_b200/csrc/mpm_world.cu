@@ -2327,63 +2327,73 @@ __global__ void __launch_bounds__(256) det_gather_kernel(WorldDev<T> w, uint32_t
 // that no cell costs the square of its size.
 constexpr uint32_t kCellRankMax = 512;
 
-template <class T>
-struct Wo {  // a weight and its node's offset from the particle
-  T w, o;
-};
-template <class T>
-struct PhysCellStage {
-  using V4 = typename V4T<T>::type;
-  V4 vm[32], a0[32], a1[32], a2[32];  // (m v, m), rows of A
-  Wo<T> wo[32 * 9];                   // wo[i * 9 + 3 axis + k]
-  int4 g[32];
-};
+// Physics mode stages what the column-lane scatter stages: per (y,z) column u = m v + A d and w_y w_z,
+// the x weights with the mass, dx times A's x column (3 shared loads per particle and node; weights,
+// offsets and A's rows staged as they are took 7, and the kernel was bound by shared memory: 95 us
+// against 88 for 1 M particles).
 template <class T, int MODE>
 struct CellStage {
   P2GPart<T> p[32];
 };
 template <class T>
-struct CellStage<T, AE_MPM_MODE_PHYSICS> : PhysCellStage<T> {};
+struct CellStage<T, AE_MPM_MODE_PHYSICS> {
+  using V4 = typename V4T<T>::type;
+  V4 col[32 * 9], wxm[32], acol[32];
+  int4 g[32];
+};
 
 template <class T>
-__device__ __forceinline__ void cell_stage_put(CellStage<T, AE_MPM_MODE_PHYSICS>& st, int i, const P2GPart<T>& p) {
-  st.vm[i] = mk4(p.v[0], p.v[1], p.v[2], p.m);
-  st.a0[i] = mk4(p.A[0], p.A[1], p.A[2], T(0));
-  st.a1[i] = mk4(p.A[3], p.A[4], p.A[5], T(0));
-  st.a2[i] = mk4(p.A[6], p.A[7], p.A[8], T(0));
+__device__ __forceinline__ void cell_stage_put(CellStage<T, AE_MPM_MODE_PHYSICS>& st, const SceneDev<T>& sc, int i,
+                                               const P2GPart<T>& p) {
+  const T dx = sc.dx;
+  T c0[3], c1[3], c2[3], qv[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+  for (int r = 0; r < 3; ++r) {
+    c0[r] = dx * p.A[3 * r + 0];
+    c1[r] = dx * p.A[3 * r + 1];
+    c2[r] = dx * p.A[3 * r + 2];
+    qv[r] = p.v[r] - (c0[r] * p.fx[0] + c1[r] * p.fx[1] + c2[r] * p.fx[2]);
+  }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) st.wo[i * 9 + 3 * a + k] = Wo<T>{p.w[a][k], p.o[a][k]};
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      st.col[i * 9 + b + 3 * c] = mk4(qv[0] + T(b) * c1[0] + T(c) * c2[0], qv[1] + T(b) * c1[1] + T(c) * c2[1],
+                                      qv[2] + T(b) * c1[2] + T(c) * c2[2], p.w[1][b] * p.w[2][c]);
+  st.wxm[i] = mk4(p.w[0][0], p.w[0][1], p.w[0][2], p.m);
+  st.acol[i] = mk4(c0[0], c0[1], c0[2], T(0));
   st.g[i] = make_int4(p.g[0], p.g[1], p.g[2], 0);
 }
 template <class T, int MODE>
-__device__ __forceinline__ void cell_stage_put(CellStage<T, MODE>& st, int i, const P2GPart<T>& p) {
+__device__ __forceinline__ void cell_stage_put(CellStage<T, MODE>& st, const SceneDev<T>&, int i, const P2GPart<T>& p) {
   st.p[i] = p;
 }
-// p2g_contrib of staged particle i at node offset (a, b, c); `inside`: every staged stencil is
+// adds staged particle i's contribution to the node at offset (a, b, c); `inside`: every staged
+// stencil lies in the grid
 template <class T>
-__device__ __forceinline__ bool cell_contrib(const CellStage<T, AE_MPM_MODE_PHYSICS>& st, const SceneDev<T>& sc, int i,
-                                             int a, int b, int c, bool inside, T& cm, T& cx, T& cy, T& cz) {
+__device__ __forceinline__ void cell_add(const CellStage<T, AE_MPM_MODE_PHYSICS>& st, const SceneDev<T>& sc, int i,
+                                         int a, int b, int c, bool inside, T& am, T& ax, T& ay, T& az) {
   if (!inside) {
     const int4 g = st.g[i];
     const int X = g.x + a, Y = g.y + b, Z = g.z + c;
-    if (X < 0 || Y < 0 || Z < 0 || X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) return false;
+    if (X < 0 || Y < 0 || Z < 0 || X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) return;
   }
-  const Wo<T> x = st.wo[i * 9 + a], y = st.wo[i * 9 + 3 + b], z = st.wo[i * 9 + 6 + c];
-  const auto v = st.vm[i];
-  const auto r0 = st.a0[i], r1 = st.a1[i], r2 = st.a2[i];
-  const T ww = x.w * y.w * z.w;
-  cm = ww * v.w;
-  cx = ww * (v.x + r0.x * x.o + r0.y * y.o + r0.z * z.o);
-  cy = ww * (v.y + r1.x * x.o + r1.y * y.o + r1.z * z.o);
-  cz = ww * (v.z + r2.x * x.o + r2.y * y.o + r2.z * z.o);
-  return true;
+  const auto u = st.col[i * 9 + b + 3 * c], r = st.wxm[i], s = st.acol[i];
+  const T fa = T(a), ww = (a == 0 ? r.x : (a == 1 ? r.y : r.z)) * u.w;
+  am += ww * r.w;
+  ax += ww * (u.x + fa * s.x);
+  ay += ww * (u.y + fa * s.y);
+  az += ww * (u.z + fa * s.z);
 }
 template <class T, int MODE>
-__device__ __forceinline__ bool cell_contrib(const CellStage<T, MODE>& st, const SceneDev<T>& sc, int i, int a, int b,
-                                             int c, bool, T& cm, T& cx, T& cy, T& cz) {
-  return p2g_contrib<T, MODE>(sc, st.p[i], a, b, c, cm, cx, cy, cz);
+__device__ __forceinline__ void cell_add(const CellStage<T, MODE>& st, const SceneDev<T>& sc, int i, int a, int b, int c,
+                                         bool, T& am, T& ax, T& ay, T& az) {
+  T cm, cx, cy, cz;
+  if (!p2g_contrib<T, MODE>(sc, st.p[i], a, b, c, cm, cx, cy, cz)) return;
+  am += cm;
+  ax += cx;
+  ay += cy;
+  az += cz;
 }
 
 template <class T, int MODE>
@@ -2405,7 +2415,65 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
     cnt = cell.y;
   }
   const int na = lane % 3, nb = (lane / 3) % 3, nc = min(lane / 9, 2);
+  T am, ax, ay, az;
+  auto add_staged = [&](int i0, int i1, bool inside) {  // staged particles in order, this lane's node
+    for (int i = i0; i < i1; ++i) cell_add(st, sc, i, na, nb, nc, inside, am, ax, ay, az);
+  };
+  auto finish = [&](uint32_t start, int g0, int g1, int g2) {
+    if (lane < 27) w.cell_rec[uint64_t(start) * 27 + lane] = mk4(am, ax, ay, az);
+    if (lane < 8) {  // the cell's stencil spans at most two blocks per axis
+      const int X = (lane & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
+      const int Y = (lane & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
+      const int Z = (lane & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
+      mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * sc.nb[1] + (Y >> 2)) * sc.nb[0] + (X >> 2));
+    }
+  };
+  auto inside_grid = [&](const P2GPart<T>& p) {
+    return p.g[0] >= 0 && p.g[1] >= 0 && p.g[2] >= 0 && p.g[0] + 2 < sc.n[0] && p.g[1] + 2 < sc.n[1] &&
+           p.g[2] + 2 < sc.n[2];
+  };
   uint32_t heads = __ballot_sync(0xffffffffu, live && first == pos);
+  const uint32_t base = pos - lane;
+
+  // cells that lie in the warp's 32 places: ordered and staged together, one particle per lane
+  const bool batch = live && first >= base && first + cnt <= base + 32u;
+  const uint32_t in_batch = __ballot_sync(0xffffffffu, batch);
+  if (in_batch) {
+    const uint32_t mine = live ? grouped[pos] : 0u;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, batch ? cnt : 0u);
+    const int l0 = batch ? int(first - base) : 0;
+    uint32_t rank = 0;
+    for (uint32_t t = 0; t < most; ++t) {
+      const uint32_t other = __shfl_sync(0xffffffffu, mine, (l0 + int(t)) & 31);
+      if (t < cnt && other < mine) ++rank;
+    }
+    P2GPart<T> p;
+    p.g[0] = p.g[1] = p.g[2] = 0;
+    bool in = true;
+    if (batch) {
+      ordered[first + rank] = mine;
+      if (key != sc.dead_key) {
+        p2g_setup<T, MODE>(w, sc, mine, p);
+        cell_stage_put(st, sc, l0 + int(rank), p);
+        in = inside_grid(p);
+      }
+    }
+    const bool inside = __all_sync(0xffffffffu, in);
+    __syncwarp();
+    for (uint32_t todo = heads & in_batch; todo; todo &= todo - 1u) {
+      const int h = __ffs(todo) - 1;
+      if (__shfl_sync(0xffffffffu, key, h) == sc.dead_key) continue;
+      const int k = int(__shfl_sync(0xffffffffu, cnt, h));
+      am = ax = ay = az = T(0);
+      add_staged(h, h + k, inside);
+      finish(base + uint32_t(h), __shfl_sync(0xffffffffu, p.g[0], h), __shfl_sync(0xffffffffu, p.g[1], h),
+             __shfl_sync(0xffffffffu, p.g[2], h));
+    }
+    heads &= ~in_batch;
+    __syncwarp();
+  }
+
+  // the others one by one: the cell that runs past the places, or cells of more than 32 particles
   while (heads) {
     const int h = __ffs(heads) - 1;
     heads &= heads - 1u;
@@ -2437,7 +2505,7 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
     }
     __syncwarp();
     if (ck == sc.dead_key) continue;  // off-grid particles of the reference modes: ordered, not summed
-    T am = T(0), ax = T(0), ay = T(0), az = T(0);
+    am = ax = ay = az = T(0);
     int g0 = 0, g1 = 0, g2 = 0;
     for (uint32_t b0 = 0; b0 < k; b0 += 32) {
       const uint32_t n = min(32u, k - b0);
@@ -2449,32 +2517,16 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
           rank = uint32_t(lane);
         }
         p2g_setup<T, MODE>(w, sc, slot, p);
-        cell_stage_put(st, int(rank), p);
+        cell_stage_put(st, sc, int(rank), p);
         g0 = p.g[0], g1 = p.g[1], g2 = p.g[2];
-        in = g0 >= 0 && g1 >= 0 && g2 >= 0 && g0 + 2 < sc.n[0] && g1 + 2 < sc.n[1] && g2 + 2 < sc.n[2];
+        in = inside_grid(p);
       }
       const bool inside = __all_sync(0xffffffffu, in);
       __syncwarp();
-      for (uint32_t i = 0; i < n; ++i) {
-        T cm, cx, cy, cz;
-        if (cell_contrib(st, sc, int(i), na, nb, nc, inside, cm, cx, cy, cz)) {
-          am += cm;
-          ax += cx;
-          ay += cy;
-          az += cz;
-        }
-      }
+      add_staged(0, int(n), inside);
       __syncwarp();
     }
-    if (lane < 27) w.cell_rec[uint64_t(start) * 27 + lane] = mk4(am, ax, ay, az);
-    // the cell's stencil spans at most two blocks per axis
-    g0 = __shfl_sync(0xffffffffu, g0, 0), g1 = __shfl_sync(0xffffffffu, g1, 0), g2 = __shfl_sync(0xffffffffu, g2, 0);
-    if (lane < 8) {
-      const int X = (lane & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
-      const int Y = (lane & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
-      const int Z = (lane & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
-      mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * sc.nb[1] + (Y >> 2)) * sc.nb[0] + (X >> 2));
-    }
+    finish(start, __shfl_sync(0xffffffffu, g0, 0), __shfl_sync(0xffffffffu, g1, 0), __shfl_sync(0xffffffffu, g2, 0));
   }
 }
 
