@@ -8,7 +8,7 @@
 // Here:
 //   * the force pass is fused into P2G: both depend on the particle state alone, so one read of a
 //     particle scatters mass, momentum and force into two 16-byte accumulators per node;
-//   * G2P of step s and P2G of step s+1 are one kernel (ck_particles_kernel<true, true>): each
+//   * G2P of step s and P2G of step s+1 are one kernel (ck_particles_kernel): each
 //     particle record is read and written once per step;
 //   * P2G flags the 4x4x4 node blocks it touches with plain stores (nothing waits on them); a
 //     sweep compacts the flags into a list, and the grid update visits only the listed blocks,
@@ -34,11 +34,14 @@
 #include <vector>
 
 #include "ae_mpm_ck.cuh"
+#include "mpm_world.cuh"
 
 namespace aemp {
 namespace {
 
-constexpr int kCkThreads = 256;     // particles per CTA
+constexpr int kCkThreads = 256;     // particles per CTA of the scatter kernels
+constexpr int kCkWarps = 4;         // gather kernel: warps per CTA, each with its own records in flight
+constexpr int kCkCtas = 6;          // ... and CTAs per SM (80 registers)
 constexpr int kRecFloats = 26;      // ae_mpm_ck_particle
 constexpr int kGridThreads = 256;   // 4 node blocks per CTA in the grid update
 
@@ -126,7 +129,8 @@ struct CkArgs {
   uint32_t* next_count;  // the counter the next step's compaction appends to
   int gn, nb;
   Spacing sp;
-  float h, dt, youngs, poisson, restitution;
+  float h, dt, restitution;
+  float mu, lambda, d_inv;  // formed on the host with the reference's f32 operations
   float g[3], bmin[3], bmax[3];
   int aligned16;
 };
@@ -136,6 +140,11 @@ __device__ __forceinline__ uint32_t node_index(int i, int j, int k, int nb) {
   const uint32_t b = (uint32_t(k >> 2) * uint32_t(nb) + uint32_t(j >> 2)) * uint32_t(nb) + uint32_t(i >> 2);
   return b * 64u + uint32_t((k & 3) * 16 + (j & 3) * 4 + (i & 3));
 }
+
+// node_index as a sum of one part per axis (the bit fields are disjoint)
+struct NodeParts {
+  uint32_t p[3][2];
+};
 
 // The 2 nodes per axis around a particle (i = floor(x / h) + {0, 1}, node at (i + 1/2) h):
 // whether each exists, its offset from the particle and its kernel weight and gradient.
@@ -175,6 +184,17 @@ __device__ __forceinline__ void make_stencil(Stencil& st, V3 pos, const Spacing&
     for (int d = 0; d < 2; ++d) st.zero[a][d] = st.zero[a][d] && fin;
 }
 
+__device__ __forceinline__ NodeParts node_parts(const Stencil& st, int nb) {
+  NodeParts q;
+  const uint32_t pitch[3] = {64u, 64u * uint32_t(nb), 64u * uint32_t(nb) * uint32_t(nb)};
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int d = 0; d < 2; ++d)
+      q.p[a][d] = uint32_t(st.i[a][d] >> 2) * pitch[a] + (uint32_t(st.i[a][d] & 3) << (2 * a));
+  return q;
+}
+
 // whether node (di, dj, dk) of the stencil exists and can contribute
 __device__ __forceinline__ bool live(const Stencil& st, int di, int dj, int dk) {
   return st.ok[0][di] && st.ok[1][dj] && st.ok[2][dk] && !(st.zero[0][di] || st.zero[1][dj] || st.zero[2][dk]);
@@ -199,12 +219,10 @@ __device__ __forceinline__ void mark_block(const CkArgs& a, uint32_t b, uint32_t
 
 // The first Piola stress of the force pass (:262-268): P = mu (F - F^-T) + lambda ln(max(det F, 1e-10)) F^-T
 __device__ __forceinline__ M3 piola_stress(const CkArgs& a, const M3& F) {
-  const float mu = a.youngs / (2.0f * (1.0f + a.poisson));
-  const float lambda = a.youngs * a.poisson / ((1.0f + a.poisson) * (1.0f - 2.0f * a.poisson));
   const float fdet = fmaxf(detm(F), 1e-10f);
   const M3 fit = inversem(transposem(F));
   const float ln_j = float(log(double(fdet)));
-  return addm(scalem(subm(F, fit), mu), scalem(fit, lambda * ln_j));
+  return addm(scalem(subm(F, fit), a.mu), scalem(fit, a.lambda * ln_j));
 }
 
 // One particle's contribution to one node (:221-240 and :276-318): wm = w m to the mass, (v + B d) wm
@@ -228,6 +246,7 @@ __device__ __forceinline__ void scatter(const CkArgs& a, V3 pos, V3 vel, const M
                                         float mass) {
   Stencil st;
   make_stencil<POW2>(st, pos, a.sp, a.gn, true);
+  const NodeParts np = node_parts(st, a.nb);
   const M3 P = piola_stress(a, F);
   const float coeff = -rest_volume;
   uint32_t last = 0xffffffffu;
@@ -243,7 +262,7 @@ __device__ __forceinline__ void scatter(const CkArgs& a, V3 pos, V3 vel, const M
         V3 mom, force;
         node_contribution(st.w[0][di], st.w[1][dj], st.w[2][dk], st.gw[0][di], st.gw[1][dj], st.gw[2][dk], diff, vel, B,
                           P, mass, coeff, wm, mom, force);
-        const uint32_t node = node_index(st.i[0][di], st.i[1][dj], st.i[2][dk], a.nb);
+        const uint32_t node = np.p[0][di] + np.p[1][dj] + np.p[2][dk];
         atomicAdd(a.acc + 2 * node, make_float4(mom.x, mom.y, mom.z, wm));
         atomicAdd(a.acc + 2 * node + 1, make_float4(force.x, force.y, force.z, 0.0f));
         mark_block(a, node >> 6, last);
@@ -272,16 +291,17 @@ __device__ __forceinline__ void reflect_axis(float& v, float node_pos, float lo,
 // G2P (:365-459) and the particle bounds (:462-478) of one particle
 template <bool POW2>
 __device__ __forceinline__ void gather_update(const CkArgs& a, V3& pos, V3& vel, M3& B, M3& F) {
-  const float h = a.h, dt = a.dt;
+  const float dt = a.dt;
   Stencil st;
   make_stencil<POW2>(st, pos, a.sp, a.gn, false);
-  const float d_inv = 4.0f / (h * h);
+  const float d_inv = a.d_inv;
+  const NodeParts idx = node_parts(st, a.nb);
   // all eight node loads first, so their latencies overlap
   float4 vnode[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int di = q & 1, dj = (q >> 1) & 1, dk = q >> 2;
-    vnode[q] = live(st, di, dj, dk) ? __ldg(a.vel + node_index(st.i[0][di], st.i[1][dj], st.i[2][dk], a.nb))
+    vnode[q] = live(st, di, dj, dk) ? __ldg(a.vel + (idx.p[0][di] + idx.p[1][dj] + idx.p[2][dk]))
                                     : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   V3 nv{0.0f, 0.0f, 0.0f};
@@ -324,9 +344,80 @@ __device__ __forceinline__ void gather_update(const CkArgs& a, V3& pos, V3& vel,
   clamp_axis(pos.z, vel.z, a.bmin[2], a.bmax[2], a.restitution);
 }
 
-// One CTA = 256 consecutive particles.  G2P: gather from a.vel and update the record in place.
-// P2G: scatter the (updated) particle into a.acc for the next grid update.
-template <bool G2P, bool P2G, bool POW2>
+// asynchronous global -> shared copies of a warp's 32 records: 16 bytes at a time where the caller's
+// array starts on a 16-byte boundary (a group of 32 records is 3328 bytes), 4 otherwise
+__device__ __forceinline__ void copy_async(void* sdst, const void* gsrc, bool wide) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+  if (wide)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void fetch_records(float* dst, const CkArgs& a, uint64_t group, int lane) {
+  const uint64_t base = group * 32;
+  if (base < a.n) {
+    const int nf = int(a.n - base < 32 ? a.n - base : 32) * kRecFloats;
+    const float* g = a.rec + base * kRecFloats;
+    const int wide = a.aligned16 ? nf / 4 : 0;
+    for (int q = lane; q < wide; q += 32) copy_async(dst + 4 * q, g + 4 * q, true);
+    for (int q = 4 * wide + lane; q < nf; q += 32) copy_async(dst + q, g + q, false);
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// G2P alone (the last step of a call, every deterministic step): gather from a.vel and update the
+// record in place.  Persistent: every warp walks over groups of 32 records, each group fetched while
+// the one before it is computed, without block barriers (78 us for 2 M particles; a CTA that loaded,
+// computed and stored its 256 records in turn took 116).
+template <bool POW2>
+__global__ void __launch_bounds__(32 * kCkWarps, kCkCtas) ck_gather_kernel(CkArgs a) {
+  __shared__ __align__(16) float srec[kCkWarps][2][32 * kRecFloats];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const uint64_t groups = (a.n + 31) / 32, stride = uint64_t(gridDim.x) * kCkWarps;
+  uint64_t t = uint64_t(blockIdx.x) * kCkWarps + wi;
+  if (t >= groups) return;
+  fetch_records(srec[wi][0], a, t, lane);
+  for (int buf = 0; t < groups; t += stride, buf ^= 1) {
+    fetch_records(srec[wi][buf ^ 1], a, t + stride, lane);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncwarp();
+    float* rows = srec[wi][buf];
+    const uint64_t base = t * 32;
+    const int cnt = int(a.n - base < 32 ? a.n - base : 32);
+    if (lane < cnt) {
+      float2* r = reinterpret_cast<float2*>(rows + lane * kRecFloats);  // 104-byte rows
+      float f[24];
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        const float2 q = r[k];
+        f[2 * k] = q.x;
+        f[2 * k + 1] = q.y;
+      }
+      V3 pos{f[0], f[1], f[2]}, vel{f[3], f[4], f[5]};
+      M3 B{{f[6], f[7], f[8]}, {f[9], f[10], f[11]}, {f[12], f[13], f[14]}};
+      M3 F{{f[15], f[16], f[17]}, {f[18], f[19], f[20]}, {f[21], f[22], f[23]}};
+      gather_update<POW2>(a, pos, vel, B, F);
+      r[0] = make_float2(pos.x, pos.y), r[1] = make_float2(pos.z, vel.x), r[2] = make_float2(vel.y, vel.z);
+      r[3] = make_float2(B.c0.x, B.c0.y), r[4] = make_float2(B.c0.z, B.c1.x), r[5] = make_float2(B.c1.y, B.c1.z);
+      r[6] = make_float2(B.c2.x, B.c2.y), r[7] = make_float2(B.c2.z, F.c0.x), r[8] = make_float2(F.c0.y, F.c0.z);
+      r[9] = make_float2(F.c1.x, F.c1.y), r[10] = make_float2(F.c1.z, F.c2.x), r[11] = make_float2(F.c2.y, F.c2.z);
+    }
+    __syncwarp();
+    float* g = a.rec + base * kRecFloats;
+    const int nf = cnt * kRecFloats, wide = a.aligned16 ? nf / 4 : 0;
+    for (int q = lane; q < wide; q += 32)
+      __stcs(reinterpret_cast<float4*>(g) + q, reinterpret_cast<const float4*>(rows)[q]);
+    for (int q = 4 * wide + lane; q < nf; q += 32) g[q] = rows[q];
+    __syncwarp();  // the buffer is free for the group after the next
+  }
+}
+
+// P2G, with G2P: the particle's G2P first.  One CTA = 256 consecutive particles: gather from a.vel and
+// update the record in place, scatter the (updated) particle into a.acc for the next grid update.
+// Bound by the node reductions and instruction issue together (170 us for 2 M particles); with
+// records fetched ahead per warp as in ck_gather_kernel it takes 179 to 187, with contributions of
+// neighbouring lanes to a node added up before they leave the warp 232.
+template <bool G2P, bool POW2>
 __global__ void __launch_bounds__(kCkThreads, 3) ck_particles_kernel(CkArgs a) {
   __shared__ __align__(16) float srec[kCkThreads * kRecFloats];
   const uint64_t base = uint64_t(blockIdx.x) * kCkThreads;
@@ -359,7 +450,7 @@ __global__ void __launch_bounds__(kCkThreads, 3) ck_particles_kernel(CkArgs a) {
       r[15] = F.c0.x, r[16] = F.c0.y, r[17] = F.c0.z, r[18] = F.c1.x, r[19] = F.c1.y, r[20] = F.c1.z;
       r[21] = F.c2.x, r[22] = F.c2.y, r[23] = F.c2.z;
     }
-    if (P2G) scatter<POW2>(a, pos, vel, B, F, rest_volume, mass);
+    scatter<POW2>(a, pos, vel, B, F, rest_volume, mass);
   }
   if (G2P) {
     __syncthreads();
@@ -663,7 +754,11 @@ CkArgs make_args(float4* acc, float4* vel, uint32_t* flags, uint32_t* lists, ae_
   a.list = lists;
   a.gn = int(cfg.grid_n);
   a.nb = int(cfg.grid_n ? (cfg.grid_n + 3) / 4 : 1);
-  a.h = cfg.grid_h, a.dt = cfg.dt, a.youngs = cfg.youngs_modulus, a.poisson = cfg.poissons_ratio;
+  a.h = cfg.grid_h, a.dt = cfg.dt;
+  const float e = cfg.youngs_modulus, nu = cfg.poissons_ratio;
+  a.mu = e / (2.0f * (1.0f + nu));
+  a.lambda = e * nu / ((1.0f + nu) * (1.0f - 2.0f * nu));
+  a.d_inv = 4.0f / (cfg.grid_h * cfg.grid_h);
   a.sp = Spacing{cfg.grid_h, 0.0f, 0.0f};
   int e2 = 0;
   *pow2 = std::isfinite(cfg.grid_h) && cfg.grid_h > 0.0f && std::frexp(cfg.grid_h, &e2) == 0.5f && e2 - 1 >= -40 &&
@@ -673,6 +768,14 @@ CkArgs make_args(float4* acc, float4* vel, uint32_t* flags, uint32_t* lists, ae_
   for (int k = 0; k < 3; ++k) a.g[k] = cfg.gravity[k], a.bmin[k] = cfg.bounds_min[k], a.bmax[k] = cfg.bounds_max[k];
   a.aligned16 = (reinterpret_cast<uintptr_t>(particles) & 15u) == 0;
   return a;
+}
+}  // namespace
+
+namespace {
+// one CTA per group of records of its warps, at most what the GPU holds at once
+unsigned particle_ctas(uint64_t n) {
+  const uint64_t want = (n + 32 * kCkWarps - 1) / (32 * kCkWarps);
+  return unsigned(std::min<uint64_t>(want, uint64_t(device_sm_count()) * kCkCtas));
 }
 }  // namespace
 
@@ -696,7 +799,7 @@ cudaError_t CkWork::step(ae_mpm_ck_particle* particles, uint64_t n, const ae_mpm
   if (e != cudaSuccess) return e;
   bool pow2 = false;
   CkArgs a = make_args(acc_, vel_, flags_, lists_, particles, n, cfg, &pow2);
-  const unsigned pgrid = unsigned((n + kCkThreads - 1) / kCkThreads);
+  const unsigned pgrid = unsigned((n + kCkThreads - 1) / kCkThreads), gpart = particle_ctas(n);
   const unsigned ggrid = unsigned(std::min<uint64_t>(148 * 4, (blocks_ + 4 * kGridU - 1) / (4 * kGridU)));
   const unsigned cgrid = unsigned(std::min<uint64_t>(148 * 8, (blocks_ + 255) / 256));
   // optional per-launch events: [2 k] before and [2 k + 1] after launch k
@@ -724,9 +827,9 @@ cudaError_t CkWork::step(ae_mpm_ck_particle* particles, uint64_t n, const ae_mpm
   a.list = lists_;
   before();
   if (pow2)
-    ck_particles_kernel<false, true, true><<<pgrid, kCkThreads, 0, s>>>(a);
+    ck_particles_kernel<false, true><<<pgrid, kCkThreads, 0, s>>>(a);
   else
-    ck_particles_kernel<false, true, false><<<pgrid, kCkThreads, 0, s>>>(a);
+    ck_particles_kernel<false, false><<<pgrid, kCkThreads, 0, s>>>(a);
   after(true);
   for (uint32_t st = 0; st < steps; ++st) {
     // counters alternate by step: this step's compaction appends to one and zeroes the other
@@ -740,13 +843,13 @@ cudaError_t CkWork::step(ae_mpm_ck_particle* particles, uint64_t n, const ae_mpm
     after(false);
     before();
     if (st + 1 < steps && pow2)
-      ck_particles_kernel<true, true, true><<<pgrid, kCkThreads, 0, s>>>(a);
+      ck_particles_kernel<true, true><<<pgrid, kCkThreads, 0, s>>>(a);
     else if (st + 1 < steps)
-      ck_particles_kernel<true, true, false><<<pgrid, kCkThreads, 0, s>>>(a);
+      ck_particles_kernel<true, false><<<pgrid, kCkThreads, 0, s>>>(a);
     else if (pow2)
-      ck_particles_kernel<true, false, true><<<pgrid, kCkThreads, 0, s>>>(a);
+      ck_gather_kernel<true><<<gpart, 32 * kCkWarps, 0, s>>>(a);
     else
-      ck_particles_kernel<true, false, false><<<pgrid, kCkThreads, 0, s>>>(a);
+      ck_gather_kernel<false><<<gpart, 32 * kCkWarps, 0, s>>>(a);
     after(true);
   }
   e = cudaGetLastError();
@@ -802,7 +905,7 @@ cudaError_t CkWork::step_deterministic(ae_mpm_ck_particle* particles, uint64_t n
   const uint32_t g1 = cfg.grid_n + 1u, dead = g1 * g1 * g1;
   int key_bits = 1;
   while (key_bits < 32 && (dead >> key_bits) != 0u) ++key_bits;
-  const unsigned pgrid = unsigned((n + kCkThreads - 1) / kCkThreads);
+  const unsigned pgrid = unsigned((n + kCkThreads - 1) / kCkThreads), gpart = particle_ctas(n);
   const unsigned sgrid = unsigned(std::min<uint64_t>(148 * 8, (n + 255) / 256));
   const unsigned ngrid = unsigned(std::min<uint64_t>(148 * 8, (blocks_ + 3) / 4));
   const unsigned ggrid = unsigned(std::min<uint64_t>(148 * 4, (blocks_ + 4 * kGridU - 1) / (4 * kGridU)));
@@ -826,9 +929,9 @@ cudaError_t CkWork::step_deterministic(ae_mpm_ck_particle* particles, uint64_t n
     ck_grid_kernel<<<ggrid, kGridThreads, 0, s>>>(a, vel_);
     ck_det_ranges_kernel<false><<<sgrid, 256, 0, s>>>(skeys, n, dead, det_range_);
     if (pow2)
-      ck_particles_kernel<true, false, true><<<pgrid, kCkThreads, 0, s>>>(a);
+      ck_gather_kernel<true><<<gpart, 32 * kCkWarps, 0, s>>>(a);
     else
-      ck_particles_kernel<true, false, false><<<pgrid, kCkThreads, 0, s>>>(a);
+      ck_gather_kernel<false><<<gpart, 32 * kCkWarps, 0, s>>>(a);
     launches += 6;
   }
   e = cudaGetLastError();
