@@ -77,6 +77,12 @@ __device__ __forceinline__ void cp_async_v4(V4* sdst, const V4* gsrc) {
     cp_async16(reinterpret_cast<char*>(sdst) + 16 * k, reinterpret_cast<const char*>(gsrc) + 16 * k);
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may start while the kernel
+// before it drains, and waits here until that one has finished and its writes are visible.  Without
+// the launch attribute both are no-ops.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 template <class T>
 __device__ __forceinline__ int floor_to_int(T v) {
   if (v != v) return 0;  // NaN -> 0, as Rust's `as isize`
@@ -119,14 +125,18 @@ __device__ __forceinline__ uint32_t cell_key(const SceneDev<T>& sc, int mode, T 
 // A world of one scene needs no table (its chunks are consecutive ranges of blockDim.x slots),
 // so its CTAs start their particle loads without first waiting for a descriptor load.
 template <class T>
-__device__ __forceinline__ int4 cta_chunk(const WorldDev<T>& w) {
+__device__ __forceinline__ int4 chunk_at(const WorldDev<T>& w, uint32_t chunk, uint32_t slots) {
   if (w.one_scene) {
-    const uint64_t lo = uint64_t(w.one_off) + uint64_t(blockIdx.x) * blockDim.x;
-    const uint64_t live = lo + blockDim.x < w.one_live_end ? lo + blockDim.x : w.one_live_end;
-    const uint64_t cap = lo + blockDim.x < w.one_cap_end ? lo + blockDim.x : w.one_cap_end;
+    const uint64_t lo = uint64_t(w.one_off) + uint64_t(chunk) * slots;
+    const uint64_t live = lo + slots < w.one_live_end ? lo + slots : w.one_live_end;
+    const uint64_t cap = lo + slots < w.one_cap_end ? lo + slots : w.one_cap_end;
     return make_int4(0, int(lo), int(live > lo ? live : lo), int(cap));
   }
-  return w.chunks[blockIdx.x];
+  return w.chunks[chunk];
+}
+template <class T>
+__device__ __forceinline__ int4 cta_chunk(const WorldDev<T>& w) {
+  return chunk_at(w, blockIdx.x, blockDim.x);
 }
 
 template <class T>
@@ -959,13 +969,14 @@ __device__ __forceinline__ void block_coords(const SceneDev<T>& sc, uint32_t gb,
   k = bz * 4 + (l >> 4);
 }
 
+// by CTA `cta` of `ctas`
 template <class T, int MODE>
-__global__ void __launch_bounds__(256) grid_update_kernel(WorldDev<T> w, uint32_t* blk_epoch, const uint32_t* epoch,
-                                                          uint32_t* zero_count) {
+__device__ __forceinline__ void grid_update(const WorldDev<T>& w, uint32_t* blk_epoch, const uint32_t* epoch,
+                                            uint32_t* zero_count, uint32_t cta, uint32_t ctas) {
   using V4 = typename V4T<T>::type;
   const uint32_t count = launch_count(w.touched_count);
   const uint32_t ep = *epoch;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (cta == 0 && threadIdx.x == 0) {
     *w.clamp_count = 0u;  // G2P of this substep refills it
     // the fused G2P + P2G appends the next substep's blocks to the other list, whose previous
     // contents the grid update of the substep before consumed
@@ -975,7 +986,7 @@ __global__ void __launch_bounds__(256) grid_update_kernel(WorldDev<T> w, uint32_
   // before using any, so a long touched list is not one latency-bound load after another
   constexpr int kU = 4;
   const int sub = threadIdx.x >> 6, l = threadIdx.x & 63;
-  for (uint32_t t0 = (blockIdx.x * 4 + sub) * kU; t0 < count; t0 += gridDim.x * 4 * kU) {
+  for (uint32_t t0 = (cta * 4 + sub) * kU; t0 < count; t0 += ctas * 4 * kU) {
     uint32_t gb[kU];
     V4 a[kU];
 #pragma unroll
@@ -1000,6 +1011,14 @@ __global__ void __launch_bounds__(256) grid_update_kernel(WorldDev<T> w, uint32_
       }
     }
   }
+}
+
+template <class T, int MODE>
+__global__ void __launch_bounds__(256) grid_update_kernel(WorldDev<T> w, uint32_t* blk_epoch, const uint32_t* epoch,
+                                                          uint32_t* zero_count) {
+  let_next_start();
+  dependency_wait();
+  grid_update<T, MODE>(w, blk_epoch, epoch, zero_count, blockIdx.x, gridDim.x);
 }
 
 // ============================================================================================
@@ -2020,18 +2039,21 @@ constexpr int kInlineClamp = 8;
 
 // G2P of substep s and P2G of substep s + 1 (physics mode).  The grid update of substep s ran
 // before; w.touched / w.touched_count are the touched-block list of substep s + 1.
-template <class T>
+// kSnow: the world has snow materials.  kPer: particles per warp; a chunk of blockDim slots takes
+// 32 / kPer CTAs.
+template <class T, bool kSnow, int kPer>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(WorldDev<T> w, uint32_t* epoch,
                                                                               int write_keys) {
   using V4 = typename V4T<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int4 ch = cta_chunk(w);
+  constexpr int kSplit = 32 / kPer;
+  const int4 ch = chunk_at(w, blockIdx.x / kSplit, blockDim.x);
   const SceneDev<T>& sc = w.scenes[ch.x];
   const int tid = threadIdx.x, lane = tid & 31;
   const WarpStage<T> st = warp_stage<T>(smem, tid >> 5);
   V4* pre = st.col;  // F, J and the material of the warp's particles (pre[k * 32 + lane]) until the scatter
-  const int j = ch.y + tid;
-  const bool live = j < ch.z;
+  const int j = ch.y + int(blockIdx.x % kSplit) * int(blockDim.x / kSplit) + (tid >> 5) * kPer + lane;
+  const bool slot = kPer == 32 || lane < kPer, live = slot && j < ch.z;
   if (blockIdx.x == 0 && tid == 0) *epoch += 1u;
   uint32_t err = 0;
   bool cl = false, need = false, has = false;
@@ -2064,12 +2086,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
     const T F[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
     const MatDev& md = mat_of(w, sc, Bits<T>::unpack(a3.z) & 0xffffu);
     g2p_physics_move<T>(sc, md, x0, pv, F, a3.y, o);
-    need = o.needs_clamp;
+    need = kSnow && o.needs_clamp;
     // Yielding snow: a warp with many such particles maps them back here; a few are left to the
     // clamp kernel, which packs 32 of them from all over into a warp.
-    const uint32_t yielding = __ballot_sync(live_mask, need);
     m = a0.w;
-    if (__popc(yielding) >= kInlineClamp) {
+    if (kSnow && __popc(__ballot_sync(live_mask, need)) >= kInlineClamp) {
       // the particle waits in the warp's staging region (past the prefetched F) during the call
       T* park = reinterpret_cast<T*>(pre + 96) + lane;
 #pragma unroll
@@ -2118,20 +2139,22 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
     }
 #pragma unroll
     for (int k = 0; k < 9; ++k) A[k] = o.C[k];
-  } else if (j < ch.w && write_keys && !w.bins) {
+  } else if (slot && j < ch.w && write_keys && !w.bins) {
     w.keys[j] = sc.dead_key;
   }
   const uint32_t e = __reduce_or_sync(0xffffffffu, err);
   const uint32_t ncl = __popc(__ballot_sync(0xffffffffu, cl));
-  const uint32_t qmask = __ballot_sync(0xffffffffu, need);
+  const uint32_t qmask = kSnow ? __ballot_sync(0xffffffffu, need) : 0u;
   uint32_t qbase = 0;
   if (lane == 0) {
     if (e) atomicOr(w.err + 4 * ch.x, e);
     if (ncl) atomicAdd(w.err + 4 * ch.x + 2, ncl);
-    if (qmask) qbase = atomicAdd(w.clamp_count, uint32_t(__popc(qmask)));
+    if (kSnow && qmask) qbase = atomicAdd(w.clamp_count, uint32_t(__popc(qmask)));
   }
-  qbase = __shfl_sync(0xffffffffu, qbase, 0);
-  if (need) w.clamp_queue[qbase + __popc(qmask & ((1u << lane) - 1u))] = make_uint2(uint32_t(j), uint32_t(ch.x));
+  if (kSnow) {
+    qbase = __shfl_sync(0xffffffffu, qbase, 0);
+    if (need) w.clamp_queue[qbase + __popc(qmask & ((1u << lane) - 1u))] = make_uint2(uint32_t(j), uint32_t(ch.x));
+  }
   __syncwarp();  // every lane has read its F, J and material: the scatter may reuse the region
   p2g_warp_scatter<T, false>(w, sc, has, xs, m, mv, A, st, uint32_t(j), write_keys);
 }
@@ -2589,13 +2612,12 @@ __device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, uint64_t nodes,
-                                                               const uint32_t* __restrict__ dead_blk,
-                                                               uint32_t* seg_total, uint32_t* done) {
+__device__ __forceinline__ void bin_scan(const WorldDev<T>& w, uint64_t nodes, const uint32_t* __restrict__ dead_blk,
+                                         uint32_t* seg_total, uint32_t* done, uint32_t cta, uint32_t ctas) {
   __shared__ uint32_t wsum[kBinThreads / 32];
   __shared__ uint32_t s_last, s_carry;
   const int tid = threadIdx.x, lane = tid & 31, wi = tid >> 5;
-  const uint64_t base = uint64_t(blockIdx.x) * kBinSeg + uint64_t(wi) * 512u;
+  const uint64_t base = uint64_t(cta) * kBinSeg + uint64_t(wi) * 512u;
   uint4* bins4 = reinterpret_cast<uint4*>(w.bins);
   uint4* off4 = reinterpret_cast<uint4*>(w.bin_off);
   uint4 c[4];
@@ -2653,20 +2675,20 @@ __global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, ui
     }
   }
   if (tid == 0) {
-    seg_total[blockIdx.x] = total;
+    seg_total[cta] = total;
     __threadfence();
-    s_last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    s_last = atomicAdd(done, 1u) == ctas - 1 ? 1u : 0u;
     s_carry = 0u;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (uint32_t s0 = 0; s0 < gridDim.x; s0 += kBinThreads * 4) {
+  for (uint32_t s0 = 0; s0 < ctas; s0 += kBinThreads * 4) {
     uint32_t v[4], t = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t i = s0 + tid * 4 + k;
-      v[k] = i < gridDim.x ? __ldcg(seg_total + i) : 0u;
+      v[k] = i < ctas ? __ldcg(seg_total + i) : 0u;
       t += v[k];
     }
     const uint32_t incl = warp_scan_incl(t, lane);
@@ -2682,7 +2704,7 @@ __global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, ui
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t i = s0 + tid * 4 + k;
-      if (i < gridDim.x) w.seg_off[i] = o;
+      if (i < ctas) w.seg_off[i] = o;
       o += v[k];
     }
     __syncthreads();
@@ -2692,9 +2714,35 @@ __global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, ui
 }
 
 template <class T>
+__global__ void __launch_bounds__(kBinThreads) bin_scan_kernel(WorldDev<T> w, uint64_t nodes,
+                                                               const uint32_t* __restrict__ dead_blk,
+                                                               uint32_t* seg_total, uint32_t* done) {
+  bin_scan(w, nodes, dead_blk, seg_total, done, blockIdx.x, gridDim.x);
+}
+
+// The scan of the next order and the grid update read nothing of each other: one launch, the first
+// `scan_ctas` CTAs scan.  Small worlds are bound by the number of dependent launches (2 300
+// particles on a 32^3 grid: 20.2 us a substep with four launches).
+template <class T>
+__global__ void __launch_bounds__(kBinThreads) scan_and_grid_kernel(WorldDev<T> w, uint64_t nodes,
+                                                                    const uint32_t* __restrict__ dead_blk,
+                                                                    uint32_t* seg_total, uint32_t* done,
+                                                                    uint32_t scan_ctas, uint32_t* blk_epoch,
+                                                                    const uint32_t* epoch, uint32_t* zero_count) {
+  let_next_start();
+  dependency_wait();
+  if (blockIdx.x < scan_ctas)
+    bin_scan(w, nodes, dead_blk, seg_total, done, blockIdx.x, scan_ctas);
+  else
+    grid_update<T, AE_MPM_MODE_PHYSICS>(w, blk_epoch, epoch, zero_count, blockIdx.x - scan_ctas, gridDim.x - scan_ctas);
+}
+
+template <class T>
 __global__ void __launch_bounds__(256) bin_scatter_kernel(WorldDev<T> w, uint32_t* __restrict__ perm,
                                                           uint32_t n_slots) {
+  let_next_start();
   const int4 ch = cta_chunk(w);
+  dependency_wait();
   const int j = ch.y + threadIdx.x, lane = threadIdx.x & 31;
   const bool live = j < ch.z;
   const uint32_t key = live ? w.keys[j] : 0xffffffffu;
@@ -3574,12 +3622,13 @@ class World final : public WorldBase {
     const uint32_t period = (interval % 2 == 0) ? interval : 2 * interval;
     uint32_t left = n;
     while (left > 0) {
-      if (opts_.use_graph && phase_ == 0 && left >= period && n_chunks_ > 0) {
-        if (!sorted_) sort_particles();
+      if (opts_.use_graph && phase_ == 0 && left >= period && n_chunks_ > 0 && graph_entry()) {
         rc = ensure_graph(period);
         if (rc) return rc;
         Graph& g = graphs_[substep_ & 1];
         AE_TRY(cudaGraphLaunch(g.exec, stream_));
+        sorted_ = g.sorted_out;
+        keys_fresh_ = g.fresh_out;
         launches_ += g.launches;
         substep_ += period;
         left -= period;
@@ -4161,7 +4210,9 @@ class World final : public WorldBase {
   int sync_scatter() {
     const int par = int(substep_ & 1);
     if (fused() && !fused_smem_set_) {  // sized for the largest block (256 threads) the world accepts
-      AE_TRY(cudaFuncSetAttribute(g2p2g_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(fused_smem(256))));
+      for (auto fn : {g2p2g_kernel<T, false, 8>, g2p2g_kernel<T, false, 16>, g2p2g_kernel<T, false, 32>,
+                      g2p2g_kernel<T, true, 32>})
+        AE_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(fused_smem(256))));
       AE_TRY(cudaFuncSetAttribute(snow_clamp_scatter_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(fused_smem(128))));
       fused_smem_set_ = true;
@@ -4201,18 +4252,68 @@ class World final : public WorldBase {
     return AE_MPM_OK;
   }
 
-  void substep_fused(WorldDev<T>& w, bool write_keys) {
-    const int sms = device_sm_count();
+  // The fused kernel of this world: without the snow code where no material needs it, and with fewer
+  // particles per warp where the warps are too few to hide one another's latency (a warp sums its
+  // runs one after another).  Water at 8 per cell, us per substep with 32 / 16 / 8 per warp: 2 309
+  // particles 16.8 / 15.4 / 14.6, 9 000 17.9 / 16.5 / 15.6, 24 000 18.4 / 17.9 / 18.5, 40 000 22.6 /
+  // 20.2 / 24.5, 64 000 20.2 / 21.7 / 26.9: 8 up to 10 such warps per SM, 16 up to 20.  With snow's
+  // return mapping in the warp 32 is the fastest from 4 600 particles on (27.6 / 30.3 / 32.7).
+  struct FusedKernel {
+    void (*fn)(WorldDev<T>, uint32_t*, int);
+    int per;
+  };
+  FusedKernel fused_kernel() const {
+    const uint64_t sms = uint64_t(device_sm_count());
+    if (has_snow_) return {g2p2g_kernel<T, true, 32>, 32};
+    if (total_cap_ <= sms * 80) return {g2p2g_kernel<T, false, 8>, 8};
+    if (total_cap_ <= sms * 320) return {g2p2g_kernel<T, false, 16>, 16};
+    return {g2p2g_kernel<T, false, 32>, 32};
+  }
+
+  // A small kernel between the fused ones.  In a world whose particles fit the GPU at once it may start
+  // while its predecessor drains; in a larger one, whose CTAs fill the GPU anyway, early CTAs would
+  // only hold room that other streams' worlds can use.  (The fused kernel itself starts after the
+  // others: early CTAs crowd on the first free SMs, 9.3 -> 18 us for 128 CTAs.)
+  template <class... P, class... A>
+  void launch_dependent(void (*kernel)(P...), unsigned ctas, unsigned threads, size_t smem, A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(ctas);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream_;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = total_cap_ <= uint64_t(device_sm_count()) * 1024 ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+    ++launches_;
+  }
+
+  // sort_first: the substep starts with the sort, whose keys and counts are there
+  void substep_fused(bool sort_first, bool write_keys) {
+    const unsigned sms = unsigned(device_sm_count());
     const int par = int(substep_ & 1);
     mark(2);  // no stand-alone P2G: the previous substep's G2P scattered this one
-    WorldDev<T> wg = with_list(w, par);
-    grid_update_kernel<T, AE_MPM_MODE_PHYSICS><<<sms * 4, 256, 0, stream_>>>(wg, blk_epoch_, counters_ + 2,
-                                                                          touched_count(par ^ 1));
+    WorldDev<T> wg = with_list(dev(sorted_), par);
+    if (sort_first) {
+      launch_dependent(scan_and_grid_kernel<T>, n_segs_ + sms * 4, kBinThreads, 0, wg, total_blocks_ * 64, dead_blk_,
+                       seg_, counters_ + 5, n_segs_, blk_epoch_, counters_ + 2, touched_count(par ^ 1));
+      launch_dependent(bin_scatter_kernel<T>, unsigned(n_chunks_), unsigned(chunk_threads_), 0, wg, bin_perm_,
+                       uint32_t(total_cap_));
+      perm_ = bin_perm_;
+      sorted_ = true;
+      keys_fresh_ = false;
+    } else {
+      launch_dependent(grid_update_kernel<T, AE_MPM_MODE_PHYSICS>, sms * 4, 256, 0, wg, blk_epoch_, counters_ + 2,
+                       touched_count(par ^ 1));
+    }
     mark(3);
-    WorldDev<T> wf = with_list(w, par ^ 1);
-    g2p2g_kernel<T><<<n_chunks_, chunk_threads_, fused_smem(chunk_threads_), stream_>>>(wf, counters_ + 2,
-                                                                                         write_keys ? 1 : 0);
-    launches_ += 2;
+    WorldDev<T> wf = with_list(dev(sorted_), par ^ 1);
+    const FusedKernel k = fused_kernel();
+    k.fn<<<unsigned(n_chunks_) * (32 / k.per), unsigned(chunk_threads_), fused_smem(chunk_threads_), stream_>>>(
+        wf, counters_ + 2, write_keys ? 1 : 0);
+    ++launches_;
     mark(5);  // the fused kernel alone ends here
     if (has_snow_) {
       snow_clamp_scatter_kernel<T><<<sms * 8, 128, fused_smem(128), stream_>>>(wf, write_keys ? 1 : 0);
@@ -4263,13 +4364,16 @@ class World final : public WorldBase {
     const bool write_keys = next == 0 && (!dense_sort_ || fused() || opts_.deterministic);
     if (n_chunks_ > 0) {
       mark(0);
-      if (phase_ == 0 && !sorted_) sort_particles();
+      const bool sort_now = phase_ == 0 && !sorted_;
+      // the scan shares its launch with the grid update
+      const bool joined = sort_now && fused() && dense_sort_ && keys_fresh_;
+      if (sort_now && !joined) sort_particles();
       mark(1);
       WorldDev<T> w = dev(sorted_);
       switch (mode_) {
         case AE_MPM_MODE_PHYSICS:
           if (fused())
-            substep_fused(w, write_keys);
+            substep_fused(joined, write_keys);
           else
             substep_mode<AE_MPM_MODE_PHYSICS>(w, write_keys);
           break;
@@ -4284,9 +4388,18 @@ class World final : public WorldBase {
     ++substep_;
   }
 
-  // A graph holds one period of substeps from sorted particles to sorted particles: lcm(2, sort
-  // interval), since buffers and touched lists alternate.  A period may start on either parity (the
-  // interval counts from the last upload), so there is one graph for each.
+  // What a graph starts from: with a sort every substep, cells counted by the substep before (the
+  // first substep after an upload runs on its own); otherwise particles in order, sorted here, once
+  // per period, outside the graph.
+  bool graph_entry() {
+    if (sort_interval() == 1 && fused() && dense_sort_) return keys_fresh_ && !sorted_;
+    if (!sorted_) sort_particles();
+    return true;
+  }
+
+  // A graph holds one period of substeps: lcm(2, sort interval), since buffers and touched lists
+  // alternate.  A period may start on either parity (the interval counts from the last upload), so
+  // there is one graph for each.
   int ensure_graph(uint32_t period) {
     Graph& gr = graphs_[substep_ & 1];
     if (gr.exec && gr.period == period && gr.variant == opts_.p2g_variant && gr.a_in == a_in_) return AE_MPM_OK;
@@ -4297,8 +4410,12 @@ class World final : public WorldBase {
     const bool a_in0 = a_in_;
     const uint64_t sub0 = substep_, l0 = launches_;
     AE_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    const bool sorted0 = sorted_, fresh0 = keys_fresh_;
     for (uint32_t k = 0; k < period; ++k) substep_eager();
-    if (!sorted_) sort_particles();
+    gr.sorted_out = sorted_;
+    gr.fresh_out = keys_fresh_;
+    sorted_ = sorted0;
+    keys_fresh_ = fresh0;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(stream_, &g);
     a_in_ = a_in0;
@@ -4418,6 +4535,7 @@ class World final : public WorldBase {
     uint64_t launches = 0;
     int variant = -1;
     bool a_in = true;
+    bool sorted_out = false, fresh_out = false;  // the world's state after it
   };
   Graph graphs_[2];  // by the parity of the period's first substep
   bool lanes_smem_set_ = false, fused_smem_set_ = false, ref_lanes_smem_set_ = false, det_smem_set_ = false;
