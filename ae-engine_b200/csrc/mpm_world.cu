@@ -3113,69 +3113,82 @@ class World final : public WorldBase {
       fill_scene_params(h, d);
       h_scenes_.push_back(h);
     }
-    AE_TRY(dmalloc(&d_scenes_, sizeof(SceneDev<T>) * n));
-    AE_TRY(dmalloc(&d_mats_, sizeof(MatDev) * h_mats_.size()));
-    AE_TRY(cudaMemcpy(d_mats_, h_mats_.data(), sizeof(MatDev) * h_mats_.size(), cudaMemcpyHostToDevice));
-    AE_TRY(dmalloc(&blk_scene_, sizeof(uint32_t) * blk));
-    AE_TRY(cudaMemcpy(blk_scene_, blk_scene.data(), sizeof(uint32_t) * blk, cudaMemcpyHostToDevice));
-    AE_TRY(dmalloc(&dead_blk_, sizeof(uint32_t) * blk));
-    AE_TRY(cudaMemcpy(dead_blk_, dead.data(), sizeof(uint32_t) * blk, cudaMemcpyHostToDevice));
-    // particles
-    const uint64_t pc = std::max<uint64_t>(cap, 1);
+    // One allocation carries every array of the world, the ones that start at zero side by side (one
+    // clear): thirty allocations and a dozen clears took most of a world's creation.
+    const uint64_t pc = std::max<uint64_t>(cap, 1), nodes = blk * 64;
+    enum { kZero, kOnes, kNone };
+    struct Region {
+      void** p;
+      size_t bytes;
+      int fill;
+    };
+    std::vector<Region> regions;
+    auto reserve = [&regions](auto** p, size_t bytes, int fill) {
+      regions.push_back({reinterpret_cast<void**>(p), bytes, fill});
+    };
+    reserve(&d_scenes_, sizeof(SceneDev<T>) * n, kNone);
+    reserve(&d_mats_, sizeof(MatDev) * h_mats_.size(), kNone);
+    reserve(&blk_scene_, sizeof(uint32_t) * blk, kNone);
+    reserve(&dead_blk_, sizeof(uint32_t) * blk, kNone);
     // particle slots past a scene's count are never read (every kernel gates on the live range),
     // so the particle arrays need no clearing
     for (int k = 0; k < 7; ++k) {
-      AE_TRY(dmalloc(&bufA_[k], sizeof(V4) * pc));
-      AE_TRY(dmalloc(&bufB_[k], sizeof(V4) * pc));
+      reserve(&bufA_[k], sizeof(V4) * pc, kNone);
+      reserve(&bufB_[k], sizeof(V4) * pc, kNone);
     }
-    AE_TRY(dmalloc(&keys_, sizeof(uint32_t) * pc));
+    reserve(&keys_, sizeof(uint32_t) * pc, kNone);
+    reserve(&clamp_queue_, sizeof(uint2) * pc, kNone);
     // Dense grouping reads every node's counter; the radix sort moves 20 bytes per key and pass.
     // The grid decides: up to 16 nodes per particle slot (or 8 M nodes, 5 us of scan) the dense
     // grouping wins, a huge grid with few particles in it keeps the radix sort.
-    dense_sort_ = blk * 64 <= 16 * cap + (uint64_t(8) << 20);
+    dense_sort_ = nodes <= 16 * cap + (uint64_t(8) << 20);
     if (dense_sort_) {
-      n_segs_ = uint32_t((blk * 64 + kBinSeg - 1) / kBinSeg);
-      AE_TRY(dmalloc(&bins_, sizeof(uint32_t) * blk * 64));
-      AE_TRY(cudaMemset(bins_, 0, sizeof(uint32_t) * blk * 64));
-      AE_TRY(dmalloc(&bin_off_, sizeof(uint32_t) * blk * 64));
-      AE_TRY(dmalloc(&seg_, sizeof(uint32_t) * 2 * n_segs_));
-      AE_TRY(dmalloc(&bin_perm_, sizeof(uint32_t) * pc));
-      AE_TRY(cudaMemset(bin_perm_, 0, sizeof(uint32_t) * pc));
+      n_segs_ = uint32_t((nodes + kBinSeg - 1) / kBinSeg);
+      reserve(&bins_, sizeof(uint32_t) * nodes, kZero);
+      reserve(&bin_off_, sizeof(uint32_t) * nodes, kNone);
+      reserve(&seg_, sizeof(uint32_t) * 2 * n_segs_, kNone);
+      reserve(&bin_perm_, sizeof(uint32_t) * pc, kZero);
       if (opts_.deterministic) {
-        AE_TRY(dmalloc(&cells_, sizeof(uint2) * blk * 64));
-        AE_TRY(cudaMemset(cells_, 0, sizeof(uint2) * blk * 64));
-        AE_TRY(dmalloc(&ordered_, sizeof(uint32_t) * pc));
-        AE_TRY(cudaMemset(ordered_, 0, sizeof(uint32_t) * pc));
+        reserve(&cells_, sizeof(uint2) * nodes, kZero);
+        reserve(&ordered_, sizeof(uint32_t) * pc, kZero);
       }
-    } else {
-      AE_TRY(sort_scratch_alloc(sort_, pc, alloc_ ? &World::sort_alloc : nullptr, alloc_));
+    } else if (opts_.deterministic) {
+      reserve(&cell_slot_, sizeof(uint32_t) * nodes, kOnes);
+      reserve(&seg_start_, sizeof(uint32_t) * pc, kNone);
     }
-    // grid
-    const uint64_t nodes = blk * 64;
-    AE_TRY(dmalloc(&acc_, sizeof(V4) * nodes));
-    AE_TRY(cudaMemset(acc_, 0, sizeof(V4) * nodes));
-    AE_TRY(dmalloc(&vel_, sizeof(V4) * nodes));
-    AE_TRY(cudaMemset(vel_, 0, sizeof(V4) * nodes));
-    AE_TRY(dmalloc(&blk_flag_, sizeof(uint32_t) * blk));
-    AE_TRY(cudaMemset(blk_flag_, 0, sizeof(uint32_t) * blk));
-    AE_TRY(dmalloc(&blk_epoch_, sizeof(uint32_t) * blk));
-    AE_TRY(cudaMemset(blk_epoch_, 0xff, sizeof(uint32_t) * blk));
+    if (opts_.deterministic) reserve(&cell_rec_, sizeof(V4) * 27 * pc, kNone);
+    reserve(&acc_, sizeof(V4) * nodes, kZero);
+    reserve(&vel_, sizeof(V4) * nodes, kZero);
+    reserve(&blk_flag_, sizeof(uint32_t) * blk, kZero);
+    reserve(&blk_epoch_, sizeof(uint32_t) * blk, kOnes);
     // two touched-block lists: the fused G2P + P2G fills the next substep's while the grid update
     // consumes the current one's
-    AE_TRY(dmalloc(&touched_, sizeof(uint32_t) * 2 * blk));
-    AE_TRY(dmalloc(&counters_, sizeof(uint32_t) * 8));
-    AE_TRY(cudaMemset(counters_, 0, sizeof(uint32_t) * 8));
-    AE_TRY(dmalloc(&clamp_queue_, sizeof(uint2) * pc));
-    AE_TRY(dmalloc(&err_, sizeof(uint32_t) * 4 * n));
-    AE_TRY(cudaMemset(err_, 0, sizeof(uint32_t) * 4 * n));
-    if (opts_.deterministic) {
-      if (!dense_sort_) {
-        AE_TRY(dmalloc(&cell_slot_, sizeof(uint32_t) * nodes));
-        AE_TRY(cudaMemset(cell_slot_, 0xff, sizeof(uint32_t) * nodes));
-        AE_TRY(dmalloc(&seg_start_, sizeof(uint32_t) * pc));
-      }
-      AE_TRY(dmalloc(&cell_rec_, sizeof(V4) * 27 * pc));
+    reserve(&touched_, sizeof(uint32_t) * 2 * blk, kNone);
+    reserve(&counters_, sizeof(uint32_t) * 8, kZero);
+    reserve(&err_, sizeof(uint32_t) * 4 * n, kZero);
+    n_chunks_alloc_ = 0;
+    for (const ae_mpm_scene_desc& d : descs_) n_chunks_alloc_ += int((d.max_particles + 127) / 128);  // smallest chunks
+    reserve(&d_chunks_, sizeof(int4) * std::max(n_chunks_alloc_, 1), kNone);
+    std::stable_sort(regions.begin(), regions.end(), [](const Region& x, const Region& y) { return x.fill < y.fill; });
+    size_t total = 0, end[2] = {0, 0};
+    for (const Region& r : regions) {
+      total += (r.bytes + 255) & ~size_t(255);
+      if (r.fill != kNone) end[r.fill] = total;
     }
+    if (end[kOnes] == 0) end[kOnes] = end[kZero];
+    AE_TRY(dmalloc(&arena_, total));
+    size_t off = 0;
+    for (const Region& r : regions) {
+      *r.p = arena_ + off;
+      off += (r.bytes + 255) & ~size_t(255);
+    }
+    AE_TRY(cudaMemsetAsync(arena_, 0, end[kZero], stream_));
+    AE_TRY(cudaMemsetAsync(arena_ + end[kZero], 0xff, end[kOnes] - end[kZero], stream_));
+    AE_TRY(cudaMemcpyAsync(d_mats_, h_mats_.data(), sizeof(MatDev) * h_mats_.size(), cudaMemcpyHostToDevice, stream_));
+    AE_TRY(cudaMemcpyAsync(blk_scene_, blk_scene.data(), sizeof(uint32_t) * blk, cudaMemcpyHostToDevice, stream_));
+    AE_TRY(cudaMemcpyAsync(dead_blk_, dead.data(), sizeof(uint32_t) * blk, cudaMemcpyHostToDevice, stream_));
+    if (!dense_sort_) AE_TRY(sort_scratch_alloc(sort_, pc, alloc_ ? &World::sort_alloc : nullptr, alloc_));
+    AE_TRY(cudaStreamSynchronize(stream_));
     return AE_MPM_OK;
   }
 
@@ -3973,14 +3986,6 @@ class World final : public WorldBase {
       chunk_first_[h_scenes_.size()] = n_chunks_;
       count_dirty_.assign(h_scenes_.size(), 0);
       any_count_dirty_ = false;
-      if (n_chunks_ > n_chunks_alloc_) {
-        dfree(d_chunks_);
-        d_chunks_ = nullptr;
-        dfree(partial_);
-        partial_ = nullptr;
-        AE_TRY(dmalloc(&d_chunks_, sizeof(int4) * n_chunks_));
-        n_chunks_alloc_ = n_chunks_;
-      }
       if (n_chunks_ > 0)
         AE_TRY(cudaMemcpyAsync(d_chunks_, h_chunks_.data(), sizeof(int4) * n_chunks_, cudaMemcpyHostToDevice, stream_));
       drop_graphs();
@@ -4449,35 +4454,9 @@ class World final : public WorldBase {
     drop_graphs();
     if (stream_) cudaStreamSynchronize(stream_);
     if (xfer_ev_) cudaEventDestroy(xfer_ev_);
-    for (int k = 0; k < 7; ++k) {
-      dfree(bufA_[k]);
-      dfree(bufB_[k]);
-      dfree(snap_[k]);
-    }
-    dfree(keys_);
+    for (int k = 0; k < 7; ++k) dfree(snap_[k]);
     sort_scratch_free(sort_, alloc_ ? &World::sort_free : nullptr, alloc_);
-    dfree(bins_);
-    dfree(bin_off_);
-    dfree(seg_);
-    dfree(bin_perm_);
-    dfree(cells_);
-    dfree(ordered_);
-    dfree(acc_);
-    dfree(vel_);
-    dfree(blk_flag_);
-    dfree(blk_epoch_);
-    dfree(touched_);
-    dfree(counters_);
-    dfree(err_);
-    dfree(cell_slot_);
-    dfree(seg_start_);
-    dfree(cell_rec_);
-    dfree(clamp_queue_);
-    dfree(d_scenes_);
-    dfree(d_mats_);
-    dfree(blk_scene_);
-    dfree(dead_blk_);
-    dfree(d_chunks_);
+    dfree(arena_);
     dfree(partial_);
     dfree(stage_);
     dfree(d_xfer_);
@@ -4486,6 +4465,7 @@ class World final : public WorldBase {
 
  public:
   DevAlloc* alloc_ = nullptr;
+  unsigned char* arena_ = nullptr;  // the world's arrays
   int mode_ = 0;
   ae_mpm_exec_opts opts_{};
   std::vector<ae_mpm_scene_desc> descs_;
