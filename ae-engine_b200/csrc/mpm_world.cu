@@ -3166,6 +3166,7 @@ class World final : public WorldBase {
     reserve(&touched_, sizeof(uint32_t) * 2 * blk, kNone);
     reserve(&counters_, sizeof(uint32_t) * 8, kZero);
     reserve(&err_, sizeof(uint32_t) * 4 * n, kZero);
+    reserve(&d_xfer_, sizeof(XferDev<T>) * n, kNone);
     n_chunks_alloc_ = 0;
     for (const ae_mpm_scene_desc& d : descs_) n_chunks_alloc_ += int((d.max_particles + 127) / 128);  // smallest chunks
     reserve(&d_chunks_, sizeof(int4) * std::max(n_chunks_alloc_, 1), kNone);
@@ -3306,14 +3307,6 @@ class World final : public WorldBase {
       }
       h_xfer_.assign(hi - lo + 1, XferDev<T>{});
       for (uint32_t i = 0; i < k; ++i) h_xfer_[scenes[i] - lo] = x[i];
-      if (h_xfer_.size() > xfer_cap_) {
-        AE_TRY(cudaStreamSynchronize(stream_));  // queued transfers may still read the old table
-        dfree(d_xfer_);
-        d_xfer_ = nullptr;
-        xfer_cap_ = 0;
-        AE_TRY(dmalloc(&d_xfer_, sizeof(XferDev<T>) * h_xfer_.size()));
-        xfer_cap_ = h_xfer_.size();
-      }
       AE_TRY(cudaMemcpyAsync(d_xfer_, h_xfer_.data(), sizeof(XferDev<T>) * h_xfer_.size(), cudaMemcpyHostToDevice,
                              stream_));
       xs.tab = d_xfer_;
@@ -4459,7 +4452,6 @@ class World final : public WorldBase {
     dfree(arena_);
     dfree(partial_);
     dfree(stage_);
-    dfree(d_xfer_);
     if (stream_) cudaStreamDestroy(stream_);
   }
 
@@ -4506,7 +4498,6 @@ class World final : public WorldBase {
   size_t stage_bytes_ = 0;
   std::vector<XferDev<T>> h_xfer_;  // many-scene transfer table
   XferDev<T>* d_xfer_ = nullptr;
-  size_t xfer_cap_ = 0;
   double* partial_ = nullptr;
   cudaStream_t stream_ = nullptr;
   struct Graph {
