@@ -781,10 +781,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) p2g_lanes_velonly
 // the x part of each of their column's three nodes and sum over each cell's run, one vector
 // reduction per node and run.
 constexpr int kRefLaneVecs = 2 * 9 + 5;  // shared vectors per particle
-template <class T>
+// kPer particles per warp, 32 / kPer CTAs per chunk: the engine's near set is sparse (about one
+// particle in twelve cells), so every particle is a run of its own and a warp sums its runs one
+// after another; 10 000 particles with 32 per warp took 30 us on 40 of the SMs.
+template <class T, int kPer>
 __global__ void __launch_bounds__(256, 1) p2g_lanes_ref_kernel(WorldDev<T> w) {
   using V4 = typename V4T<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int kSplit = 32 / kPer;
   const int nt = blockDim.x;
   V4* cu = reinterpret_cast<V4*>(smem);  // cu[q * 9 + j] = (u, wy)
   V4* cf = cu + 9 * nt;                  // cf[q * 9 + j] = (f, wz)
@@ -795,11 +799,11 @@ __global__ void __launch_bounds__(256, 1) p2g_lanes_ref_kernel(WorldDev<T> w) {
   V4* pe = ps + nt;                      // pe[q] = (N'_x of the three x nodes) / dx
   int4* gk = reinterpret_cast<int4*>(pe + nt);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int4 ch = cta_chunk(w);
+  const int4 ch = chunk_at(w, blockIdx.x / kSplit, blockDim.x);
   const SceneDev<T>& sc = w.scenes[ch.x];
   const int n0 = sc.n[0], n1 = sc.n[1], n2 = sc.n[2];
-  const int j = ch.y + tid;
-  const bool live = j < ch.z;
+  const int j = ch.y + int(blockIdx.x % kSplit) * int(blockDim.x / kSplit) + warp * kPer + lane;
+  const bool live = (kPer == 32 || lane < kPer) && j < ch.z;
   bool has = false;
   P2GPart<T> p;
   p.g[0] = p.g[1] = p.g[2] = 0;
@@ -1370,18 +1374,34 @@ __device__ __forceinline__ void g2p_reference(const VelTile<T>& vt, const SceneD
     g[a] = max(gu, 0);
   }
   T nv[3] = {0, 0, 0}, nc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, gvm[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  T wgt[3][3], dwg[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      wgt[a][k] = b_spline(T(k) - fx[a]);
+      dwg[a][k] = b_spline_deriv(T(k) - fx[a]) * sc.inv_dx;
+    }
 #pragma unroll 1
-  for (int dk = 0; dk < 3; ++dk)
-#pragma unroll 1
+  for (int dk = 0; dk < 3; ++dk) {
+    // the plane's nine nodes first, so that their loads overlap (a node outside the grid weighs 0)
+    V4 node[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const int X = g[0] + q % 3, Y = g[1] + q / 3, Z = g[2] + dk;
+      node[q] = (X < sc.n[0] && Y < sc.n[1] && Z < sc.n[2]) ? vt(sc, X, Y, Z) : mk4(T(0), T(0), T(0), T(0));
+    }
+    const T wz = dk == 0 ? wgt[2][0] : (dk == 1 ? wgt[2][1] : wgt[2][2]);
+    const T dwz = dk == 0 ? dwg[2][0] : (dk == 1 ? dwg[2][1] : dwg[2][2]);
+#pragma unroll
     for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
       for (int di = 0; di < 3; ++di) {
-        T wx = b_spline(T(di) - fx[0]), wy = b_spline(T(dj) - fx[1]), wz = b_spline(T(dk) - fx[2]);
+        T wx = wgt[0][di], wy = wgt[1][dj];
         T ww = wx * wy * wz;
         if (ww < T(1e-10)) continue;
         int X = g[0] + di, Y = g[1] + dj, Z = g[2] + dk;
-        if (X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) continue;
-        V4 gv = vt(sc, X, Y, Z);
+        const V4 gv = node[dj * 3 + di];
         if (gv.w < T(1e-12)) continue;
         T g3[3] = {gv.x, gv.y, gv.z};
         nv[0] += ww * g3[0];
@@ -1394,13 +1414,13 @@ __device__ __forceinline__ void g2p_reference(const VelTile<T>& vt, const SceneD
         for (int r = 0; r < 3; ++r)
 #pragma unroll
           for (int c = 0; c < 3; ++c) nc[r * 3 + c] += scale * g3[r] * d3[c];
-        T dw[3] = {b_spline_deriv(T(di) - fx[0]) * sc.inv_dx, b_spline_deriv(T(dj) - fx[1]) * sc.inv_dx,
-                   b_spline_deriv(T(dk) - fx[2]) * sc.inv_dx};
+        T dw[3] = {dwg[0][di], dwg[1][dj], dwz};
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
           for (int c = 0; c < 3; ++c) gvm[r * 3 + c] -= ww * g3[r] * dw[c];
       }
+  }
   if (!t_finite(nv[0]) || !t_finite(nv[1]) || !t_finite(nv[2])) {
     nv[0] = nv[1] = nv[2] = T(0);
 #pragma unroll
@@ -2163,9 +2183,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
 // then scattered into the next substep's accumulator with its final A.  A warp takes consecutive
 // queue entries (possibly of several scenes of a world): as many as spread the queue over all warps,
 // between 4 and 32, because scattered particles are runs of their own that a warp sums one after
-// another (a short queue took 16 us with 32 entries per warp).
+// another (a short queue took 16 us with 32 entries per warp).  80 registers and 6 CTAs per SM: at 64
+// and 8 the return mapping spills (16.7 against 19.3 us a launch in a batch of snow and other scenes).
 template <class T>
-__global__ void __launch_bounds__(128, 8) snow_clamp_scatter_kernel(WorldDev<T> w, int write_keys) {
+__global__ void __launch_bounds__(128, 6) snow_clamp_scatter_kernel(WorldDev<T> w, int write_keys) {
   using V4 = typename V4T<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
@@ -4104,10 +4125,15 @@ class World final : public WorldBase {
     if (MODE == AE_MPM_MODE_REFERENCE && opts_.p2g_variant == kVarLanes) {
       const size_t per = sizeof(V4) * kRefLaneVecs + sizeof(int4);
       if (!ref_lanes_smem_set_) {  // sized for the largest block (256 threads) the world accepts
-        cudaFuncSetAttribute(p2g_lanes_ref_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * 256));
+        for (auto fn : {p2g_lanes_ref_kernel<T, 8>, p2g_lanes_ref_kernel<T, 32>})
+          cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(per * 256));
         ref_lanes_smem_set_ = true;
       }
-      p2g_lanes_ref_kernel<T><<<n_chunks_, chunk_threads_, per * chunk_threads_, stream_>>>(w);
+      // one CTA of 256 threads per SM (shared memory): 8 particles per warp while all of them run at once
+      if (total_cap_ <= uint64_t(device_sm_count()) * 128)
+        p2g_lanes_ref_kernel<T, 8><<<n_chunks_ * 4, chunk_threads_, per * chunk_threads_, stream_>>>(w);
+      else
+        p2g_lanes_ref_kernel<T, 32><<<n_chunks_, chunk_threads_, per * chunk_threads_, stream_>>>(w);
       return;
     }
     if (MODE == AE_MPM_MODE_VELOCITY_ONLY && opts_.p2g_variant == kVarLanes) {
