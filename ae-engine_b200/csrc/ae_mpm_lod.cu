@@ -11,10 +11,9 @@
 //                 the candidates into the kept near list and the tail appended to the mid list.
 //   far_field     one thread per far particle: gravity on y, position, nearest-cell sample.
 //   coarse_field  the near particles' cells are radix-sorted (stable, so each cell keeps the
-//                 reference's index order), each cell's run is located, and one thread per cell
-//                 sums its run sequentially, which
-//                 reproduces the reference's serial accumulation exactly; then relaxation and one
-//                 FTCS step, one thread per cell.
+//                 reference's index order), each cell's run is located, and one lane per cell
+//                 sums its run sequentially, which reproduces the reference's serial accumulation
+//                 exactly, and relaxes the cell; then one FTCS step, one thread per cell.
 #include "ae_mpm_lod.cuh"
 
 #include <algorithm>
@@ -50,40 +49,53 @@ struct PosClass {
   float px, py, pz, near2, mid2;
   __device__ __forceinline__ int operator()(uint64_t idx, uint64_t& item, float& d2) const {
     item = idx;
-    d2 = 0.0f;
-    if (active && !active[idx]) return 3;
+    const bool on = !active || active[idx];
     const float dx = __fsub_rn(pos[3 * idx], px), dy = __fsub_rn(pos[3 * idx + 1], py), dz = __fsub_rn(pos[3 * idx + 2], pz);
     d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-    return d2 < near2 ? 0 : (d2 < mid2 ? 1 : 2);  // NaN compares false: far
+    return !on ? 3 : (d2 < near2 ? 0 : (d2 < mid2 ? 1 : 2));  // NaN compares false: far
   }
 };
 
-// near candidate k: 0 kept, 1 culled to mid
+// near candidate k of *n: 0 kept, 1 culled to mid; all kept when they do not exceed the cap
 struct KeepClass {
   const uint64_t* near;
   const uint8_t* keep;
+  const uint32_t* n;
+  uint32_t cap;
   __device__ __forceinline__ int operator()(uint64_t k, uint64_t& item, float& d2) const {
     item = near[k];
     d2 = 0.0f;
-    return keep[k] ? 0 : 1;
+    return *n <= cap || (cap && keep[k]) ? 0 : 1;
   }
 };
 
+// The item count of a partition is `n`, or *n_dev where an earlier kernel found it (CTAs past it
+// leave at once).
+__device__ __forceinline__ uint64_t part_items(uint64_t n, const uint32_t* n_dev) { return n_dev ? *n_dev : n; }
+
 template <class Cls>
-__global__ void __launch_bounds__(kPT) part_count(Cls cls, uint64_t n, uint32_t* tile_counts, uint32_t tiles) {
+__global__ void __launch_bounds__(kPT) part_count(Cls cls, uint64_t n_items, const uint32_t* n_dev, uint32_t* tile_counts,
+                                                  uint32_t tiles) {
   __shared__ uint32_t wc[kPWarps][3];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint64_t n = part_items(n_items, n_dev);
+  if (uint64_t(blockIdx.x) * kPTile >= n) return;
   const uint64_t base = uint64_t(blockIdx.x) * kPTile + uint64_t(w) * (32 * kPItems);
   uint32_t c0 = 0, c1 = 0, c2 = 0;
+  int k[kPItems];
 #pragma unroll
-  for (int r = 0; r < kPItems; ++r) {
+  for (int r = 0; r < kPItems; ++r) {  // no branch or vote between the 8 items' loads (1 M: 5.9 -> 3.7 us)
     const uint64_t idx = base + uint64_t(r) * 32 + lane;
     uint64_t item;
     float d2;
-    const int k = idx < n ? cls(idx, item, d2) : 3;
-    c0 += __popc(__ballot_sync(0xffffffffu, k == 0));
-    c1 += __popc(__ballot_sync(0xffffffffu, k == 1));
-    c2 += __popc(__ballot_sync(0xffffffffu, k == 2));
+    k[r] = cls(min(idx, n - 1), item, d2);
+    if (idx >= n) k[r] = 3;
+  }
+#pragma unroll
+  for (int r = 0; r < kPItems; ++r) {
+    c0 += __popc(__ballot_sync(0xffffffffu, k[r] == 0));
+    c1 += __popc(__ballot_sync(0xffffffffu, k[r] == 1));
+    c2 += __popc(__ballot_sync(0xffffffffu, k[r] == 2));
   }
   if (lane == 0) {
     wc[w][0] = c0;
@@ -98,45 +110,57 @@ __global__ void __launch_bounds__(kPT) part_count(Cls cls, uint64_t n, uint32_t*
   }
 }
 
-// one block: exclusive scan of each class's tile counts, and the class totals
+// one block: exclusive scan of the three classes' tile counts together, and the class totals
 __global__ void __launch_bounds__(1024) part_scan(const uint32_t* tile_counts, uint32_t* tile_offs, uint32_t tiles,
-                                                  uint32_t* totals) {
-  __shared__ uint32_t ws[32];
-  __shared__ uint32_t carry;
+                                                  uint64_t n_items, const uint32_t* n_dev, uint32_t* totals) {
+  __shared__ uint32_t ws[3][32];
+  __shared__ uint32_t carry[3];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  for (int c = 0; c < 3; ++c) {
-    if (tid == 0) carry = 0;
-    __syncthreads();
-    for (uint32_t start = 0; start < tiles; start += 1024) {
-      const uint32_t i = start + tid;
-      const uint32_t x = i < tiles ? tile_counts[uint64_t(c) * tiles + i] : 0u;
-      const uint32_t incl = warp_scan_incl(x, lane);
-      if (lane == 31) ws[w] = incl;
-      __syncthreads();
-      if (w == 0) {
-        const uint32_t v = ws[lane];
-        ws[lane] = warp_scan_incl(v, lane) - v;
-      }
-      __syncthreads();
-      const uint32_t cc = carry;
-      if (i < tiles) tile_offs[uint64_t(c) * tiles + i] = cc + ws[w] + incl - x;
-      __syncthreads();
-      if (tid == 1023) carry = cc + ws[w] + incl;
-      __syncthreads();
+  const uint32_t used = uint32_t((part_items(n_items, n_dev) + kPTile - 1) / kPTile);
+  if (tid < 3) carry[tid] = 0;
+  __syncthreads();
+  for (uint32_t start = 0; start < used; start += 1024) {
+    const uint32_t i = start + tid;
+    uint32_t x[3], incl[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[c] = i < used ? tile_counts[uint64_t(c) * tiles + i] : 0u;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      incl[c] = warp_scan_incl(x[c], lane);
+      if (lane == 31) ws[c][w] = incl[c];
     }
-    if (tid == 0) totals[c] = carry;
+    __syncthreads();
+    if (w < 3) {
+      const uint32_t v = ws[w][lane];
+      ws[w][lane] = warp_scan_incl(v, lane) - v;
+    }
+    __syncthreads();
+    uint32_t at[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      at[c] = carry[c] + ws[c][w] + incl[c];
+      if (i < used) tile_offs[uint64_t(c) * tiles + i] = at[c] - x[c];
+    }
+    __syncthreads();
+    if (tid == 1023)
+      for (int c = 0; c < 3; ++c) carry[c] = at[c];
     __syncthreads();
   }
+  if (tid < 3) totals[tid] = carry[tid];
 }
 
-// writes each item at its class's tile offset + rank in index order; class 1 lands at out1_base +
+// writes each item at its class's tile offset + rank in index order; class 1 lands at *out1_from +
 // position, class 0 optionally also writes its squared distance
 template <class Cls>
-__global__ void __launch_bounds__(kPT) part_scatter(Cls cls, uint64_t n, const uint32_t* tile_offs, uint32_t tiles,
-                                                    uint64_t* out0, float* d2_0, uint64_t* out1, uint64_t out1_base,
+__global__ void __launch_bounds__(kPT) part_scatter(Cls cls, uint64_t n_items, const uint32_t* n_dev,
+                                                    const uint32_t* tile_offs, uint32_t tiles, uint64_t* out0,
+                                                    float* d2_0, uint64_t* out1, const uint32_t* out1_from,
                                                     uint64_t* out2) {
   __shared__ uint32_t wc[kPWarps][3];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint64_t n = part_items(n_items, n_dev);
+  if (uint64_t(blockIdx.x) * kPTile >= n) return;
+  const uint64_t out1_base = out1_from ? *out1_from : 0;
   const uint64_t base = uint64_t(blockIdx.x) * kPTile + uint64_t(w) * (32 * kPItems);
   int k[kPItems];
   uint64_t item[kPItems];
@@ -145,7 +169,11 @@ __global__ void __launch_bounds__(kPT) part_scatter(Cls cls, uint64_t n, const u
 #pragma unroll
   for (int r = 0; r < kPItems; ++r) {
     const uint64_t idx = base + uint64_t(r) * 32 + lane;
-    k[r] = idx < n ? cls(idx, item[r], d2[r]) : 3;
+    k[r] = cls(min(idx, n - 1), item[r], d2[r]);
+    if (idx >= n) k[r] = 3;
+  }
+#pragma unroll
+  for (int r = 0; r < kPItems; ++r) {
     c0 += __popc(__ballot_sync(0xffffffffu, k[r] == 0));
     c1 += __popc(__ballot_sync(0xffffffffu, k[r] == 1));
     c2 += __popc(__ballot_sync(0xffffffffu, k[r] == 2));
@@ -184,74 +212,98 @@ __global__ void __launch_bounds__(kPT) part_scatter(Cls cls, uint64_t n, const u
   }
 }
 
-// One block: flags the k smallest of n keys (k >= 1, k < n), equal keys by position.  Four 8-bit
-// radix-select passes find the k-th smallest key T and how many of the keys equal to T are kept;
-// the keys below T and the first of those equal to T (a block-wide scan of per-thread counts over
-// contiguous chunks gives their positional ranks) are flagged.
+// One block: flags the k smallest of *n_dev keys (k >= 1), equal keys by position; nothing when
+// there are no more than k.  Radix-select passes of 11 bits, from the highest bit in which the
+// keys differ, find the k-th smallest key T and how many of the keys equal to T are kept; the keys
+// below T and the first of those equal to T (each warp ranks a contiguous part, a scan over the
+// warps' counts) are flagged.
+// One SM's shared-memory atomics are the time.  With 8-bit digits from bit 31 the first digit of
+// 31 000 squared distances was two or three values (their exponents), so nearly all atomics of a
+// warp hit one counter: 26 us, 15.5 now.  Counting a warp's equal digits first (match) took 51 us.
 constexpr uint32_t kSelectSmemKeys = 40960;  // 160 KB: candidates up to this count are read once
-__global__ void __launch_bounds__(1024) select_keep(const uint32_t* gkeys, uint32_t n, uint32_t k, uint8_t* keep) {
-  extern __shared__ uint32_t skeys[];  // n keys when n <= kSelectSmemKeys (dynamic size 0 otherwise)
-  __shared__ uint32_t hist[256];
-  __shared__ uint32_t s_prefix, s_mask, s_rem;
+constexpr int kSelectBits = 11, kSelectBins = 1 << kSelectBits;
+__global__ void __launch_bounds__(1024) select_keep(const uint32_t* gkeys, const uint32_t* n_dev, uint32_t k,
+                                                    uint8_t* keep) {
+  extern __shared__ uint32_t skeys[];  // kSelectSmemKeys keys
+  const uint32_t n = *n_dev;
+  if (n <= k) return;
+  __shared__ uint32_t hist[kSelectBins];
+  __shared__ uint32_t s_prefix, s_rem, s_min, s_max;
   __shared__ uint32_t wsum[32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const bool cached = n <= kSelectSmemKeys;
-  if (cached)
-    for (uint32_t i = tid; i < n; i += 1024) skeys[i] = gkeys[i];
-  const uint32_t* keys = cached ? skeys : gkeys;
   if (tid == 0) {
-    s_prefix = 0;
-    s_mask = 0;
+    s_min = 0xffffffffu;
+    s_max = 0;
     s_rem = k;
   }
   __syncthreads();
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    if (tid < 256) hist[tid] = 0;
+  uint32_t lo = 0xffffffffu, hi = 0;
+#pragma unroll 8
+  for (uint32_t i = tid; i < n; i += 1024) {
+    const uint32_t key = gkeys[i];
+    if (cached) skeys[i] = key;
+    lo = min(lo, key);
+    hi = max(hi, key);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) {
+    atomicMin(&s_min, lo);
+    atomicMax(&s_max, hi);
+  }
+  __syncthreads();
+  const uint32_t* keys = cached ? skeys : gkeys;
+  int top = 32 - __clz(s_min ^ s_max);  // bits below this one differ
+  if (tid == 0) s_prefix = top < 32 ? s_min >> top << top : 0u;
+  __syncthreads();
+  while (top > 0) {
+    const int shift = max(0, top - kSelectBits);
+    const uint32_t digits = (1u << (top - shift)) - 1u, mask = top < 32 ? ~0u << top : 0u, prefix = s_prefix;
+    hist[tid] = hist[tid + 1024] = 0;
     __syncthreads();
-    const uint32_t prefix = s_prefix, mask = s_mask;
+#pragma unroll 4
     for (uint32_t i = tid; i < n; i += 1024) {
       const uint32_t key = keys[i];
-      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
+      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & digits], 1u);
     }
     __syncthreads();
-    if (w == 0) {  // the digit whose bucket holds the s_rem-th smallest remaining key
-      uint32_t c = 0;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) c += hist[8 * lane + b];
-      const uint32_t incl = warp_scan_incl(c, lane), rem = s_rem;
-      const uint32_t hit = __ballot_sync(0xffffffffu, incl >= rem);
-      if (lane == __ffs(hit) - 1) {
-        uint32_t cum = incl - c;
-        int d = 8 * lane;
-        for (int b = 0; b < 8; ++b, ++d) {
-          if (cum + hist[d] >= rem) break;
-          cum += hist[d];
-        }
-        s_prefix = prefix | (uint32_t(d) << shift);
-        s_mask = mask | (255u << shift);
-        s_rem = rem - cum;
-      }
+    // the digit whose bucket holds the s_rem-th smallest remaining key: two buckets per thread
+    const uint32_t h0 = hist[2 * tid], h1 = hist[2 * tid + 1], rem = s_rem;
+    const uint32_t incl = warp_scan_incl(h0 + h1, lane);
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+      const uint32_t v = wsum[lane];
+      wsum[lane] = warp_scan_incl(v, lane) - v;
     }
     __syncthreads();
+    const uint32_t below = wsum[w] + incl - h0 - h1;
+    if (below < rem && rem <= below + h0 + h1) {
+      const bool second = rem > below + h0;
+      s_prefix = prefix | ((2u * tid + second) << shift);
+      s_rem = rem - below - (second ? h0 : 0u);
+    }
+    __syncthreads();
+    top = shift;
   }
   const uint32_t T = s_prefix, rem = s_rem;
-  const uint32_t chunk = (n + 1023) / 1024, c0 = min(n, tid * chunk), c1 = min(n, c0 + chunk);
+  const uint32_t chunk = (n + 1023) / 1024 * 32, c0 = w * chunk;
   uint32_t eq = 0;
-  for (uint32_t i = c0; i < c1; ++i) eq += keys[i] == T;
-  const uint32_t incl = warp_scan_incl(eq, lane);
-  if (lane == 31) wsum[w] = incl;
-  __syncthreads();
-  if (w == 0) {
-    const uint32_t v = wsum[lane];
-    wsum[lane] = warp_scan_incl(v, lane) - v;
+  for (uint32_t r = 0; r < chunk; r += 32) {
+    const uint32_t i = c0 + r + lane;
+    eq += __popc(__ballot_sync(0xffffffffu, i < n && keys[i] == T));
   }
+  if (lane == 0) wsum[w] = eq;
   __syncthreads();
-  uint32_t before = wsum[w] + incl - eq;
-  for (uint32_t i = c0; i < c1; ++i) {
-    const uint32_t key = keys[i];
-    bool kp = key < T;
-    if (key == T) kp = before++ < rem;
-    keep[i] = kp ? 1 : 0;
+  uint32_t before = 0;
+  for (int ww = 0; ww < w; ++ww) before += wsum[ww];
+  for (uint32_t r = 0; r < chunk; r += 32) {
+    const uint32_t i = c0 + r + lane;
+    const uint32_t key = i < n ? keys[i] : 0xffffffffu;
+    const uint32_t same = __ballot_sync(0xffffffffu, i < n && key == T);
+    if (i < n) keep[i] = key < T || (key == T && before + __popc(same & ((1u << lane) - 1u)) < rem) ? 1 : 0;
+    before += __popc(same);
   }
 }
 
@@ -260,24 +312,29 @@ __global__ void far_field_kernel(float* pos, float* vel, float* temp, const uint
                                  const float* coarse, uint32_t cn, float cdx, float ox, float oy, float oz, float far_dt) {
   for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
     const uint64_t i = idx ? idx[k] : k;
-    const float vy = __fsub_rn(vel[3 * i + 1], __fmul_rn(9.81f, far_dt));
+    // every input is loaded before the first store, so that the loads are in flight together (480 000
+    // of 1 M particles: 11.6 -> 8.4 us)
+    const float vy0 = vel[3 * i + 1], px = pos[3 * i], py0 = pos[3 * i + 1], pz = pos[3 * i + 2], t = temp[i];
+    const float vy = __fsub_rn(vy0, __fmul_rn(9.81f, far_dt));
     vel[3 * i + 1] = vy;
-    const float py = __fadd_rn(pos[3 * i + 1], __fmul_rn(vy, far_dt));
+    const float py = __fadd_rn(py0, __fmul_rn(vy, far_dt));
     pos[3 * i + 1] = py;
-    const int64_t gx = as_isize(__fdiv_rn(__fsub_rn(pos[3 * i], ox), cdx));
+    const int64_t gx = as_isize(__fdiv_rn(__fsub_rn(px, ox), cdx));
     const int64_t gy = as_isize(__fdiv_rn(__fsub_rn(py, oy), cdx));
-    const int64_t gz = as_isize(__fdiv_rn(__fsub_rn(pos[3 * i + 2], oz), cdx));
+    const int64_t gz = as_isize(__fdiv_rn(__fsub_rn(pz, oz), cdx));
     if (gx >= 0 && gy >= 0 && gz >= 0 && gx < int64_t(cn) && gy < int64_t(cn) && gz < int64_t(cn)) {
       const float field = coarse[gx + gy * int64_t(cn) + gz * int64_t(cn) * int64_t(cn)];
-      const float t = temp[i];
       temp[i] = __fadd_rn(t, __fmul_rn(__fmul_rn(__fsub_rn(field, t), 0.02f), far_dt));
     }
   }
 }
 
-// cell key of near particle k (simulation.rs:889-905), or `dead` when skipped
+// cell key of near particle k (simulation.rs:889-905), or `dead` when skipped; empties every cell's run
 __global__ void coarse_keys(const float* pos, const uint8_t* active, const uint64_t* idx, uint64_t n, uint32_t cn,
-                            float inv_dx, float ox, float oy, float oz, uint32_t dead, uint32_t* keys) {
+                            float inv_dx, float ox, float oy, float oz, uint32_t dead, uint32_t* keys,
+                            uint32_t* run_start, uint32_t* run_end) {
+  for (uint64_t c = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; c < dead; c += uint64_t(gridDim.x) * blockDim.x)
+    run_start[c] = run_end[c] = 0u;
   for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
     const uint64_t i = idx ? idx[k] : k;
     uint32_t key = dead;
@@ -292,21 +349,16 @@ __global__ void coarse_keys(const float* pos, const uint8_t* active, const uint6
   }
 }
 
-// the near particles' (temperature x mass, mass) in cell order (simulation.rs:906-908)
+// the near particles' (temperature x mass, mass) in cell order (simulation.rs:906-908), and each
+// cell's run [start, end) in that order (cells without particles keep start == end == 0)
 __global__ void coarse_gather(const float* mass, const float* temp, const uint64_t* idx, const uint32_t* perm,
-                              uint64_t n, float* tm, float* m) {
+                              const uint32_t* skeys, uint64_t n, uint32_t dead, float2* tm_m, uint32_t* run_start,
+                              uint32_t* run_end) {
   for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
     const uint64_t kk = perm[k];
     const uint64_t i = idx ? idx[kk] : kk;
     const float mi = fmaxf(mass[i], 1e-6f);
-    tm[k] = __fmul_rn(temp[i], mi);
-    m[k] = mi;
-  }
-}
-
-// each cell's run [start, end) in the sorted order (cells without particles keep start == end == 0)
-__global__ void coarse_runs(const uint32_t* skeys, uint64_t n, uint32_t dead, uint32_t* run_start, uint32_t* run_end) {
-  for (uint64_t k = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; k < n; k += uint64_t(gridDim.x) * blockDim.x) {
+    tm_m[k] = make_float2(__fmul_rn(temp[i], mi), mi);
     const uint32_t key = skeys[k];
     if (key == dead) continue;
     if (k == 0 || skeys[k - 1] != key) run_start[key] = uint32_t(k);
@@ -315,43 +367,45 @@ __global__ void coarse_runs(const uint32_t* skeys, uint64_t n, uint32_t dead, ui
 }
 
 // One warp per cell: the warp stages its cell's run in shared memory 256 entries at a time
-// (coalesced loads) and lane 0 adds them in order, as the reference's serial loop does.
+// (coalesced loads) and lane 0 adds them in order, as the reference's serial loop does; then the
+// cell relaxes toward the injected temperature (simulation.rs:914-923).  The order is the
+// reference's, so the two chains of additions are the time: 8 entries are loaded ahead of them.
 constexpr int kSumBatch = 256;
-__global__ void __launch_bounds__(256) coarse_sums(const uint32_t* run_start, const uint32_t* run_end, const float* tm,
-                                                   const float* m, uint64_t cells, float* cell_tm, float* cell_m) {
-  __shared__ float st[8][2][kSumBatch];
+__global__ void __launch_bounds__(256) coarse_sums(const uint32_t* run_start, const uint32_t* run_end, const float2* tm_m,
+                                                   uint64_t cells, const float* coarse, float blend, float* blended) {
+  __shared__ float2 st[8][kSumBatch];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (uint64_t c = blockIdx.x * 8ull + w; c < cells; c += uint64_t(gridDim.x) * 8) {
-    const uint32_t s0 = run_start[c], e0 = run_end[c];
+    const uint32_t s0 = run_start ? run_start[c] : 0u, e0 = run_start ? run_end[c] : 0u;
     float a = 0.0f, b = 0.0f;
     for (uint32_t base = s0; base < e0; base += kSumBatch) {
       const uint32_t cnt = min(uint32_t(kSumBatch), e0 - base);
-      for (uint32_t t = lane; t < cnt; t += 32) {
-        st[w][0][t] = tm[base + t];
-        st[w][1][t] = m[base + t];
-      }
+      for (uint32_t t = lane; t < cnt; t += 32) st[w][t] = tm_m[base + t];
       __syncwarp();
-      if (lane == 0)
-        for (uint32_t t = 0; t < cnt; ++t) {
-          a = __fadd_rn(a, st[w][0][t]);
-          b = __fadd_rn(b, st[w][1][t]);
+      if (lane == 0) {
+        uint32_t t = 0;
+        for (; t + 8 <= cnt; t += 8) {
+          float2 q[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) q[u] = st[w][t + u];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            a = __fadd_rn(a, q[u].x);
+            b = __fadd_rn(b, q[u].y);
+          }
         }
+        for (; t < cnt; ++t) {
+          a = __fadd_rn(a, st[w][t].x);
+          b = __fadd_rn(b, st[w][t].y);
+        }
+      }
       __syncwarp();
     }
     if (lane == 0) {
-      cell_tm[c] = a;
-      cell_m[c] = b;
+      float t = coarse[c];
+      if (b > 1e-6f) t = __fadd_rn(t, __fmul_rn(__fsub_rn(__fdiv_rn(a, b), t), blend));
+      blended[c] = t;
     }
-  }
-}
-
-// relaxation toward the injected temperature (simulation.rs:914-923)
-__global__ void coarse_blend(const float* coarse, const float* cell_tm, const float* cell_m, uint64_t cells, float blend,
-                             float* blended) {
-  for (uint64_t c = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; c < cells; c += uint64_t(gridDim.x) * blockDim.x) {
-    float t = coarse[c];
-    if (cell_m[c] > 1e-6f) t = __fadd_rn(t, __fmul_rn(__fsub_rn(__fdiv_rn(cell_tm[c], cell_m[c]), t), blend));
-    blended[c] = t;
   }
 }
 
@@ -396,43 +450,55 @@ __device__ __forceinline__ uint8_t phase_hop(uint16_t m, uint8_t cur, float t) {
 
 // MpssBuffer housekeeping after the substep (ae_engine/src/lib.rs:347-358): per active particle,
 // reflecting world bounds (mpss.rs:449-476), temperature clamp (:479-497), phase transitions with
-// up to 3 hops (:500-548), in that order; passes selects them (1, 2, 4).  The loop bounds are
-// warp-uniform so the transition count is a warp ballot.
+// up to 3 hops (:500-548), in that order; passes selects them (1, 2, 4).  Each CTA adds its
+// transitions with one atomic: one per warp, 31 000 on one address, took longer
+// than the passes (1 M particles, most of them in transition: 30 -> 14.6 us).
 __global__ void housekeeping_kernel(float* pos, float* vel, float* temp, uint8_t* phase, const uint16_t* mat,
                                     const uint8_t* active, uint64_t n, float x0, float y0, float z0, float x1, float y1,
                                     float z1, float tmin, float tmax, uint32_t passes, uint32_t* transitions) {
+  // a particle's inputs are all loaded before anything is decided, the velocity components once the
+  // bounds are known: two memory latencies per particle instead of one per component and pass
   const float lo[3] = {x0, y0, z0}, hi[3] = {x1, y1, z1};
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t base = uint64_t(blockIdx.x) * blockDim.x; base < n; base += stride) {
-    const uint64_t i = base + threadIdx.x;
-    bool changed = false;
-    if (i < n && (!active || active[i])) {
+  const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  bool changed = false;
+  if (i < n) {
+    const bool on = !active || active[i];
+    float p[3] = {0.0f, 0.0f, 0.0f}, v[3] = {0.0f, 0.0f, 0.0f}, t = 0.0f;
+    uint16_t m = 0;
+    uint8_t cur = 0;
+    if (passes & 1u)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) p[d] = pos[3 * i + d];
+    if (passes & 6u) t = temp[i];
+    if (passes & 4u) {
+      m = mat[i];
+      cur = phase[i];
+    }
+    if (on) {
       if (passes & 1u) {
+        bool below[3], above[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          const float p = pos[3 * i + d];
-          if (p < lo[d]) {
-            pos[3 * i + d] = lo[d];
-            const float v = vel[3 * i + d];
-            if (v < 0.0f) vel[3 * i + d] = __fmul_rn(-v, 0.5f);
-          } else if (p > hi[d]) {
-            pos[3 * i + d] = hi[d];
-            const float v = vel[3 * i + d];
-            if (v > 0.0f) vel[3 * i + d] = __fmul_rn(-v, 0.5f);
-          }
+          below[d] = p[d] < lo[d];
+          above[d] = !below[d] && p[d] > hi[d];
+          if (below[d] || above[d]) v[d] = vel[3 * i + d];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (!(below[d] || above[d])) continue;
+          pos[3 * i + d] = below[d] ? lo[d] : hi[d];
+          if (below[d] ? v[d] < 0.0f : v[d] > 0.0f) vel[3 * i + d] = __fmul_rn(-v[d], 0.5f);
         }
       }
       if (passes & 2u) {
-        const float t = temp[i];
+        const float before = t;
         if (t > tmax)
-          temp[i] = tmax;
+          t = tmax;
         else if (t < tmin)
-          temp[i] = tmin;
+          t = tmin;
+        if (t != before) temp[i] = t;
       }
       if (passes & 4u) {
-        const float t = temp[i];
-        const uint16_t m = mat[i];
-        const uint8_t cur = phase[i];
         uint8_t next = cur;
         for (int hop = 0; hop < 3; ++hop) {
           const uint8_t h = phase_hop(m, next, t);
@@ -445,9 +511,9 @@ __global__ void housekeeping_kernel(float* pos, float* vel, float* temp, uint8_t
         }
       }
     }
-    const uint32_t c = __popc(__ballot_sync(0xffffffffu, changed));
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(transitions, c);
   }
+  const int c = __syncthreads_count(changed);
+  if (threadIdx.x == 0 && c) atomicAdd(transitions, uint32_t(c));
 }
 
 inline unsigned grid_for(uint64_t n, int threads) {
@@ -470,45 +536,45 @@ int bits_for(uint64_t v) {  // bits needed to hold values 0..v
   } while (0)
 
 LodWork::~LodWork() {
-  void* ps[] = {tile_counts_, tile_offs_, totals_, near_tmp_, near_key_, keep_, tm_, m_, cell_a_, cell_b_, field_tmp_,
+  void* ps[] = {tile_counts_, tile_offs_, totals_, near_tmp_, near_key_, keep_, tm_m_, field_tmp_,
                 run_start_, run_end_};
   for (void* p : ps)
     if (p) cudaFree(p);
+  if (host_totals_) cudaFreeHost(host_totals_);
   sort_scratch_free(sort_);
 }
 
 cudaError_t LodWork::grow(uint64_t count, uint64_t cells) {
   if (count > cap_ || !totals_) {
     const uint64_t cap = std::max<uint64_t>(count, std::max<uint64_t>(cap_ * 2, 4096));
-    void* ps[] = {tile_counts_, tile_offs_, near_tmp_, near_key_, keep_, tm_, m_};
+    void* ps[] = {tile_counts_, tile_offs_, near_tmp_, near_key_, keep_, tm_m_};
     for (void* p : ps)
       if (p) cudaFree(p);
     tile_counts_ = tile_offs_ = near_key_ = nullptr;
     near_tmp_ = nullptr;
     keep_ = nullptr;
-    tm_ = m_ = nullptr;
+    tm_m_ = nullptr;
     cap_ = 0;
     const uint64_t tiles = (cap + kPTile - 1) / kPTile;
     LOD_TRY(cudaMalloc(&tile_counts_, sizeof(uint32_t) * 3 * tiles));
     LOD_TRY(cudaMalloc(&tile_offs_, sizeof(uint32_t) * 3 * tiles));
-    if (!totals_) LOD_TRY(cudaMalloc(&totals_, sizeof(uint32_t) * 4));
+    // [class totals of the first partition, transitions, class totals of the second]
+    if (!totals_) LOD_TRY(cudaMalloc(&totals_, sizeof(uint32_t) * 8));
+    if (!host_totals_) LOD_TRY(cudaHostAlloc(&host_totals_, sizeof(uint32_t) * 4, cudaHostAllocDefault));
     LOD_TRY(cudaMalloc(&near_tmp_, sizeof(uint64_t) * cap));
     LOD_TRY(cudaMalloc(&near_key_, sizeof(uint32_t) * cap));
     LOD_TRY(cudaMalloc(&keep_, cap));
-    LOD_TRY(cudaMalloc(&tm_, sizeof(float) * cap));
-    LOD_TRY(cudaMalloc(&m_, sizeof(float) * cap));
+    LOD_TRY(cudaMalloc(&tm_m_, sizeof(float2) * cap));
     LOD_TRY(sort_scratch_alloc(sort_, cap));
     cap_ = cap;
   }
   if (cells > cells_cap_) {
-    void* ps[] = {cell_a_, cell_b_, field_tmp_, run_start_, run_end_};
+    void* ps[] = {field_tmp_, run_start_, run_end_};
     for (void* p : ps)
       if (p) cudaFree(p);
-    cell_a_ = cell_b_ = field_tmp_ = nullptr;
+    field_tmp_ = nullptr;
     run_start_ = run_end_ = nullptr;
     cells_cap_ = 0;
-    LOD_TRY(cudaMalloc(&cell_a_, sizeof(float) * cells));
-    LOD_TRY(cudaMalloc(&cell_b_, sizeof(float) * cells));
     LOD_TRY(cudaMalloc(&field_tmp_, sizeof(float) * cells));
     LOD_TRY(cudaMalloc(&run_start_, sizeof(uint32_t) * cells));
     LOD_TRY(cudaMalloc(&run_end_, sizeof(uint32_t) * cells));
@@ -526,44 +592,33 @@ cudaError_t LodWork::classify(const float* pos, const uint8_t* active, uint64_t 
   const uint32_t tiles = uint32_t((count + kPTile - 1) / kPTile);
   // squared distances as the reference computes them (simulation.rs:484-485)
   const PosClass pc{pos, active, player[0], player[1], player[2], near_dist * near_dist, mid_dist * mid_dist};
-  part_count<PosClass><<<tiles, kPT, 0, s>>>(pc, count, tile_counts_, tiles);
-  part_scan<<<1, 1024, 0, s>>>(tile_counts_, tile_offs_, tiles, totals_);
-  part_scatter<PosClass><<<tiles, kPT, 0, s>>>(pc, count, tile_offs_, tiles, near_tmp_,
-                                               reinterpret_cast<float*>(near_key_), mid_out, uint64_t(0), far_out);
-  LOD_TRY(cudaGetLastError());
-  uint32_t tot[4] = {0, 0, 0, 0};
-  LOD_TRY(cudaMemcpyAsync(tot, totals_, sizeof(tot), cudaMemcpyDeviceToHost, s));
-  LOD_TRY(cudaStreamSynchronize(s));
-  const uint64_t n_near = tot[0], n_mid = tot[1], n_far = tot[2];
-  if (n_near <= max_near) {
-    if (n_near) LOD_TRY(cudaMemcpyAsync(near_out, near_tmp_, sizeof(uint64_t) * n_near, cudaMemcpyDeviceToDevice, s));
-    counts[0] = n_near;
-    counts[1] = n_mid;
-    counts[2] = n_far;
-    return cudaSuccess;
-  }
-  // cap (simulation.rs:519-530): the max_near smallest squared distances stay near, ties by index
-  if (max_near) {
-    const size_t sm = n_near <= kSelectSmemKeys ? sizeof(uint32_t) * n_near : 0;
+  part_count<PosClass><<<tiles, kPT, 0, s>>>(pc, count, nullptr, tile_counts_, tiles);
+  part_scan<<<1, 1024, 0, s>>>(tile_counts_, tile_offs_, tiles, count, nullptr, totals_);
+  part_scatter<PosClass><<<tiles, kPT, 0, s>>>(pc, count, nullptr, tile_offs_, tiles, near_tmp_,
+                                               reinterpret_cast<float*>(near_key_), mid_out, nullptr, far_out);
+  // cap (simulation.rs:519-530): the max_near smallest squared distances stay near, ties by index.
+  // The number of candidates stays on the device: the host waits once, for the final counts.
+  const uint32_t cap = uint32_t(std::min<uint64_t>(max_near, 0xffffffffu));
+  if (cap && cap < count) {
     if (!select_smem_set_) {
       LOD_TRY(cudaFuncSetAttribute(select_keep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(sizeof(uint32_t) * kSelectSmemKeys)));
       select_smem_set_ = true;
     }
-    select_keep<<<1, 1024, sm, s>>>(near_key_, uint32_t(n_near), uint32_t(max_near), keep_);
+    select_keep<<<1, 1024, sizeof(uint32_t) * kSelectSmemKeys, s>>>(near_key_, totals_, cap, keep_);
   }
-  else
-    LOD_TRY(cudaMemsetAsync(keep_, 0, n_near, s));
-  const uint32_t tiles2 = uint32_t((n_near + kPTile - 1) / kPTile);
-  const KeepClass kc{near_tmp_, keep_};
-  part_count<KeepClass><<<tiles2, kPT, 0, s>>>(kc, n_near, tile_counts_, tiles2);
-  part_scan<<<1, 1024, 0, s>>>(tile_counts_, tile_offs_, tiles2, totals_);
-  part_scatter<KeepClass><<<tiles2, kPT, 0, s>>>(kc, n_near, tile_offs_, tiles2, near_out, static_cast<float*>(nullptr),
-                                                 mid_out, n_mid, static_cast<uint64_t*>(nullptr));
+  const KeepClass kc{near_tmp_, keep_, totals_, cap};
+  part_count<KeepClass><<<tiles, kPT, 0, s>>>(kc, 0, totals_, tile_counts_, tiles);
+  part_scan<<<1, 1024, 0, s>>>(tile_counts_, tile_offs_, tiles, 0, totals_, totals_ + 4);
+  part_scatter<KeepClass><<<tiles, kPT, 0, s>>>(kc, 0, totals_, tile_offs_, tiles, near_out, static_cast<float*>(nullptr),
+                                                mid_out, totals_ + 1, static_cast<uint64_t*>(nullptr));
   LOD_TRY(cudaGetLastError());
-  counts[0] = max_near;
-  counts[1] = n_mid + (n_near - max_near);
-  counts[2] = n_far;
+  LOD_TRY(cudaMemcpyAsync(host_totals_, totals_, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  LOD_TRY(cudaStreamSynchronize(s));
+  const uint64_t n_near = host_totals_[0];
+  counts[0] = std::min<uint64_t>(n_near, max_near);
+  counts[1] = host_totals_[1] + (n_near - counts[0]);
+  counts[2] = host_totals_[2];
   return cudaSuccess;
 }
 
@@ -575,12 +630,14 @@ cudaError_t LodWork::housekeeping(float* pos, float* vel, float* temp, uint8_t* 
   if (n == 0) return cudaSuccess;
   LOD_TRY(grow(1, 0));
   LOD_TRY(cudaMemsetAsync(totals_ + 3, 0, sizeof(uint32_t), s));
-  housekeeping_kernel<<<grid_for(n, 256), 256, 0, s>>>(pos, vel, temp, phase, material, active, n, bmin[0], bmin[1],
-                                                      bmin[2], bmax[0], bmax[1], bmax[2], min_temp, max_temp, passes,
-                                                      totals_ + 3);
+  housekeeping_kernel<<<unsigned((n + 511) / 512), 512, 0, s>>>(pos, vel, temp, phase, material, active, n, bmin[0],
+                                                               bmin[1], bmin[2], bmax[0], bmax[1], bmax[2], min_temp,
+                                                               max_temp, passes, totals_ + 3);
   LOD_TRY(cudaGetLastError());
-  LOD_TRY(cudaMemcpyAsync(transitions, totals_ + 3, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  return cudaStreamSynchronize(s);
+  LOD_TRY(cudaMemcpyAsync(host_totals_, totals_ + 3, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  LOD_TRY(cudaStreamSynchronize(s));
+  *transitions = host_totals_[0];
+  return cudaSuccess;
 }
 
 cudaError_t LodWork::far_field(float* pos, float* vel, float* temp, const uint64_t* far_idx, uint64_t n,
@@ -598,29 +655,24 @@ cudaError_t LodWork::coarse_field(const float* pos, const float* mass, const flo
   const uint64_t cells = uint64_t(cn) * cn * cn;
   if (cells == 0) return cudaSuccess;
   LOD_TRY(grow(std::max<uint64_t>(n, 1), cells));
-  if (n == 0) {  // no particles: the injection adds nothing
-    LOD_TRY(cudaMemsetAsync(cell_a_, 0, sizeof(float) * cells, s));
-    LOD_TRY(cudaMemsetAsync(cell_b_, 0, sizeof(float) * cells, s));
-  }
-  if (n > 0) {
-    const uint32_t dead = uint32_t(cells);
-    const float inv_dx = 1.0f / cdx;
-    coarse_keys<<<grid_for(n, 256), 256, 0, s>>>(pos, active, near_idx, n, cn, inv_dx, origin[0], origin[1], origin[2],
-                                                dead, near_key_);
-    const uint32_t *sorted = nullptr, *perm = nullptr;
-    radix_sort_pairs(near_key_, n, bits_for(cells), sort_, s, &sorted, &perm);
-    coarse_gather<<<grid_for(n, 256), 256, 0, s>>>(mass, temp, near_idx, perm, n, tm_, m_);
-    LOD_TRY(cudaMemsetAsync(run_start_, 0, sizeof(uint32_t) * cells, s));
-    LOD_TRY(cudaMemsetAsync(run_end_, 0, sizeof(uint32_t) * cells, s));
-    coarse_runs<<<grid_for(n, 256), 256, 0, s>>>(sorted, n, dead, run_start_, run_end_);
-    coarse_sums<<<unsigned(std::min<uint64_t>((cells + 7) / 8, 148 * 16)), 256, 0, s>>>(run_start_, run_end_, tm_, m_,
-                                                                                      cells, cell_a_, cell_b_);
-  }
   const float inject_rate = 0.1f;
   const float blend = std::fmin(inject_rate * dt, 1.0f);
   const float alpha = 10.0f;
   const float coef = std::fmin(alpha * dt / (cdx * cdx), 0.16f);
-  coarse_blend<<<grid_for(cells, 256), 256, 0, s>>>(coarse, cell_a_, cell_b_, cells, blend, field_tmp_);
+  if (n > 0) {
+    const uint32_t dead = uint32_t(cells);
+    const float inv_dx = 1.0f / cdx;
+    coarse_keys<<<grid_for(std::max(n, cells), 256), 256, 0, s>>>(pos, active, near_idx, n, cn, inv_dx, origin[0],
+                                                                 origin[1], origin[2], dead, near_key_, run_start_,
+                                                                 run_end_);
+    const uint32_t *sorted = nullptr, *perm = nullptr;
+    radix_sort_pairs(near_key_, n, bits_for(cells), sort_, s, &sorted, &perm);
+    coarse_gather<<<grid_for(n, 256), 256, 0, s>>>(mass, temp, near_idx, perm, sorted, n, dead, tm_m_, run_start_,
+                                                  run_end_);
+  }
+  // without particles the injection adds nothing
+  coarse_sums<<<unsigned(std::min<uint64_t>((cells + 7) / 8, 148 * 16)), 256, 0, s>>>(
+      n > 0 ? run_start_ : nullptr, run_end_, tm_m_, cells, coarse, blend, field_tmp_);
   coarse_diffuse<<<grid_for(cells, 256), 256, 0, s>>>(field_tmp_, cn, coef, coarse);
   return cudaGetLastError();
 }

@@ -49,14 +49,12 @@ class LodWork {
   bool select_smem_set_ = false;
   uint32_t* tile_counts_ = nullptr;  // [3][tiles]
   uint32_t* tile_offs_ = nullptr;    // [3][tiles]
-  uint32_t* totals_ = nullptr;       // [4]: class totals, housekeeping transition count
+  uint32_t* totals_ = nullptr;       // [8]: class totals, housekeeping transitions, totals after the cap
+  uint32_t* host_totals_ = nullptr;  // [4] pinned: where the host reads them
   uint64_t* near_tmp_ = nullptr;     // [cap] near candidates (ascending index)
   uint32_t* near_key_ = nullptr;     // [cap] their squared distance, as bits; later cell keys
   uint8_t* keep_ = nullptr;          // [cap]
-  float* tm_ = nullptr;              // [cap] temperature x mass (coarse field), sorted by cell
-  float* m_ = nullptr;               // [cap] mass, sorted by cell
-  float* cell_a_ = nullptr;          // [cells] sums of temperature x mass
-  float* cell_b_ = nullptr;          // [cells] sums of mass
+  float2* tm_m_ = nullptr;           // [cap] (temperature x mass, mass) of the coarse field, sorted by cell
   float* field_tmp_ = nullptr;       // [cells]
   uint32_t* run_start_ = nullptr;    // [cells] each cell's run in the cell-sorted near list
   uint32_t* run_end_ = nullptr;      // [cells]
