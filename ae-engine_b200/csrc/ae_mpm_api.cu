@@ -48,8 +48,8 @@ struct ae_mpm_ctx {
   aemp::CkWork* ck = nullptr;
   void* dstage = nullptr;
   size_t dstage_bytes = 0;
-  // completion events of the drop-in's whole-array copies back to the host
-  cudaEvent_t out_ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  // completion events of a staged drop-in call's pieces on their way back to the host
+  cudaEvent_t out_ev[8] = {};
 };
 
 struct ae_mpm_world {
@@ -152,87 +152,149 @@ ae_mpm_particles pinned_view(ae_mpm_ctx* ctx, uint64_t n) {
   return v;
 }
 
-// Drop-in calls whose indices are ascending and select a quarter or more of the buffer copy the
-// buffer's arrays whole and gather / scatter the selected particles on the device.  `full`: every
-// field travels (reference mode); otherwise position, velocity and mass only, with F = I, C = 0,
-// J = 1 (the velocity-only substep reads none of them and writes back position and velocity).
-__global__ void dropin_gather_kernel(ae_mpm_particles src, const uint64_t* __restrict__ idx, uint64_t n,
-                                     ae_mpm_particles dst, int full) {
-  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const uint64_t i = idx[k];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    dst.pos[3 * k + a] = src.pos[3 * i + a];
-    dst.vel[3 * k + a] = src.vel[3 * i + a];
-  }
-  dst.mass[k] = src.mass[i];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) {
-    dst.strain[9 * k + q] = full ? src.strain[9 * i + q] : ((q % 4 == 0) ? 1.0f : 0.0f);
-    dst.c[9 * k + q] = full ? src.c[9 * i + q] : 0.0f;
-  }
-  dst.jacobian[k] = full ? src.jacobian[i] : 1.0f;
-  dst.material_idx[k] = full ? src.material_idx[i] : uint16_t(0);
-}
-
-__global__ void dropin_scatter_kernel(ae_mpm_particles src, const uint64_t* __restrict__ idx, uint64_t n,
-                                      ae_mpm_particles dst, int full) {
-  const uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const uint64_t i = idx[k];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    dst.pos[3 * i + a] = src.pos[3 * k + a];
-    dst.vel[3 * i + a] = src.vel[3 * k + a];
-  }
-  if (full) {
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      dst.strain[9 * i + q] = src.strain[9 * k + q];
-      dst.c[9 * i + q] = src.c[9 * k + q];
-    }
-    dst.jacobian[i] = src.jacobian[k];
+// Rows of kRow bytes between the caller's array and a packed one.  The indices ascend strictly, so a
+// list whose ends are as far apart as it is long is one block of memory.
+template <size_t kRow>
+void copy_rows(char* packed, char* rows, const uint64_t* idx, uint64_t n, bool pack) {
+  if (idx[n - 1] - idx[0] == n - 1) {
+    char* r = rows + idx[0] * kRow;
+    std::memcpy(pack ? packed : r, pack ? r : packed, n * kRow);
+  } else if (pack) {
+    for (uint64_t k = 0; k < n; ++k) std::memcpy(packed + k * kRow, rows + idx[k] * kRow, kRow);
+  } else {
+    for (uint64_t k = 0; k < n; ++k) std::memcpy(rows + idx[k] * kRow, packed + k * kRow, kRow);
   }
 }
 
-// Host copy between the caller's (pageable) arrays and pinned staging, split over up to 8 threads
-// for large arrays: the driver's own pageable copies run on one thread at a fraction of the link's
-// bandwidth, while copies from pinned staging run at the link's speed.
-void host_copy(void* dst, const void* src, size_t bytes) {
-  const int t_max = bytes >= (size_t(8) << 20) ? std::min(8, omp_get_max_threads()) : 1;
-  if (t_max <= 1) {
-    std::memcpy(dst, src, bytes);
-    return;
-  }
-  const size_t chunk = ((bytes + size_t(t_max) - 1) / size_t(t_max) + 63) & ~size_t(63);
-#pragma omp parallel for num_threads(t_max) schedule(static)
-  for (int t = 0; t < t_max; ++t) {
-    const size_t lo = size_t(t) * chunk;
-    if (lo < bytes)
-      std::memcpy(static_cast<char*>(dst) + lo, static_cast<const char*>(src) + lo, std::min(chunk, bytes - lo));
-  }
-}
-
-// Carves the device staging of a whole-array drop-in call: the buffer's arrays (capacity particles),
-// the index list and the selected particles (n), each region on a 16-byte boundary.
-struct DropinLayout {
-  size_t off[16];
-  size_t bytes;
+// One array of a staged drop-in call: the caller's rows and their packed place in the staging.
+struct DropinArray {
+  char* rows;
+  size_t row, off;
 };
-DropinLayout dropin_layout(uint64_t capacity, uint64_t n, bool full) {
-  const size_t sz[15] = {12 * capacity, 12 * capacity, 4 * capacity, full ? 36 * capacity : 0, full ? 36 * capacity : 0,
-                         full ? 4 * capacity : 0, full ? 2 * capacity : 0, 8 * n, 12 * n, 12 * n, 36 * n, 4 * n, 36 * n,
-                         4 * n, 2 * n};
-  DropinLayout l{};
-  size_t o = 0;
-  for (int r = 0; r < 15; ++r) {
-    l.off[r] = o;
-    o += (sz[r] + 15) & ~size_t(15);
+
+// Part of a staging area: the packed rows lo..hi of arrays, back to back, in one copy over the link.
+struct DropinPiece {
+  struct Part {
+    DropinArray a;
+    uint64_t lo, hi;
+  };
+  std::vector<Part> parts;
+  size_t begin() const { return parts.front().a.off + parts.front().lo * parts.front().a.row; }
+  size_t end() const { return parts.back().a.off + parts.back().hi * parts.back().a.row; }
+  // between the caller's arrays and the staging; every thread takes its share of each part
+  void copy(char* staging, const uint64_t* idx, bool pack, int threads) const {
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int t = 0; t < threads; ++t)
+      for (const Part& p : parts) {
+        const uint64_t n = p.hi - p.lo, lo = p.lo + n * t / threads, hi = p.lo + n * (t + 1) / threads;
+        if (lo >= hi) continue;
+        char* at = staging + p.a.off + lo * p.a.row;
+        switch (p.a.row) {
+          case 2: copy_rows<2>(at, p.a.rows, idx + lo, hi - lo, pack); break;
+          case 4: copy_rows<4>(at, p.a.rows, idx + lo, hi - lo, pack); break;
+          case 12: copy_rows<12>(at, p.a.rows, idx + lo, hi - lo, pack); break;
+          default: copy_rows<36>(at, p.a.rows, idx + lo, hi - lo, pack); break;
+        }
+      }
   }
-  l.off[15] = o;
-  l.bytes = o;
-  return l;
+  // n rows of arrays that lie back to back, cut after every `size` bytes (to the row)
+  static std::vector<DropinPiece> cut(const std::vector<DropinArray>& arrays, uint64_t n, size_t size) {
+    std::vector<DropinPiece> ps(1);
+    size_t have = 0;
+    for (const DropinArray& a : arrays)
+      for (uint64_t lo = 0; lo < n;) {
+        if (have >= size) {
+          ps.emplace_back();
+          have = 0;
+        }
+        const uint64_t hi = std::min<uint64_t>(n, lo + (size - have + a.row - 1) / a.row);
+        ps.back().parts.push_back({a, lo, hi});
+        have += (hi - lo) * a.row;
+        lo = hi;
+      }
+    return ps;
+  }
+};
+
+// Staged drop-in call, for ascending lists: the selected particles travel in pieces, the host packing
+// one while the previous one crosses the link, both ways.  A velocity-only call moves position, velocity
+// and mass only.  Packing costs the host less than the link would take for the unselected particles
+// (490 000 of 1 M particles: whole arrays 2.0 ms, packed 1.0), and the pieces overlap (75 000 of 1 M:
+// 800 -> 320 us).  6, 8 or 12 pieces differ by less than two runs do; smaller ones than 512 KB lose.
+// The line: 4 000 particles of a velocity-only call take 240 us in one copy of every array and 140
+// staged, 2 000 the same either way; a reference call moves all arrays in both forms, 10 000 particles
+// take 191 us in one copy and 210 in pieces, 20 000 the same, 40 000 of 1 M 660 -> 530.
+constexpr size_t kStagedMotion = size_t(64) << 10, kStagedFull = size_t(2) << 20;  // bytes that travel in
+constexpr size_t kPieceLeast = size_t(512) << 10, kPieces = 6;
+
+int dropin_staged(ae_mpm_ctx* ctx, WorldBase* w, const ae_mpm_particles* buffer, const uint64_t* idx, uint64_t n,
+                  bool full, uint32_t substeps) {
+  // the arrays that are written back come first; mass and material only travel in
+  std::vector<DropinArray> in;
+  size_t bytes = 0, out_arrays = 0;
+  const auto add = [&](void* rows, size_t row) {
+    in.push_back({static_cast<char*>(rows), row, bytes});
+    bytes += (row * n + 15) & ~size_t(15);
+  };
+  add(buffer->pos, 12);
+  add(buffer->vel, 12);
+  if (full) {
+    add(buffer->strain, 36);
+    add(buffer->c, 36);
+    add(buffer->jacobian, 4);
+  }
+  out_arrays = in.size();
+  add(buffer->mass, 4);
+  if (full) add(buffer->material_idx, 2);
+  int rc = ensure_dstage(ctx, bytes);
+  if (rc || (rc = ensure_pinned(ctx, bytes))) return rc;
+  char* const dev = static_cast<char*>(ctx->dstage);
+  char* const pin = reinterpret_cast<char*>(ctx->pin);
+  const cudaStream_t st = w->stream();
+  const int threads = std::min(8, omp_get_max_threads());
+  const size_t size = std::max(kPieceLeast, bytes / kPieces + 1);
+  cudaError_t e = cudaSuccess;
+  for (const DropinPiece& p : DropinPiece::cut(in, n, size)) {
+    p.copy(pin, idx, true, threads);
+    e = cudaMemcpyAsync(dev + p.begin(), pin + p.begin(), p.end() - p.begin(), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return fail(ctx, AE_MPM_ECUDA, std::string("drop-in upload: ") + cudaGetErrorString(e));
+  }
+  ae_mpm_particles v{};
+  const auto f32 = [&](size_t a) { return reinterpret_cast<float*>(dev + in[a].off); };
+  v.pos = f32(0);
+  v.vel = f32(1);
+  v.mass = f32(out_arrays);
+  if (full) {
+    v.strain = f32(2);
+    v.c = f32(3);
+    v.jacobian = f32(4);
+    v.material_idx = reinterpret_cast<uint16_t*>(dev + in[6].off);
+  }
+  if (full)
+    rc = w->upload(0, &v, n, false);
+  else
+    rc = w->upload_motion(v.pos, v.vel, v.mass, n);
+  if (rc || (rc = w->step(substeps))) return fail(ctx, rc, w->err);
+  if (full)
+    rc = w->download(0, &v, false);
+  else
+    rc = w->download_motion(v.pos, v.vel);
+  if (rc) return fail(ctx, rc, w->err);
+  in.resize(out_arrays);
+  const std::vector<DropinPiece> back = DropinPiece::cut(in, n, size);
+  for (size_t k = 0; k < back.size() && e == cudaSuccess; ++k) {
+    const DropinPiece& p = back[k];
+    if (!ctx->out_ev[k]) e = cudaEventCreateWithFlags(&ctx->out_ev[k], cudaEventDisableTiming);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(pin + p.begin(), dev + p.begin(), p.end() - p.begin(), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaEventRecord(ctx->out_ev[k], st);
+  }
+  for (size_t k = 0; k < back.size() && e == cudaSuccess; ++k) {
+    e = cudaEventSynchronize(ctx->out_ev[k]);
+    if (e == cudaSuccess) back[k].copy(pin, idx, false, threads);
+  }
+  if (e != cudaSuccess) return fail(ctx, AE_MPM_ECUDA, std::string("drop-in download: ") + cudaGetErrorString(e));
+  return AE_MPM_OK;
 }
 
 int dropin_run(ae_mpm_ctx* ctx, int mode, const ae_mpm_particles* buffer, uint64_t capacity, const ae_mpm_grid* grid,
@@ -308,90 +370,16 @@ int dropin_run(ae_mpm_ctx* ctx, int mode, const ae_mpm_particles* buffer, uint64
   }
   WorldBase* w = ctx->dropin;
   const bool full = mode == AE_MPM_MODE_REFERENCE;
-  if (ascending && 4 * n >= capacity) {
-    // whole arrays in, gather and scatter on the device, whole arrays out: the unselected particles
-    // travel both ways unchanged (the caller holds the buffer exclusively for the call)
-    const DropinLayout l = dropin_layout(capacity, n, full);
-    rc = ensure_dstage(ctx, l.bytes);
-    if (rc) return rc;
-    char* dst = static_cast<char*>(ctx->dstage);
-    ae_mpm_particles dfull{}, dsel{};
-    dfull.pos = reinterpret_cast<float*>(dst + l.off[0]);
-    dfull.vel = reinterpret_cast<float*>(dst + l.off[1]);
-    dfull.mass = reinterpret_cast<float*>(dst + l.off[2]);
-    if (full) {
-      dfull.strain = reinterpret_cast<float*>(dst + l.off[3]);
-      dfull.c = reinterpret_cast<float*>(dst + l.off[4]);
-      dfull.jacobian = reinterpret_cast<float*>(dst + l.off[5]);
-      dfull.material_idx = reinterpret_cast<uint16_t*>(dst + l.off[6]);
-    }
-    uint64_t* didx = reinterpret_cast<uint64_t*>(dst + l.off[7]);
-    dsel.pos = reinterpret_cast<float*>(dst + l.off[8]);
-    dsel.vel = reinterpret_cast<float*>(dst + l.off[9]);
-    dsel.strain = reinterpret_cast<float*>(dst + l.off[10]);
-    dsel.jacobian = reinterpret_cast<float*>(dst + l.off[11]);
-    dsel.c = reinterpret_cast<float*>(dst + l.off[12]);
-    dsel.mass = reinterpret_cast<float*>(dst + l.off[13]);
-    dsel.material_idx = reinterpret_cast<uint16_t*>(dst + l.off[14]);
-    // pinned staging mirrors the device layout of the whole arrays and the index list
-    rc = ensure_pinned(ctx, l.off[8]);
-    if (rc) return rc;
-    char* hp = reinterpret_cast<char*>(ctx->pin);
-    cudaStream_t st = w->stream();
-    cudaError_t e = cudaSuccess;
-    // each array: host copy into pinned staging, then its DMA, which overlaps the next host copy
-    auto in = [&](int r, const void* src, size_t b) {
-      if (e != cudaSuccess) return;
-      host_copy(hp + l.off[r], src, b);
-      e = cudaMemcpyAsync(dst + l.off[r], hp + l.off[r], b, cudaMemcpyHostToDevice, st);
-    };
-    in(0, buffer->pos, 12 * capacity);
-    in(1, buffer->vel, 12 * capacity);
-    in(2, buffer->mass, 4 * capacity);
-    if (full) {
-      in(3, buffer->strain, 36 * capacity);
-      in(4, buffer->c, 36 * capacity);
-      in(5, buffer->jacobian, 4 * capacity);
-      in(6, buffer->material_idx, 2 * capacity);
-    }
-    in(7, idx, 8 * n);
-    const unsigned blocks = unsigned((n + 255) / 256);
-    if (e == cudaSuccess) {
-      dropin_gather_kernel<<<blocks, 256, 0, st>>>(dfull, didx, n, dsel, full ? 1 : 0);
-      e = cudaGetLastError();
-    }
-    if (e != cudaSuccess) return fail(ctx, AE_MPM_ECUDA, std::string("drop-in gather: ") + cudaGetErrorString(e));
-    if ((rc = w->upload(0, &dsel, n, false)) || (rc = w->step(uint32_t(config->substeps))) ||
-        (rc = w->download(0, &dsel, false)))
-      return fail(ctx, rc, w->err);
-    dropin_scatter_kernel<<<blocks, 256, 0, st>>>(dsel, didx, n, dfull, full ? 1 : 0);
-    e = cudaGetLastError();
-    // the written arrays back: DMA into pinned staging, then host copies into the caller's arrays
-    const int outs[5] = {0, 1, 3, 4, 5};
-    const size_t out_b[5] = {12 * capacity, 12 * capacity, 36 * capacity, 36 * capacity, 4 * capacity};
-    void* const out_dst[5] = {buffer->pos, buffer->vel, buffer->strain, buffer->c, buffer->jacobian};
-    const int n_out = full ? 5 : 2;
-    // each array's host copy starts when its own DMA has landed, while the next one transfers
-    for (int k = 0; k < n_out && e == cudaSuccess; ++k) {
-      if (!ctx->out_ev[k]) e = cudaEventCreateWithFlags(&ctx->out_ev[k], cudaEventDisableTiming);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(hp + l.off[outs[k]], dst + l.off[outs[k]], out_b[k], cudaMemcpyDeviceToHost, st);
-      if (e == cudaSuccess) e = cudaEventRecord(ctx->out_ev[k], st);
-    }
-    for (int k = 0; k < n_out && e == cudaSuccess; ++k) {
-      e = cudaEventSynchronize(ctx->out_ev[k]);
-      if (e == cudaSuccess) host_copy(out_dst[k], hp + l.off[outs[k]], out_b[k]);
-    }
-    if (e != cudaSuccess) return fail(ctx, AE_MPM_ECUDA, std::string("drop-in scatter: ") + cudaGetErrorString(e));
-    return AE_MPM_OK;
-  }
+  if (ascending && (full ? n * 106 >= kStagedFull : n * 28 >= kStagedMotion))
+    return dropin_staged(ctx, w, buffer, idx, n, full, uint32_t(config->substeps));
   // gather the selected particles into pinned staging
   rc = ensure_pinned(ctx, sizeof(float) * 26 * n + sizeof(uint16_t) * n + 64);
   if (rc) return rc;
   ae_mpm_particles v = pinned_view(ctx, n);
-  // long lists gather on the OpenMP team (reads only); the scatter back is parallel only for
+  // lists of some length gather on the OpenMP team (reads only; 4 000 particles on one thread made the
+  // call 320 us, 10 000 on eight 190); the scatter back is parallel only for
   // ascending (hence distinct) indices, so a repeated index keeps the reference's last-write-wins
-  const int t_host = n >= 4096 ? std::min(8, omp_get_max_threads()) : 1;
+  const int t_host = n >= 1024 ? std::min(8, omp_get_max_threads()) : 1;
 #pragma omp parallel for num_threads(t_host) schedule(static)
   for (int64_t kk = 0; kk < int64_t(n); ++kk) {
     const uint64_t k = uint64_t(kk);

@@ -2795,8 +2795,8 @@ struct XferSet {
 
 // Caller's layout -> slots, one launch for all scenes of a transfer (a launch per scene, 4.6 us each
 // for 19 000 particles, took 2.4 ms for 512 scenes against 0.4 together).  Bound by memory: 106 bytes
-// read and 112 written per particle run at the copy rate.
-template <class T>
+// read and 112 written per particle run at the copy rate.  kMotion: position, velocity and mass only.
+template <class T, bool kMotion>
 __global__ void __launch_bounds__(256) pack_kernel(WorldDev<T> w, XferSet<T> xs) {
   using V4 = typename V4T<T>::type;
   const int4 ch = cta_chunk(w);
@@ -2807,19 +2807,19 @@ __global__ void __launch_bounds__(256) pack_kernel(WorldDev<T> w, XferSet<T> xs)
   if (i >= d.n) return;
   V4* const* dst = const_cast<V4* const*>(w.in);
   const T *pos = d.f[0], *vel = d.f[1], *F = d.f[2], *C = d.f[4];
-  const T J = d.f[3][i], m = d.f[5][i];
-  const uint32_t mi = d.mat[i];
+  const T J = kMotion ? T(1) : d.f[3][i], m = d.f[5][i];
+  const uint32_t mi = kMotion ? 0u : d.mat[i];
   T f[9], c[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    f[k] = F[9 * i + k];
-    c[k] = C[9 * i + k];
+    f[k] = kMotion ? T(k % 4 == 0 ? 1 : 0) : F[9 * i + k];
+    c[k] = kMotion ? T(0) : C[9 * i + k];
   }
   dst[0][s] = mk4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], m);
   dst[1][s] = mk4(f[0], f[1], f[2], f[3]);
   dst[2][s] = mk4(f[4], f[5], f[6], f[7]);
   dst[3][s] = mk4(f[8], J, Bits<T>::pack(mi), Bits<T>::pack(uint32_t(i)));
-  if (sc.mode == AE_MPM_MODE_PHYSICS) {  // the C slot holds A = m C - k tau on the device
+  if (!kMotion && sc.mode == AE_MPM_MODE_PHYSICS) {  // the C slot holds A = m C - k tau on the device
     const MatDev& md = w.mats[sc.mat_off + (mi < sc.n_mat ? mi : sc.n_mat)];
     T a[9];
     affine_from_c(sc, md, m, c, f, J, a);
@@ -2864,7 +2864,7 @@ __device__ __forceinline__ void store_rows(T* dst, uint64_t i0, uint64_t n, cons
   __syncwarp();
 }
 
-template <class T>
+template <class T, bool kMotion>
 __global__ void __launch_bounds__(256) unpack_kernel(WorldDev<T> w, XferSet<T> xs, const uint32_t* __restrict__ inv) {
   using V4 = typename V4T<T>::type;
   __shared__ T rows[8][32 * 9];
@@ -2880,6 +2880,17 @@ __global__ void __launch_bounds__(256) unpack_kernel(WorldDev<T> w, XferSet<T> x
   if (has) {
     s = inv[sc.p_off + i];
     has = s - sc.p_off < d.n;
+  }
+  if constexpr (kMotion) {
+    T x[3], v[3];
+    if (has) {
+      const V4 a0 = ld4(w.in[0] + s), a4 = ld4(w.in[4] + s);
+      x[0] = a0.x, x[1] = a0.y, x[2] = a0.z;
+      v[0] = a4.x, v[1] = a4.y, v[2] = a4.z;
+    }
+    store_rows<3>(d.f[0], i0, d.n, x, buf, has, lane);
+    store_rows<3>(d.f[1], i0, d.n, v, buf, has, lane);
+    return;
   }
   T f[9], c[9], x[3], v[3], J = T(0), m = T(0);
   uint32_t mi = 0;
@@ -3346,7 +3357,7 @@ class World final : public WorldBase {
     return std::adjacent_find(v.begin(), v.end()) != v.end();
   }
 
-  int launch_pack(uint32_t k, const uint32_t* scenes, const XferDev<T>* x) {
+  int launch_pack(uint32_t k, const uint32_t* scenes, const XferDev<T>* x, bool motion = false) {
     if (k > 1 && has_repeats(k, scenes)) {
       int rc = AE_MPM_OK;
       for (uint32_t i = 0; i < k && rc == AE_MPM_OK; ++i) rc = launch_pack(1, scenes + i, x + i);
@@ -3357,13 +3368,14 @@ class World final : public WorldBase {
     int blocks = 0;
     const int rc = xfer_range(k, scenes, x, w, xs, blocks);
     if (rc || blocks == 0) return rc;
-    pack_kernel<T><<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs);
+    const auto pack = motion ? pack_kernel<T, true> : pack_kernel<T, false>;
+    pack<<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs);
     AE_TRY(cudaGetLastError());
     return AE_MPM_OK;
   }
 
   // the slot index lives in the clamp queue, which is empty between substeps
-  int launch_unpack(uint32_t k, const uint32_t* scenes, const XferDev<T>* x) {
+  int launch_unpack(uint32_t k, const uint32_t* scenes, const XferDev<T>* x, bool motion = false) {
     if (k > 1 && has_repeats(k, scenes)) {
       int rc = AE_MPM_OK;
       for (uint32_t i = 0; i < k && rc == AE_MPM_OK; ++i) rc = launch_unpack(1, scenes + i, x + i);
@@ -3376,7 +3388,8 @@ class World final : public WorldBase {
     if (rc || blocks == 0) return rc;
     uint32_t* inv = reinterpret_cast<uint32_t*>(clamp_queue_);
     unpack_index_kernel<T><<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs, inv);
-    unpack_kernel<T><<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs, inv);
+    const auto unpack = motion ? unpack_kernel<T, true> : unpack_kernel<T, false>;
+    unpack<<<unsigned(blocks), chunk_threads_, 0, stream_>>>(w, xs, inv);
     AE_TRY(cudaGetLastError());
     return AE_MPM_OK;
   }
@@ -3423,15 +3436,53 @@ class World final : public WorldBase {
       const int rc = launch_pack(1, &s, &x);
       if (rc) return rc;
     }
+    uploaded(s, n);
+    return AE_MPM_OK;
+  }
+
+  // the same count keeps the scene table, the chunks and the captured graph (which replays from
+  // the upload's buffers); the cell keys are recomputed before the next substep either way
+  void uploaded(uint32_t s, uint64_t n) {
     scatter_invalid_ = true;
-    // the same count keeps the scene table, the chunks and the captured graph (which replays from
-    // the upload's buffers); the cell keys are recomputed before the next substep either way
     if (h_scenes_[s].p_count != uint32_t(n)) {
       h_scenes_[s].p_count = uint32_t(n);
       count_changed(s);
     }
     keys_stale_ = true;
-    return AE_MPM_OK;
+  }
+
+  int upload_motion(const float* pos, const float* vel, const float* mass, uint64_t n) override {
+    if constexpr (sizeof(T) == 4) {
+      if (mode_ == AE_MPM_MODE_VELOCITY_ONLY && n <= h_scenes_[0].p_cap) {
+        XferDev<T> x{};
+        x.f[0] = const_cast<float*>(pos);
+        x.f[1] = const_cast<float*>(vel);
+        x.f[5] = const_cast<float*>(mass);
+        x.n = uint32_t(n);
+        const uint32_t s = 0;
+        const int rc = n > 0 ? launch_pack(1, &s, &x, true) : AE_MPM_OK;
+        if (rc) return rc;
+        uploaded(0, n);
+        return AE_MPM_OK;
+      }
+    }
+    err = "not a velocity-only FP32 world of that capacity";
+    return AE_MPM_EINVAL;
+  }
+
+  int download_motion(float* pos, float* vel) override {
+    if constexpr (sizeof(T) == 4) {
+      if (mode_ == AE_MPM_MODE_VELOCITY_ONLY) {
+        XferDev<T> x{};
+        x.f[0] = pos;
+        x.f[1] = vel;
+        x.n = h_scenes_[0].p_count;
+        const uint32_t s = 0;
+        return x.n > 0 ? launch_unpack(1, &s, &x, true) : AE_MPM_OK;
+      }
+    }
+    err = "not a velocity-only FP32 world";
+    return AE_MPM_EINVAL;
   }
 
   int download(uint32_t s, void* host, bool f64) override {

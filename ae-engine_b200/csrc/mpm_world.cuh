@@ -106,6 +106,11 @@ struct WorldBase {
   virtual ~WorldBase() {}
   virtual int upload(uint32_t scene, const void* host, uint64_t n, bool f64) = 0;
   virtual int download(uint32_t scene, void* host, bool f64) = 0;
+  // Scene 0 of a velocity-only FP32 world from and to arrays on the world's device: position, velocity
+  // and mass of n particles (F = I, C = 0, J = 1, which the mode neither reads nor changes), and their
+  // positions and velocities back, ordered on stream().
+  virtual int upload_motion(const float* pos, const float* vel, const float* mass, uint64_t n) = 0;
+  virtual int download_motion(float* pos, float* vel) = 0;
   // Many scenes per call (f32 worlds): every host<->device copy is queued back to back through one
   // staging area, so the copies run at link speed instead of one scene, one wait at a time.
   // upload_many is asynchronous like upload; download_many waits once, at the end.
