@@ -679,8 +679,11 @@ int ae_mpm_batch_create(ae_mpm_ctx* ctx, const ae_mpm_scene_desc* scenes, uint32
     b->worlds.push_back(w);
     // earlier groups on higher stream priorities: the GPU serves group g first and fills its
     // kernels' launch gaps and tails with later groups' work, so group g finishes (and its
-    // results start across PCIe) while later groups still compute
-    const int prio = greatest + int(g) < least ? greatest + int(g) : least;
+    // results start across PCIe) while later groups still compute.  The device has six levels: with
+    // more groups the first ones share the highest.  Had the last ones shared the lowest, they would
+    // end together and their results would cross one after the other behind them (8 groups, 96 scenes,
+    // 60 substeps: 19.3 ms against 18.4)
+    const int prio = std::max(greatest, least - int(g_n - 1 - g));
     if ((rc = w->set_stream_priority(prio))) {
       const std::string why2 = w->err;
       delete b;
