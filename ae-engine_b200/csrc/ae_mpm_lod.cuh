@@ -47,10 +47,11 @@ class LodWork {
   cudaError_t grow(uint64_t count, uint64_t cells);
   uint64_t cap_ = 0, cells_cap_ = 0;
   bool select_smem_set_ = false;
+  void* items_ = nullptr;            // one allocation: the arrays per particle and tile
+  void* cells_ = nullptr;            // one allocation: the arrays per cell
   uint32_t* tile_counts_ = nullptr;  // [3][tiles]
   uint32_t* tile_offs_ = nullptr;    // [3][tiles]
   uint32_t* totals_ = nullptr;       // [8]: class totals, housekeeping transitions, totals after the cap
-  uint32_t* host_totals_ = nullptr;  // [4] pinned: where the host reads them
   uint64_t* near_tmp_ = nullptr;     // [cap] near candidates (ascending index)
   uint32_t* near_key_ = nullptr;     // [cap] their squared distance, as bits; later cell keys
   uint8_t* keep_ = nullptr;          // [cap]
