@@ -1,15 +1,16 @@
 // mpm_world.cu -- the MPM substep on sm_100a: kernels and the world driver.
 //
 // Substep (every scene of a world at once):
-//   sort     radix sort of cell keys -> perm (sorted position -> storage slot)
-//   P2G      one block per chunk of sorted particles; the chunk's stencil bounding box is a
-//            shared-memory tile with halo that absorbs all same-cell contributions, then is
-//            flushed with 16-byte vector atomics (red.global.add.v4.f32) into the grid
+//   sort     counts per grid node -> places (radix sort of cell keys where the grid is huge for its
+//            particles) -> perm (sorted position -> storage slot)
 //   grid     one pass over the blocks P2G touched: momentum -> velocity, gravity, walls;
 //            clears the accumulator and the touched flags for the next substep
 //   G2P      one thread per sorted particle: gather, APIC C, F update and material return
 //            mapping, written to the other particle buffer in sorted order (the reorder costs
 //            nothing extra), plus the next substep's cell key
+//   P2G      sums per cell run of a warp, added to the grid with 16-byte vector atomics
+//            (red.global.add.v4.f32).  In physics mode the G2P kernel scatters its particles for
+//            the next substep while they are in registers; P2G alone is the first substep's
 // Deterministic mode replaces P2G's float atomics with per-cell fixed-order sums and a per-node
 // fixed-order gather (no float atomics anywhere), so two runs are bitwise identical.
 #include <cuda_runtime.h>

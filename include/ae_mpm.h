@@ -181,7 +181,7 @@ enum { AE_MPM_P2G_AUTO = 0, AE_MPM_P2G_TILE = 1, AE_MPM_P2G_WARP_AGG = 2, AE_MPM
 typedef struct ae_mpm_exec_opts {
   int32_t precision;      /* 32 or 64                                                        */
   int32_t deterministic;  /* 1: fixed-order segmented sums, no float atomics (bitwise replay) */
-  int32_t sort_interval;  /* radix sort every k substeps (>=1; deterministic mode forces 1)   */
+  int32_t sort_interval;  /* group by cell every k substeps (>=1; deterministic mode: 1)     */
   int32_t p2g_variant;    /* AE_MPM_P2G_*; AUTO takes the autotuned choice                    */
   int32_t block_threads;  /* particles per P2G/G2P block (128 or 256); 0 = autotuned          */
   int32_t use_graph;      /* 1: replay substeps from a captured CUDA graph                    */
@@ -329,7 +329,7 @@ uint64_t ae_mpm_world_scene_particles(const ae_mpm_world* world, uint32_t scene)
 int ae_mpm_radix_sort_keys(ae_mpm_ctx* ctx, const uint32_t* keys, uint64_t n, uint32_t key_bits,
                            uint32_t* sorted_keys_out, uint32_t* perm_out);
 
-/* The grouping sort that non-deterministic worlds with keys of at most 16 bits use (a 32^3 grid):
+/* A grouping sort of keys of at most 16 bits (the cells of a 32^3 grid):
  * one histogram, one scan and one scatter instead of radix passes.  Same buffers as
  * ae_mpm_radix_sort_keys; sorted_keys_out comes out ascending, but equal keys in no defined order,
  * and perm_out is a permutation with keys[perm_out[i]] == sorted_keys_out[i].  Up to 16384 keys the
