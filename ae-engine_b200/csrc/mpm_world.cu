@@ -149,6 +149,20 @@ __device__ __forceinline__ void mark_block(const WorldDev<T>& w, uint32_t gb) {
   }
 }
 
+// Deterministic sums: marks block `corner` (0..7) of the at most two blocks per axis that the stencil
+// based at (g0, g1, g2) spans.  A particle uploaded outside the grid has that base unclamped until its
+// first G2P, so a corner may lie outside too: the clamps below are one-sided, and such a corner is no block.
+template <class T>
+__device__ __forceinline__ void mark_stencil_corner(const WorldDev<T>& w, const SceneDev<T>& sc, int corner, int g0,
+                                                    int g1, int g2) {
+  const int X = (corner & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
+  const int Y = (corner & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
+  const int Z = (corner & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
+  if (X < 0 || Y < 0 || Z < 0 || X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) return;
+  mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * uint32_t(sc.nb[1]) + uint32_t(Y >> 2)) * uint32_t(sc.nb[0]) +
+                    uint32_t(X >> 2));
+}
+
 template <class T>
 __device__ __forceinline__ const MatDev& mat_of(const WorldDev<T>& w, const SceneDev<T>& sc, uint32_t m) {
   return w.mats[sc.mat_off + (m < sc.n_mat ? m : sc.n_mat)];
@@ -2307,13 +2321,7 @@ __global__ void __launch_bounds__(128) det_cellsum_kernel(WorldDev<T> w, uint64_
     }
 #pragma unroll
     for (int o = 0; o < 27; ++o) w.cell_rec[uint64_t(s) * 27 + o] = mk4(acc[o][0], acc[o][1], acc[o][2], acc[o][3]);
-    // the cell's stencil spans at most two blocks per axis
-    for (int t = 0; t < 8; ++t) {
-      int X = (t & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
-      int Y = (t & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
-      int Z = (t & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
-      mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * sc.nb[1] + (Y >> 2)) * sc.nb[0] + (X >> 2));
-    }
+    for (int t = 0; t < 8; ++t) mark_stencil_corner(w, sc, t, g0, g1, g2);
   }
 }
 
@@ -2470,12 +2478,7 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
   };
   auto finish = [&](uint32_t start, int g0, int g1, int g2) {
     if (lane < 27) w.cell_rec[uint64_t(start) * 27 + lane] = mk4(am, ax, ay, az);
-    if (lane < 8) {  // the cell's stencil spans at most two blocks per axis
-      const int X = (lane & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
-      const int Y = (lane & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
-      const int Z = (lane & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
-      mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * sc.nb[1] + (Y >> 2)) * sc.nb[0] + (X >> 2));
-    }
+    if (lane < 8) mark_stencil_corner(w, sc, lane, g0, g1, g2);
   };
   auto inside_grid = [&](const P2GPart<T>& p) {
     return p.g[0] >= 0 && p.g[1] >= 0 && p.g[2] >= 0 && p.g[0] + 2 < sc.n[0] && p.g[1] + 2 < sc.n[1] &&

@@ -147,3 +147,30 @@ def test_deterministic_reference_modes_with_off_grid_particles_repeat(ctx, mode)
     for f in ("pos", "vel", "F", "J", "C"):
         assert np.array_equal(getattr(out[0], f), getattr(out[1], f)), f
     assert rel(out[0].pos, out[2].pos) <= 2e-5
+
+
+@pytest.mark.parametrize("grid", [20, 216])
+def test_deterministic_world_takes_particles_far_outside_its_grid(ctx, grid):
+    # physics mode clamps a position into the grid in its first G2P; until then a stencil may lie wholly
+    # outside: such particles add nothing to the grid, mark no block of it, and come back at its border.
+    # Two scenes of 216^3 nodes with these few particles take the radix-sorted form of the same sums.
+    rng = np.random.default_rng(grid)
+    n, dx = 900, 1.0 / grid
+    x = (8.0 + 4.0 * rng.random((n, 3))) * dx
+    far = np.arange(0, n, 9)
+    x[far, rng.integers(0, 3, far.size)] = np.where(rng.random(far.size) < 0.5, -7.3, grid + 9.4) * dx
+    p = S.make_particles(x, (0.2, -0.1, 0.3), 1e-5, 0)
+    p.J[:] = 1.0
+    sc = M.Scene(n=(grid, grid, grid), dx=dx, dt=1e-4, materials=[S.jelly(E=100.0)], max_particles=n)
+    out = []
+    for det in (1, 1, 0):
+        w = M.World(ctx, [sc, sc], M.exec_opts(deterministic=det))
+        w.upload(0, p)
+        w.upload(1, p)
+        w.step(4)
+        assert w.sync(raise_on_error=False) == M.EDOMAIN
+        out.append((w.download(0, n), w.download(1, n)))
+        w.close()
+    for f in ("pos", "vel", "F", "J", "C"):
+        assert np.array_equal(getattr(out[0][0], f), getattr(out[1][1], f)), f
+    assert rel(out[0][0].pos, out[2][0].pos) <= 1e-6
