@@ -72,7 +72,10 @@ int fail(ae_mpm_ctx* ctx, int code, const std::string& msg) {
   return code;
 }
 
+// Every call starts here: on the context's device, and without an error that an earlier call left
+// behind and reported (an allocation that did not fit, say).  An error that ended the context stays.
 int set_device(ae_mpm_ctx* ctx) {
+  cudaGetLastError();
   cudaError_t e = cudaSetDevice(ctx->device);
   if (e != cudaSuccess) return fail(ctx, AE_MPM_ECUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
   return AE_MPM_OK;

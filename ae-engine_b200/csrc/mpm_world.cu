@@ -3032,6 +3032,7 @@ uint64_t scene_device_bytes(const ae_mpm_scene_desc& d, int precision) {
     cudaError_t e_ = (call);                                                                   \
     if (e_ != cudaSuccess) {                                                                   \
       err = std::string(#call) + ": " + cudaGetErrorString(e_);                                \
+      cudaGetLastError(); /* reported here: the next call's check must not find it again */    \
       return (e_ == cudaErrorMemoryAllocation) ? AE_MPM_ENOMEM : AE_MPM_ECUDA;                 \
     }                                                                                          \
   } while (0)

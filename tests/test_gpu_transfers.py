@@ -117,3 +117,17 @@ def test_many_scene_transfers_mix_device_and_host_views(ctx):
             assert np.array_equal(getattr(got, f), getattr(want, f)), (s, f)
     ref.close()
     w.close()
+
+
+def test_a_reported_cuda_error_does_not_fail_the_next_call(ctx):
+    # a world that no device can hold is refused; what runs after it starts clean
+    sc, p = scene(500, 0x62)
+    huge, _ = scene(1, 0x63)
+    huge.max_particles = (1 << 31) - 1
+    w = M.World(ctx, [sc], M.exec_opts(deterministic=1))
+    with pytest.raises(M.MpmError):
+        M.World(ctx, [huge])
+    w.upload(0, p)
+    w.step(2)
+    assert w.sync(raise_on_error=False) == M.OK
+    w.close()
