@@ -3056,6 +3056,27 @@ HostView<double> host_view<double>(const void* host) {
   return HostView<double>{{h->pos, h->vel, h->strain, h->jacobian, h->c, h->mass}, h->material_idx};
 }
 
+// [lo, hi) of the device allocation that address a lies in, as the driver knows it
+static bool device_allocation(uintptr_t a, uintptr_t& lo, uintptr_t& hi) {
+  typedef int (*RangeFn)(unsigned long long*, size_t*, unsigned long long);
+  static const RangeFn range = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<RangeFn>(fn);
+  }();
+  unsigned long long base = 0;
+  size_t size = 0;
+  if (!range || range(&base, &size, a) != 0) return false;
+  lo = uintptr_t(base);
+  hi = lo + size;
+  return true;
+}
+
 template <class T>
 class World final : public WorldBase {
  public:
@@ -3308,24 +3329,37 @@ class World final : public WorldBase {
     return XferDev<T>{{hv.f[0], hv.f[1], hv.f[2], hv.f[3], hv.f[4], hv.f[5]}, hv.mat, uint32_t(n), 0u};
   }
 
-  // Whether the kernels may use the caller's arrays in place: every one of them ordinary memory of
-  // the world's device, aligned for its type.  Anything else (host, managed or another device's
-  // memory, odd addresses) travels through the staging area.
-  static bool direct_view(const HostView<T>& hv) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    for (int k = 0; k < 7; ++k) {
-      const void* p = k < 6 ? static_cast<const void*>(hv.f[k]) : hv.mat;
-      if (reinterpret_cast<uintptr_t>(p) % (k < 6 ? sizeof(T) : sizeof(uint16_t)) != 0) return false;
-      cudaPointerAttributes a{};
-      if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+  // Which views of one transfer the kernels may use in place.  Every array has to be ordinary memory of
+  // the world's device, aligned for its type, and to end inside its allocation: a copy of too short an
+  // array is refused by the driver, a kernel would run past it.  Anything else (host, managed or another
+  // device's memory, odd addresses, short arrays) travels through the staging area.
+  struct DirectViews {
+    uintptr_t lo = 0, hi = 0;  // the allocation the last array lay in
+
+    bool array(const void* p, size_t bytes, size_t align) {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+      if (a % align != 0) return false;
+      if (a < lo || a >= hi) {
+        int dev = 0;
+        cudaPointerAttributes at{};
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+          cudaGetLastError();
+          return false;
+        }
+        if (at.type != cudaMemoryTypeDevice || at.device != dev || !device_allocation(a, lo, hi)) {
+          lo = hi = 0;
+          return false;
+        }
       }
-      if (a.type != cudaMemoryTypeDevice || a.device != dev) return false;
+      return a >= lo && a < hi && bytes <= hi - a;
     }
-    return true;
-  }
+    bool takes(const HostView<T>& hv, uint64_t n) {
+      const uint64_t len[6] = {3, 3, 9, 1, 9, 1};
+      bool ok = array(hv.mat, sizeof(uint16_t) * n, sizeof(uint16_t));
+      for (int k = 0; k < 6 && ok; ++k) ok = array(hv.f[k], sizeof(T) * len[k] * n, sizeof(T));
+      return ok;
+    }
+  };
 
   // Launch range and description of a transfer of k scenes (x[i] describes scene scenes[i]); false
   // when no particle moves.  A single scene travels as a launch parameter, several as a table.
@@ -3435,7 +3469,7 @@ class World final : public WorldBase {
     }
     if (n > 0) {
       XferDev<T> x = view_xfer(hv, n);
-      if (!direct_view(hv)) {
+      if (!DirectViews().takes(hv, n)) {
         const int rs = ensure_stage(n);
         if (rs) return rs;
         const int rc = stage_in(stage_, hv, n, stream_);
@@ -3511,7 +3545,7 @@ class World final : public WorldBase {
       err = "particle view has a null array";
       return AE_MPM_EINVAL;
     }
-    const bool direct = direct_view(hv);
+    const bool direct = DirectViews().takes(hv, n);
     XferDev<T> x = view_xfer(hv, n);
     if (!direct) {
       const int rs = ensure_stage(n);
@@ -3594,10 +3628,11 @@ class World final : public WorldBase {
     // views in device memory are read in place; the others get a region of the staging area each
     std::vector<XferDev<T>> x(k);
     std::vector<uint8_t> staged(k, 0);
+    DirectViews in_place;
     for (uint32_t i = 0; i < k; ++i) {
       const HostView<T> hv = host_view<T>(&views[i]);
       x[i] = view_xfer(hv, counts[i]);
-      staged[i] = counts[i] > 0 && !direct_view(hv);
+      staged[i] = counts[i] > 0 && !in_place.takes(hv, counts[i]);
       if (staged[i]) total += stage_region(counts[i]);
     }
     if (total > 0) {
@@ -3662,11 +3697,12 @@ class World final : public WorldBase {
     }
     std::vector<XferDev<T>> x(k);
     std::vector<uint64_t> at(k, UINT64_MAX);  // offset of a staged scene's region
+    DirectViews in_place;
     for (uint32_t i = 0; i < k; ++i) {
       const uint64_t n = h_scenes_[scenes[i]].p_count;
       const HostView<T> hv = host_view<T>(&views[i]);
       x[i] = view_xfer(hv, n);
-      if (n == 0 || direct_view(hv)) continue;
+      if (n == 0 || in_place.takes(hv, n)) continue;
       at[i] = total;
       total += stage_region(n);
     }

@@ -131,3 +131,36 @@ def test_a_reported_cuda_error_does_not_fail_the_next_call(ctx):
     w.step(2)
     assert w.sync(raise_on_error=False) == M.OK
     w.close()
+
+
+@pytest.mark.parametrize("short", FIELDS)
+@pytest.mark.parametrize("way", ["up", "down"])
+def test_device_view_with_a_short_array_is_refused(ctx, way, short):
+    # the array's allocation holds half of what the call would read or write: refused, and the context
+    # and the world stay usable
+    import torch
+
+    torch.zeros(1, device="cuda")
+    rt = C.CDLL("libcudart.so.12")
+    sc, p = scene(5000, 0x61)
+    w = M.World(ctx, [sc], M.exec_opts(deterministic=1))
+    w.upload(0, p)
+    before = w.download(0, p.n)
+    ptrs = []
+    for f in FIELDS:
+        q = C.c_void_p()
+        size = getattr(p, f).nbytes // (2 if f == short else 1)
+        assert rt.cudaMalloc(C.byref(q), C.c_size_t(size)) == 0
+        assert rt.cudaMemset(q, 0, C.c_size_t(size)) == 0
+        ptrs.append(q)
+    v = M.ParticlesView(*(q.value for q in ptrs))
+    call = ctx.lib.ae_mpm_world_upload if way == "up" else ctx.lib.ae_mpm_world_download
+    args = (w.h, 0, C.byref(v)) + ((p.n,) if way == "up" else ())
+    assert call(*args) != M.OK
+    w.upload(0, p)
+    after = w.download(0, p.n)
+    for f in FIELDS:
+        assert np.array_equal(getattr(after, f), getattr(before, f)), f
+    for q in ptrs:
+        assert rt.cudaFree(q) == 0
+    w.close()
