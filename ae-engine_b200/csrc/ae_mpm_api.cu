@@ -760,9 +760,12 @@ int ae_mpm_batch_run(ae_mpm_batch* batch, const ae_mpm_particles* in, const uint
     mark(w->stream());
     host_mark();
   }
+  // the groups' streams are not ordered among one another: views that share memory are copied on the
+  // download stream, in scene order
+  const bool in_place = !aemp::views_overlap(out, counts, batch->first.back());
   for (uint32_t g = 0; g < g_n; ++g) {
     const uint32_t f = batch->first[g], k = batch->first[g + 1] - f;
-    if ((rc = batch->worlds[g]->download_many(k, ids.data(), out + f, batch->down))) return group_fail(g, rc);
+    if ((rc = batch->worlds[g]->download_many(k, ids.data(), out + f, batch->down, in_place))) return group_fail(g, rc);
     mark(batch->down);
     host_mark();
   }

@@ -3056,6 +3056,34 @@ HostView<double> host_view<double>(const void* host) {
   return HostView<double>{{h->pos, h->vel, h->strain, h->jacobian, h->c, h->mass}, h->material_idx};
 }
 
+// Whether two arrays of k views share memory.  Results copied out of a staging area one after another
+// leave the later one there; kernels that write both in place would leave a mixture.
+template <class T>
+static bool arrays_overlap(const HostView<T>* views, const uint64_t* counts, uint32_t k) {
+  std::vector<std::pair<uintptr_t, uintptr_t>> used;
+  used.reserve(7 * size_t(k));
+  const uint64_t len[6] = {3, 3, 9, 1, 9, 1};
+  for (uint32_t i = 0; i < k; ++i) {
+    if (counts[i] == 0) continue;
+    for (int q = 0; q < 6; ++q) {
+      const uintptr_t a = reinterpret_cast<uintptr_t>(views[i].f[q]);
+      used.emplace_back(a, a + sizeof(T) * len[q] * counts[i]);
+    }
+    const uintptr_t a = reinterpret_cast<uintptr_t>(views[i].mat);
+    used.emplace_back(a, a + sizeof(uint16_t) * counts[i]);
+  }
+  std::sort(used.begin(), used.end());
+  for (size_t q = 1; q < used.size(); ++q)
+    if (used[q].first < used[q - 1].second) return true;
+  return false;
+}
+
+bool views_overlap(const ae_mpm_particles* views, const uint64_t* counts, uint32_t k) {
+  std::vector<HostView<float>> v(k);
+  for (uint32_t i = 0; i < k; ++i) v[i] = host_view<float>(&views[i]);
+  return arrays_overlap(v.data(), counts, k);
+}
+
 // [lo, hi) of the device allocation that address a lies in, as the driver knows it
 static bool device_allocation(uintptr_t a, uintptr_t& lo, uintptr_t& hi) {
   typedef int (*RangeFn)(unsigned long long*, size_t*, unsigned long long);
@@ -3545,7 +3573,7 @@ class World final : public WorldBase {
       err = "particle view has a null array";
       return AE_MPM_EINVAL;
     }
-    const bool direct = DirectViews().takes(hv, n);
+    const bool direct = DirectViews().takes(hv, n) && !arrays_overlap(&hv, &n, 1);
     XferDev<T> x = view_xfer(hv, n);
     if (!direct) {
       const int rs = ensure_stage(n);
@@ -3672,7 +3700,8 @@ class World final : public WorldBase {
     return AE_MPM_OK;
   }
 
-  int download_many(uint32_t k, const uint32_t* scenes, ae_mpm_particles* views, cudaStream_t copy) override {
+  int download_many(uint32_t k, const uint32_t* scenes, ae_mpm_particles* views, cudaStream_t copy,
+                    bool in_place) override {
     if (sizeof(T) != 4) {
       err = "many-scene transfers are for f32 worlds";
       return AE_MPM_EINVAL;
@@ -3696,15 +3725,16 @@ class World final : public WorldBase {
       }
     }
     std::vector<XferDev<T>> x(k);
-    std::vector<uint64_t> at(k, UINT64_MAX);  // offset of a staged scene's region
-    DirectViews in_place;
+    std::vector<uint64_t> counts(k), at(k, UINT64_MAX);  // at: offset of a staged scene's region
+    DirectViews direct;
+    for (uint32_t i = 0; i < k; ++i) counts[i] = h_scenes_[scenes[i]].p_count;
+    in_place = in_place && !views_overlap(views, counts.data(), k);
     for (uint32_t i = 0; i < k; ++i) {
-      const uint64_t n = h_scenes_[scenes[i]].p_count;
       const HostView<T> hv = host_view<T>(&views[i]);
-      x[i] = view_xfer(hv, n);
-      if (n == 0 || in_place.takes(hv, n)) continue;
+      x[i] = view_xfer(hv, counts[i]);
+      if (counts[i] == 0 || (in_place && direct.takes(hv, counts[i]))) continue;
       at[i] = total;
-      total += stage_region(n);
+      total += stage_region(counts[i]);
     }
     if (total > 0) {
       const int rs = ensure_stage_bytes(total);

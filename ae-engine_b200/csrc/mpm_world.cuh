@@ -117,10 +117,12 @@ struct WorldBase {
   // With a copy stream, the host<->device copies go on that stream instead (ordered against the
   // world's own stream by events), so that they overlap another world's substeps; download_many
   // then returns without waiting and the results are in place once `copy` has drained.
+  // in_place = false: no view is written by the world's own kernels (its arrays may be another world's
+  // too), every result is copied in the order of the calls.
   virtual int upload_many(uint32_t n, const uint32_t* scenes, const ae_mpm_particles* views, const uint64_t* counts,
                           cudaStream_t copy = nullptr) = 0;
   virtual int download_many(uint32_t n, const uint32_t* scenes, ae_mpm_particles* views,
-                            cudaStream_t copy = nullptr) = 0;
+                            cudaStream_t copy = nullptr, bool in_place = true) = 0;
   virtual int step(uint32_t n) = 0;
   virtual int sync() = 0;
   virtual int totals(uint32_t scene, double out[5]) = 0;
@@ -157,6 +159,9 @@ struct WorldBase {
 // Creates a world on the current device; returns nullptr and fills `why` on failure.
 WorldBase* make_world(const ae_mpm_scene_desc* scenes, uint32_t n_scenes, const ae_mpm_exec_opts& opts,
                       std::string& why, int* status, DevAlloc* alloc = nullptr);
+
+// Whether two arrays of the k views (counts[i] particles each) share memory.
+bool views_overlap(const ae_mpm_particles* views, const uint64_t* counts, uint32_t k);
 
 // Estimated device bytes for one scene (used by the server's HBM admission).
 uint64_t scene_device_bytes(const ae_mpm_scene_desc& d, int precision);

@@ -164,3 +164,56 @@ def test_device_view_with_a_short_array_is_refused(ctx, way, short):
     for q in ptrs:
         assert rt.cudaFree(q) == 0
     w.close()
+
+
+def test_download_into_shared_device_arrays_keeps_the_copy_order(ctx):
+    # a caller that wants neither J nor C points both at one buffer, or every scene at one view: the
+    # array and the scene that come last are left there whole
+    import torch
+
+    pairs = [scene(n, 0x90 + n) for n in (5000, 4097)]
+    w = M.World(ctx, [sc for sc, _ in pairs], M.exec_opts(deterministic=1))
+    for i, (_, p) in enumerate(pairs):
+        w.upload(i, p)
+    w.step(3)
+    want = [w.download(i, p.n) for i, (_, p) in enumerate(pairs)]
+    n = pairs[0][1].n
+    keep, v = device_view(pairs[0][1], 0)
+    v.jacobian = v.c  # C is copied after J
+    extra = torch.zeros(10 * n, dtype=torch.float32, device="cuda")
+    v.strain = extra.data_ptr()
+    v.mass = extra.data_ptr() + 4 * (9 * n - 12)  # the mass is copied after F: over its last 12 values
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.ae_mpm_world_download(w.h, 0, C.byref(v)))
+    got = host_of(keep, 0, pairs[0][1])
+    assert np.array_equal(got.C, want[0].C) and np.array_equal(got.pos, want[0].pos)
+    f = extra.cpu().numpy()
+    assert np.array_equal(f[9 * n - 12:10 * n - 12], want[0].mass)
+    assert np.array_equal(f[:9 * n - 12], want[0].F.ravel()[:9 * n - 12])
+    keep, v = device_view(pairs[0][1], 0)
+    views = (M.ParticlesView * 2)(v, v)
+    ids = np.array([0, 1], np.uint32)
+    ctx.check(ctx.lib.ae_mpm_world_download_many(w.h, 2, ids.ctypes.data, C.addressof(views)))
+    got, m = host_of(keep, 0, pairs[0][1]), pairs[1][1].n
+    for f in FIELDS:
+        assert np.array_equal(getattr(got, f)[:m], getattr(want[1], f)), f
+        assert np.array_equal(getattr(got, f)[m:], getattr(want[0], f)[m:]), f
+    w.close()
+
+
+def test_batch_groups_into_one_device_view_keep_the_scene_order(ctx):
+    pairs = [scene(n, 0xA0 + n) for n in (3000, 2900, 2800, 2700)]
+    parts = [p for _, p in pairs]
+    want = [p.copy() for p in parts]
+    b = M.Batch(ctx, [sc for sc, _ in pairs], M.exec_opts(deterministic=1), groups=4)
+    b.run(parts, 3, out=want)
+    keep, v = device_view(parts[0], 0)
+    ins, outs = (M.ParticlesView * 4)(*[p.view() for p in parts]), (M.ParticlesView * 4)(v, v, v, v)
+    counts = np.array([p.n for p in parts], np.uint64)
+    ctx.check(ctx.lib.ae_mpm_batch_run(b.h, C.addressof(ins), counts.ctypes.data, C.addressof(outs), 3))
+    got = host_of(keep, 0, parts[0])
+    for s in (0, 1, 2, 3):  # scene s shows where the later, shorter ones end
+        lo, hi = (parts[s + 1].n if s < 3 else 0), parts[s].n
+        for f in FIELDS:
+            assert np.array_equal(getattr(got, f)[lo:hi], getattr(want[s], f)[lo:hi]), (s, f)
+    b.close()
