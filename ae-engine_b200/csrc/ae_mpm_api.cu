@@ -373,8 +373,14 @@ int dropin_run(ae_mpm_ctx* ctx, int mode, const ae_mpm_particles* buffer, uint64
   }
   WorldBase* w = ctx->dropin;
   const bool full = mode == AE_MPM_MODE_REFERENCE;
+  // copies queued before a failing step may still read or write the staging areas, which the next call
+  // packs into: a failed call returns once they are done
+  const auto settled = [w](int code) {
+    if (code) cudaStreamSynchronize(w->stream());
+    return code;
+  };
   if (ascending && (full ? n * 106 >= kStagedFull : n * 28 >= kStagedMotion))
-    return dropin_staged(ctx, w, buffer, idx, n, full, uint32_t(config->substeps));
+    return settled(dropin_staged(ctx, w, buffer, idx, n, full, uint32_t(config->substeps)));
   // gather the selected particles into pinned staging
   rc = ensure_pinned(ctx, sizeof(float) * 26 * n + sizeof(uint16_t) * n + 64);
   if (rc) return rc;
@@ -404,7 +410,7 @@ int dropin_run(ae_mpm_ctx* ctx, int mode, const ae_mpm_particles* buffer, uint64
     v.material_idx[k] = buffer->material_idx ? buffer->material_idx[i] : 0;
   }
   if ((rc = w->upload(0, &v, n, false)) || (rc = w->step(uint32_t(config->substeps))) || (rc = w->download(0, &v, false)))
-    return fail(ctx, rc, w->err);
+    return settled(fail(ctx, rc, w->err));
 #pragma omp parallel for num_threads(ascending ? t_host : 1) schedule(static)
   for (int64_t kk = 0; kk < int64_t(n); ++kk) {
     const uint64_t k = uint64_t(kk);
