@@ -251,7 +251,7 @@ struct ae_mpm_server {
         Slot s;
         s.cls = c;
         std::vector<ae_mpm_material> tmp;
-        s.bytes = aemp::scene_device_bytes(slot_desc(s, tmp), 32);
+        s.bytes = aemp::scene_device_bytes(slot_desc(s, tmp), opts.exec);
         want.emplace_back(s, 0);
         i = int(want.size()) - 1;
       }
@@ -639,7 +639,8 @@ int ae_mpm_server_submit(ae_mpm_server* s, const ae_mpm_scene_desc* scene, const
     ae_mpm_scene_desc cd = r->desc;
     for (int a = 0; a < 3; ++a) cd.n[a] = c.n[a];
     cd.max_particles = c.particles;
-    if (aemp::scene_device_bytes(cd, 32) > s->opts.hbm_budget_bytes) {
+    cd.n_materials = c.materials;
+    if (aemp::scene_device_bytes(cd, s->opts.exec) > s->opts.hbm_budget_bytes) {
       delete r;
       return AE_MPM_EBUDGET;
     }

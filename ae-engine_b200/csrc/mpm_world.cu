@@ -3020,13 +3020,6 @@ static uint64_t blocks_of(const ae_mpm_scene_desc& d) {
   return uint64_t((d.n[0] + 3) / 4) * ((d.n[1] + 3) / 4) * ((d.n[2] + 3) / 4) + 1;  // + spare block
 }
 
-uint64_t scene_device_bytes(const ae_mpm_scene_desc& d, int precision) {
-  uint64_t es = precision == 64 ? 8 : 4;
-  uint64_t parts = d.max_particles * (2 * 7 * 4 * es + 5 * 4 + 26 * es + 2);
-  uint64_t grid = blocks_of(d) * 64 * (2 * 4 * es) + blocks_of(d) * 16;
-  return parts + grid;
-}
-
 #define AE_TRY(call)                                                                           \
   do {                                                                                         \
     cudaError_t e_ = (call);                                                                   \
@@ -3206,64 +3199,19 @@ class World final : public WorldBase {
     // One allocation carries every array of the world, the ones that start at zero side by side (one
     // clear): thirty allocations and a dozen clears took most of a world's creation.
     const uint64_t pc = std::max<uint64_t>(cap, 1), nodes = blk * 64;
-    enum { kZero, kOnes, kNone };
-    struct Region {
-      void** p;
-      size_t bytes;
-      int fill;
-    };
-    std::vector<Region> regions;
-    auto reserve = [&regions](auto** p, size_t bytes, int fill) {
-      regions.push_back({reinterpret_cast<void**>(p), bytes, fill});
-    };
-    reserve(&d_scenes_, sizeof(SceneDev<T>) * n, kNone);
-    reserve(&d_mats_, sizeof(MatDev) * h_mats_.size(), kNone);
-    reserve(&blk_scene_, sizeof(uint32_t) * blk, kNone);
-    reserve(&dead_blk_, sizeof(uint32_t) * blk, kNone);
-    // particle slots past a scene's count are never read (every kernel gates on the live range),
-    // so the particle arrays need no clearing
-    for (int k = 0; k < 7; ++k) {
-      reserve(&bufA_[k], sizeof(V4) * pc, kNone);
-      reserve(&bufB_[k], sizeof(V4) * pc, kNone);
-    }
-    reserve(&keys_, sizeof(uint32_t) * pc, kNone);
-    reserve(&clamp_queue_, sizeof(uint2) * pc, kNone);
     // Dense grouping reads every node's counter; the radix sort moves 20 bytes per key and pass.
     // The grid decides: up to 16 nodes per particle slot (or 8 M nodes, 5 us of scan) the dense
     // grouping wins, a huge grid with few particles in it keeps the radix sort.
     dense_sort_ = nodes <= 16 * cap + (uint64_t(8) << 20);
-    if (dense_sort_) {
-      n_segs_ = uint32_t((nodes + kBinSeg - 1) / kBinSeg);
-      reserve(&bins_, sizeof(uint32_t) * nodes, kZero);
-      reserve(&bin_off_, sizeof(uint32_t) * nodes, kNone);
-      reserve(&seg_, sizeof(uint32_t) * 2 * n_segs_, kNone);
-      reserve(&bin_perm_, sizeof(uint32_t) * pc, kZero);
-      if (opts_.deterministic) {
-        reserve(&cells_, sizeof(uint2) * nodes, kZero);
-        reserve(&ordered_, sizeof(uint32_t) * pc, kZero);
-      }
-    } else if (opts_.deterministic) {
-      reserve(&cell_slot_, sizeof(uint32_t) * nodes, kOnes);
-      reserve(&seg_start_, sizeof(uint32_t) * pc, kNone);
-    }
-    if (opts_.deterministic) reserve(&cell_rec_, sizeof(V4) * 27 * pc, kNone);
-    reserve(&acc_, sizeof(V4) * nodes, kZero);
-    reserve(&vel_, sizeof(V4) * nodes, kZero);
-    reserve(&blk_flag_, sizeof(uint32_t) * blk, kZero);
-    reserve(&blk_epoch_, sizeof(uint32_t) * blk, kOnes);
-    // two touched-block lists: the fused G2P + P2G fills the next substep's while the grid update
-    // consumes the current one's
-    reserve(&touched_, sizeof(uint32_t) * 2 * blk, kNone);
-    reserve(&counters_, sizeof(uint32_t) * 8, kZero);
-    reserve(&err_, sizeof(uint32_t) * 4 * n, kZero);
-    reserve(&d_xfer_, sizeof(XferDev<T>) * n, kNone);
+    if (dense_sort_) n_segs_ = uint32_t((nodes + kBinSeg - 1) / kBinSeg);
     n_chunks_alloc_ = 0;
     for (const ae_mpm_scene_desc& d : descs_) n_chunks_alloc_ += int((d.max_particles + 127) / 128);  // smallest chunks
-    reserve(&d_chunks_, sizeof(int4) * std::max(n_chunks_alloc_, 1), kNone);
+    std::vector<Region> regions =
+        plan(this, {n, h_mats_.size(), blk, pc, uint64_t(n_chunks_alloc_), dense_sort_, opts_.deterministic != 0});
     std::stable_sort(regions.begin(), regions.end(), [](const Region& x, const Region& y) { return x.fill < y.fill; });
     size_t total = 0, end[2] = {0, 0};
     for (const Region& r : regions) {
-      total += (r.bytes + 255) & ~size_t(255);
+      total += r.rounded();
       if (r.fill != kNone) end[r.fill] = total;
     }
     if (end[kOnes] == 0) end[kOnes] = end[kZero];
@@ -3271,7 +3219,7 @@ class World final : public WorldBase {
     size_t off = 0;
     for (const Region& r : regions) {
       *r.p = arena_ + off;
-      off += (r.bytes + 255) & ~size_t(255);
+      off += r.rounded();
     }
     AE_TRY(cudaMemsetAsync(arena_, 0, end[kZero], stream_));
     AE_TRY(cudaMemsetAsync(arena_ + end[kZero], 0xff, end[kOnes] - end[kZero], stream_));
@@ -3281,6 +3229,78 @@ class World final : public WorldBase {
     if (!dense_sort_) AE_TRY(sort_scratch_alloc(sort_, pc, alloc_ ? &World::sort_alloc : nullptr, alloc_));
     AE_TRY(cudaStreamSynchronize(stream_));
     return AE_MPM_OK;
+  }
+
+  // The arrays of a world: where each goes (null without a world), its bytes and what it starts with.
+  enum { kZero, kOnes, kNone };
+  struct Region {
+    void** p;
+    size_t bytes;
+    int fill;
+    size_t rounded() const { return (bytes + 255) & ~size_t(255); }
+  };
+  struct Extent {
+    uint64_t scenes, mats, blk, pc, chunks;
+    bool dense, deterministic;
+  };
+  static std::vector<Region> plan(World* w, const Extent& x) {
+    std::vector<Region> regions;
+    const uint64_t nodes = x.blk * 64, segs = (nodes + kBinSeg - 1) / kBinSeg;
+    auto reserve = [&](auto World::*m, size_t bytes, int fill) {
+      regions.push_back({w ? reinterpret_cast<void**>(&(w->*m)) : nullptr, bytes, fill});
+    };
+    reserve(&World::d_scenes_, sizeof(SceneDev<T>) * x.scenes, kNone);
+    reserve(&World::d_mats_, sizeof(MatDev) * x.mats, kNone);
+    reserve(&World::blk_scene_, sizeof(uint32_t) * x.blk, kNone);
+    reserve(&World::dead_blk_, sizeof(uint32_t) * x.blk, kNone);
+    // particle slots past a scene's count are never read (every kernel gates on the live range),
+    // so the particle arrays need no clearing
+    for (int k = 0; k < 7; ++k) {
+      regions.push_back({w ? reinterpret_cast<void**>(&w->bufA_[k]) : nullptr, sizeof(V4) * x.pc, kNone});
+      regions.push_back({w ? reinterpret_cast<void**>(&w->bufB_[k]) : nullptr, sizeof(V4) * x.pc, kNone});
+    }
+    reserve(&World::keys_, sizeof(uint32_t) * x.pc, kNone);
+    reserve(&World::clamp_queue_, sizeof(uint2) * x.pc, kNone);
+    if (x.dense) {
+      reserve(&World::bins_, sizeof(uint32_t) * nodes, kZero);
+      reserve(&World::bin_off_, sizeof(uint32_t) * nodes, kNone);
+      reserve(&World::seg_, sizeof(uint32_t) * 2 * segs, kNone);
+      reserve(&World::bin_perm_, sizeof(uint32_t) * x.pc, kZero);
+      if (x.deterministic) {
+        reserve(&World::cells_, sizeof(uint2) * nodes, kZero);
+        reserve(&World::ordered_, sizeof(uint32_t) * x.pc, kZero);
+      }
+    } else if (x.deterministic) {
+      reserve(&World::cell_slot_, sizeof(uint32_t) * nodes, kOnes);
+      reserve(&World::seg_start_, sizeof(uint32_t) * x.pc, kNone);
+    }
+    if (x.deterministic) reserve(&World::cell_rec_, sizeof(V4) * 27 * x.pc, kNone);
+    reserve(&World::acc_, sizeof(V4) * nodes, kZero);
+    reserve(&World::vel_, sizeof(V4) * nodes, kZero);
+    reserve(&World::blk_flag_, sizeof(uint32_t) * x.blk, kZero);
+    reserve(&World::blk_epoch_, sizeof(uint32_t) * x.blk, kOnes);
+    // two touched-block lists: the fused G2P + P2G fills the next substep's while the grid update
+    // consumes the current one's
+    reserve(&World::touched_, sizeof(uint32_t) * 2 * x.blk, kNone);
+    reserve(&World::counters_, sizeof(uint32_t) * 8, kZero);
+    reserve(&World::err_, sizeof(uint32_t) * 4 * x.scenes, kZero);
+    reserve(&World::d_xfer_, sizeof(XferDev<T>) * x.scenes, kNone);
+    reserve(&World::d_chunks_, sizeof(int4) * std::max<uint64_t>(x.chunks, 1), kNone);
+    return regions;
+  }
+
+  // Device bytes that a scene adds to a world at most: its share of the world's arrays, of the radix
+  // sort's scratch where the world may sort so (its other scenes decide), and of the transfer staging.
+  static uint64_t device_bytes_of(const ae_mpm_scene_desc& d, bool deterministic) {
+    const uint64_t pc = std::max<uint64_t>(d.max_particles, 1), chunks = (d.max_particles + 127) / 128;
+    uint64_t most = 0;
+    for (const bool dense : {false, true}) {
+      uint64_t sum = dense ? 0 : sort_scratch_bytes(pc);
+      for (const Region& r : plan(nullptr, {1, uint64_t(d.n_materials) + 1, blocks_of(d), pc, chunks, dense, deterministic}))
+        sum += r.rounded();
+      most = std::max(most, sum);
+    }
+    return most + pc * (26 * sizeof(T) + sizeof(uint16_t)) + 64;
   }
 
   void fill_scene_params(SceneDev<T>& h, const ae_mpm_scene_desc& d) {
@@ -4677,6 +4697,11 @@ class World final : public WorldBase {
   bool sorted_ = false;      // perm_ orders the current particle state
   uint32_t phase_ = 0;       // substeps since the last sort was due
 };
+
+uint64_t scene_device_bytes(const ae_mpm_scene_desc& d, const ae_mpm_exec_opts& opts) {
+  return opts.precision == 64 ? World<double>::device_bytes_of(d, opts.deterministic != 0)
+                              : World<float>::device_bytes_of(d, opts.deterministic != 0);
+}
 
 WorldBase* make_world(const ae_mpm_scene_desc* scenes, uint32_t n_scenes, const ae_mpm_exec_opts& opts, std::string& why,
                       int* status, DevAlloc* alloc) {

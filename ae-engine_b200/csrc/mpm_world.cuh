@@ -163,8 +163,9 @@ WorldBase* make_world(const ae_mpm_scene_desc* scenes, uint32_t n_scenes, const 
 // Whether two arrays of the k views (counts[i] particles each) share memory.
 bool views_overlap(const ae_mpm_particles* views, const uint64_t* counts, uint32_t k);
 
-// Estimated device bytes for one scene (used by the server's HBM admission).
-uint64_t scene_device_bytes(const ae_mpm_scene_desc& d, int precision);
+// Device bytes that one scene adds to a world at most (used by the server's HBM admission): a world
+// never holds more than the sum over its scenes.
+uint64_t scene_device_bytes(const ae_mpm_scene_desc& d, const ae_mpm_exec_opts& opts);
 
 // Device SM count (cached per device).
 int device_sm_count();

@@ -358,6 +358,15 @@ cudaError_t sort_scratch_alloc(SortScratch& s, uint64_t n, SortAllocFn alloc, vo
   return cudaSuccess;
 }
 
+uint64_t sort_scratch_bytes(uint64_t n) {
+  const uint64_t m = n > 0 ? n : 1, tiles = sort_tiles(m);
+  const uint64_t words[4] = {kMaxRadix * tiles, kMaxRadix * tiles, 4 * kMaxRadix,
+                             n > uint64_t(kSmallSortMax) ? uint64_t(1) << kCountingSortBits : 0};
+  uint64_t sum = 0;
+  for (uint64_t v : words) sum += (sizeof(uint32_t) * v + 255) & ~uint64_t(255);
+  return sum + 3 * ((sizeof(uint32_t) * m + 255) & ~uint64_t(255));
+}
+
 void sort_scratch_free(SortScratch& s, SortFreeFn release, void* user) {
   uint32_t* ps[7] = {s.hist, s.offsets, s.totals, s.keys_alt, s.vals_a, s.vals_b, s.bins};
   for (uint32_t* p : ps)

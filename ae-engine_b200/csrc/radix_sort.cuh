@@ -67,6 +67,7 @@ inline uint64_t sort_tiles(uint64_t n) { return (n + kSortTile - 1) / kSortTile;
 // `alloc(p, bytes)` / `release(p)` default to cudaMalloc / cudaFree.
 typedef cudaError_t (*SortAllocFn)(void* user, void** p, size_t bytes);
 typedef void (*SortFreeFn)(void* user, void* p);
+uint64_t sort_scratch_bytes(uint64_t n);  // of such a scratch, each array rounded to 256
 cudaError_t sort_scratch_alloc(SortScratch& s, uint64_t n, SortAllocFn alloc = nullptr, void* user = nullptr);
 void sort_scratch_free(SortScratch& s, SortFreeFn release = nullptr, void* user = nullptr);
 

@@ -324,6 +324,33 @@ def test_server_budget_and_cancel(ctx):
     srv.close()
 
 
+@pytest.mark.parametrize("deterministic", [0, 1])
+@pytest.mark.parametrize("grid,n", [(96, 1500), (24, 60000)])
+def test_server_counts_at_least_the_device_memory_it_takes(ctx, grid, n, deterministic):
+    # sparse and dense scenes: what the device lost to the server's world is within the bytes that the
+    # budget was charged with (the driver hands memory out in pieces of 2 MB)
+    import torch
+
+    sc, p = S.tiny_scene(n, grid, S.jelly(), seed=5)
+    sc.dt = 1e-5
+    lost = []
+    for measured in (False, True):  # the first server loads the kernels
+        torch.cuda.synchronize()
+        free0 = torch.cuda.mem_get_info()[0]
+        srv = M.Server(ctx, hbm_budget_bytes=8 << 30, substeps_per_tick=4,
+                       exec_options=M.exec_opts(deterministic=deterministic))
+        ids = [srv.submit(sc, p, 400) for _ in range(6)]
+        for _ in range(20000):
+            if srv.stats()["ticks"] >= 8:
+                break
+            time.sleep(0.001)
+        lost.append((free0 - torch.cuda.mem_get_info()[0], srv.stats()["resident_bytes"]))
+        assert srv.drain(120.0) == M.OK and len(ids) == 6
+        srv.close()
+    took, charged = lost[1]
+    assert 0 < took <= charged + (4 << 20)
+
+
 # ------------------------------------------------------------------ the benchmark configurations
 def test_config1_fp32_vs_fp64_after_200_substeps(ctx):
     # target: <= 1e-4 relative position error against the FP64 kernels after 200 substeps
