@@ -151,16 +151,15 @@ __device__ __forceinline__ void mark_block(const WorldDev<T>& w, uint32_t gb) {
 
 // Deterministic sums: marks block `corner` (0..7) of the at most two blocks per axis that the stencil
 // based at (g0, g1, g2) spans.  A particle uploaded outside the grid has that base unclamped until its
-// first G2P, so a corner may lie outside too: the clamps below are one-sided, and such a corner is no block.
+// first G2P, wherever it lies: both ends are clamped into the grid (a block marked without need is an
+// update of unchanged nodes).
 template <class T>
 __device__ __forceinline__ void mark_stencil_corner(const WorldDev<T>& w, const SceneDev<T>& sc, int corner, int g0,
                                                     int g1, int g2) {
-  const int X = (corner & 1) ? min(g0 + 2, sc.n[0] - 1) : max(g0, 0);
-  const int Y = (corner & 2) ? min(g1 + 2, sc.n[1] - 1) : max(g1, 0);
-  const int Z = (corner & 4) ? min(g2 + 2, sc.n[2] - 1) : max(g2, 0);
-  if (X < 0 || Y < 0 || Z < 0 || X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) return;
-  mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * uint32_t(sc.nb[1]) + uint32_t(Y >> 2)) * uint32_t(sc.nb[0]) +
-                    uint32_t(X >> 2));
+  const int X = min(max(g0 + 2 * (corner & 1), 0), sc.n[0] - 1);
+  const int Y = min(max(g1 + (corner & 2), 0), sc.n[1] - 1);
+  const int Z = min(max(g2 + ((corner & 4) >> 1), 0), sc.n[2] - 1);
+  mark_block(w, sc.blk_off + (uint32_t(Z >> 2) * sc.nb[1] + (Y >> 2)) * sc.nb[0] + (X >> 2));
 }
 
 template <class T>
