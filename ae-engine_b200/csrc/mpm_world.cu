@@ -1673,7 +1673,7 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
   }
   if (kTile) __syncthreads();
   uint32_t err = 0;
-  bool cl = false, need = false;
+  bool cl = false, need = false, off = false;
   const uint32_t live_mask = __ballot_sync(0xffffffffu, live);
   if (live) {
     const T x0[3] = {a0.x, a0.y, a0.z};
@@ -1729,12 +1729,17 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
         const uint32_t peers = __match_any_sync(live_mask, key);
         if (lane == __ffs(peers) - 1) atomicAdd(w.bins + key, uint32_t(__popc(peers)));
       }
+      off = key == sc.dead_key;
     }
     err = o.err;
     cl = o.clamped;
     need = o.needs_clamp;
   } else if (j < ch.w && write_keys && !w.bins) {
     w.keys[j] = sc.dead_key;
+  }
+  if (kTile && write_keys && w.dead_cnt) {
+    const int c = __syncthreads_count(off);
+    if (tid == 0) w.dead_cnt[blockIdx.x] = uint32_t(c);
   }
   // warp-aggregated error words, counters and clamp-queue appends
   const uint32_t e = __reduce_or_sync(0xffffffffu, err);
@@ -2270,6 +2275,15 @@ __global__ void discard_scatter_kernel(typename V4T<T>::type* acc, uint32_t* blk
   }
 }
 
+__device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  return x;
+}
+
 // dense grouping (bin_scan_kernel): nodes per scan CTA
 constexpr int kBinSeg = 4096;
 constexpr int kBinThreads = 256;
@@ -2379,9 +2393,73 @@ __global__ void __launch_bounds__(256) det_gather_kernel(WorldDev<T> w, uint32_t
 // (det_cellsum_kernel) left the chip to a few spilling warps: 211 us for 1 M particles at 8 per cell.
 //
 // Slot order: up to 32 particles rank each other by shuffles, up to kCellRankMax by comparing with
-// the whole cell; a larger cell (a collapsed scene) is collected in one pass over its scene's keys, so
-// that no cell costs the square of its size.
-constexpr uint32_t kCellRankMax = 512;
+// the whole cell; a larger cell is radix-sorted by its warp, at a cost per particle below that of the sum
+// that follows, which one warp walks too.  The off-grid particles of the reference modes come in slot order
+// from their placement (bin_scatter_kernel).  1 M particles, one cell of 500 / 600 / 5 000: 372 / 13 800 /
+// 14 300 us a substep while cells above 512 were collected in a walk over the scene's keys, 302 / 301 / 843
+// now (2 360 / 16 700 with one thread per cell over radix-sorted particles).  The line: 1 000 cells of 200
+// take 352 us ranked and 331 sorted, 2 000 cells of 64 the same either way.
+constexpr uint32_t kCellRankMax = 128;
+
+// Sorts the k slots at run into out by one warp: 8 bits of slot - base per pass, each pass counted, scanned
+// and placed 32 slots at a time in input order.  tmp: k entries, hist: 256 counters of the warp's own.
+// out and tmp take the passes in turn so that the last one ends in out; run is only read.
+__device__ __noinline__ void warp_sort_slots(const uint32_t* run, uint32_t* out, uint32_t* tmp, uint32_t k,
+                                                uint32_t base, uint32_t slots, uint32_t* hist, int lane) {
+  const int passes = slots > 1u ? (39 - __clz(slots - 1u)) / 8 : 1;
+  const uint32_t* src = run;
+  constexpr uint32_t kAhead = 4;  // loads in flight per lane
+  for (int p = 0; p < passes; ++p) {
+    uint32_t* dst = ((passes - 1 - p) & 1) ? tmp : out;
+    const int shift = 8 * p;
+    __syncwarp();
+    for (int q = 0; q < 8; ++q) hist[q * 32 + lane] = 0u;
+    __syncwarp();
+    for (uint32_t b0 = 0; b0 < k; b0 += 32 * kAhead) {
+      uint32_t v[kAhead];
+#pragma unroll
+      for (uint32_t q = 0; q < kAhead; ++q) {
+        const uint32_t i = b0 + 32 * q + lane;
+        v[q] = i < k ? src[i] : 0u;
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < kAhead; ++q)
+        if (b0 + 32 * q + lane < k) atomicAdd(hist + ((v[q] - base) >> shift & 255u), 1u);
+    }
+    __syncwarp();
+    uint32_t c[8], sum = 0;
+    for (int q = 0; q < 8; ++q) {
+      c[q] = sum;
+      sum += hist[lane * 8 + q];
+    }
+    const uint32_t before = warp_scan_incl(sum, lane) - sum;
+    for (int q = 0; q < 8; ++q) hist[lane * 8 + q] = before + c[q];
+    __syncwarp();
+    for (uint32_t b0 = 0; b0 < k; b0 += 32 * kAhead) {
+      uint32_t v[kAhead];
+#pragma unroll
+      for (uint32_t q = 0; q < kAhead; ++q) {
+        const uint32_t i = b0 + 32 * q + lane;
+        v[q] = i < k ? src[i] : 0u;
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < kAhead; ++q) {
+        const bool in = b0 + 32 * q + lane < k;
+        const uint32_t d = in ? (v[q] - base) >> shift & 255u : 256u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t at = in ? hist[d] + uint32_t(__popc(peers & ((1u << lane) - 1u))) : 0u;
+        __syncwarp();
+        if (in) {
+          if (lane == __ffs(peers) - 1) hist[d] += uint32_t(__popc(peers));
+          dst[at] = v[q];
+        }
+        __syncwarp();
+      }
+    }
+    src = dst;
+  }
+  __syncwarp();
+}
 
 // Physics mode stages what the column-lane scatter stages: per (y,z) column u = m v + A d and w_y w_z,
 // the x weights with the mass, dx times A's x column (3 shared loads per particle and node; weights,
@@ -2458,12 +2536,18 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
   using V4 = typename V4T<T>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   auto& st = reinterpret_cast<CellStage<T, MODE>*>(smem)[threadIdx.x >> 5];
+  static_assert(sizeof(st) >= 256 * sizeof(uint32_t), "warp_sort_slots counts in the staging");
   const int4 ch = cta_chunk(w);
   const SceneDev<T>& sc = w.scenes[ch.x];
   const int lane = threadIdx.x & 31;
   const uint32_t pos = uint32_t(ch.y) + threadIdx.x;
-  const bool live = int(pos) < ch.z;
-  const uint32_t key = live ? w.keys[grouped[pos]] : 0u;
+  bool live = int(pos) < ch.z;
+  const uint32_t mine = live ? grouped[pos] : 0u;
+  const uint32_t key = live ? w.keys[mine] : 0u;
+  if (MODE != AE_MPM_MODE_PHYSICS && live && key == sc.dead_key) {  // off the grid: in order, not summed
+    ordered[pos] = mine;
+    live = false;
+  }
   uint32_t first = 0xffffffffu, cnt = 0;
   if (live) {
     const uint2 cell = w.cells[key];
@@ -2490,7 +2574,6 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
   const bool batch = live && first >= base && first + cnt <= base + 32u;
   const uint32_t in_batch = __ballot_sync(0xffffffffu, batch);
   if (in_batch) {
-    const uint32_t mine = live ? grouped[pos] : 0u;
     const uint32_t most = __reduce_max_sync(0xffffffffu, batch ? cnt : 0u);
     const int l0 = batch ? int(first - base) : 0;
     uint32_t rank = 0;
@@ -2503,17 +2586,14 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
     bool in = true;
     if (batch) {
       ordered[first + rank] = mine;
-      if (key != sc.dead_key) {
-        p2g_setup<T, MODE>(w, sc, mine, p);
-        cell_stage_put(st, sc, l0 + int(rank), p);
-        in = inside_grid(p);
-      }
+      p2g_setup<T, MODE>(w, sc, mine, p);
+      cell_stage_put(st, sc, l0 + int(rank), p);
+      in = inside_grid(p);
     }
     const bool inside = __all_sync(0xffffffffu, in);
     __syncwarp();
     for (uint32_t todo = heads & in_batch; todo; todo &= todo - 1u) {
       const int h = __ffs(todo) - 1;
-      if (__shfl_sync(0xffffffffu, key, h) == sc.dead_key) continue;
       const int k = int(__shfl_sync(0xffffffffu, cnt, h));
       am = ax = ay = az = T(0);
       add_staged(h, h + k, inside);
@@ -2529,7 +2609,6 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
     const int h = __ffs(heads) - 1;
     heads &= heads - 1u;
     const uint32_t start = __shfl_sync(0xffffffffu, first, h), k = __shfl_sync(0xffffffffu, cnt, h);
-    const uint32_t ck = __shfl_sync(0xffffffffu, key, h);
     const uint32_t* run = grouped + start;
     uint32_t* out = ordered + start;
     uint32_t slot = 0, rank = 0;
@@ -2545,17 +2624,11 @@ __global__ void __launch_bounds__(256) det_cells_kernel(WorldDev<T> w, const uin
         if (s != 0xffffffffu) out[r] = s;
       }
     } else {
-      uint32_t r = 0;
-      const uint32_t end = sc.p_off + sc.p_count;
-      for (uint32_t j0 = sc.p_off; j0 < end; j0 += 32) {
-        const bool hit = j0 + lane < end && w.keys[j0 + lane] == ck;
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (hit) out[r + __popc(m & ((1u << lane) - 1u))] = j0 + lane;
-        r += __popc(m);
-      }
+      // the clamp queue is empty until this substep's G2P
+      warp_sort_slots(run, out, reinterpret_cast<uint32_t*>(w.clamp_queue) + start, k, sc.p_off, sc.p_cap,
+                      reinterpret_cast<uint32_t*>(&st), lane);
     }
     __syncwarp();
-    if (ck == sc.dead_key) continue;  // off-grid particles of the reference modes: ordered, not summed
     am = ax = ay = az = T(0);
     int g0 = 0, g1 = 0, g2 = 0;
     for (uint32_t b0 = 0; b0 < k; b0 += 32) {
@@ -2613,6 +2686,10 @@ __global__ void init_keys_kernel(WorldDev<T> w) {
     w.keys[j] = key;
     if (int(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(w.bins + key, uint32_t(__popc(peers)));
   }
+  if (MODE != AE_MPM_MODE_PHYSICS && w.dead_cnt) {
+    const int c = __syncthreads_count(live && key == sc.dead_key);
+    if (threadIdx.x == 0) w.dead_cnt[blockIdx.x] = uint32_t(c);
+  }
 }
 
 // ============================================================================================
@@ -2629,15 +2706,6 @@ __global__ void init_keys_kernel(WorldDev<T> w) {
 // One CTA scans 4096 nodes (64 blocks) and zeroes the counts it read, so the array is clean for
 // the next count; offsets are written only where a count is not zero.  The CTA that finishes last
 // scans the segment totals (no CTA waits for another).
-
-__device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  return x;
-}
 
 template <class T>
 __device__ __forceinline__ void bin_scan(const WorldDev<T>& w, uint64_t nodes, const uint32_t* __restrict__ dead_blk,
@@ -2765,7 +2833,9 @@ __global__ void __launch_bounds__(kBinThreads) scan_and_grid_kernel(WorldDev<T> 
     grid_update<T, AE_MPM_MODE_PHYSICS>(w, blk_epoch, epoch, zero_count, blockIdx.x - scan_ctas, gridDim.x - scan_ctas);
 }
 
-template <class T>
+// kOff: the deterministic reference modes, whose particles off the grid, any number of them on one key,
+// are placed in slot order: after those of the scene's earlier chunks, in order within their own.
+template <class T, bool kOff>
 __global__ void __launch_bounds__(256) bin_scatter_kernel(WorldDev<T> w, uint32_t* __restrict__ perm,
                                                           uint32_t n_slots) {
   let_next_start();
@@ -2774,11 +2844,33 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(WorldDev<T> w, uint32_
   const int j = ch.y + threadIdx.x, lane = threadIdx.x & 31;
   const bool live = j < ch.z;
   const uint32_t key = live ? w.keys[j] : 0xffffffffu;
+  const bool count_off = kOff && w.dead_cnt[blockIdx.x] != 0u;  // uniform over the CTA
+  bool off = false;
+  uint32_t pos = 0;
+  if (count_off) {
+    __shared__ uint32_t warp_off[8], earlier;
+    const SceneDev<T>& sc = w.scenes[ch.x];
+    off = key == sc.dead_key;
+    if (threadIdx.x == 0) earlier = 0u;
+    const uint32_t mask = __ballot_sync(0xffffffffu, off);
+    if (lane == 0) warp_off[threadIdx.x >> 5] = uint32_t(__popc(mask));
+    uint32_t sum = 0;
+    for (uint32_t c = blockIdx.x - (uint32_t(ch.y) - sc.p_off) / blockDim.x + threadIdx.x; c < blockIdx.x; c += blockDim.x)
+      sum += w.dead_cnt[c];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    __syncthreads();
+    if (lane == 0 && sum) atomicAdd(&earlier, sum);
+    __syncthreads();
+    pos = earlier + uint32_t(__popc(mask & ((1u << lane) - 1u)));
+    for (uint32_t k = 0; k < (threadIdx.x >> 5); ++k) pos += warp_off[k];
+    if (off) pos += w.bin_off[key] + w.seg_off[key / kBinSeg];
+  }
   const uint32_t peers = __match_any_sync(0xffffffffu, key);
   const int leader = __ffs(peers) - 1;
-  uint32_t pos = 0;
-  if (live && lane == leader) pos = atomicAdd(w.bin_off + key, uint32_t(__popc(peers))) + w.seg_off[key / kBinSeg];
-  pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
+  uint32_t at = 0;
+  if (live && !off && lane == leader) at = atomicAdd(w.bin_off + key, uint32_t(__popc(peers))) + w.seg_off[key / kBinSeg];
+  at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & ((1u << lane) - 1u));
+  if (!off) pos = at;
   if (live && pos < n_slots) perm[pos] = uint32_t(j);
 }
 
@@ -3268,6 +3360,7 @@ class World final : public WorldBase {
       if (x.deterministic) {
         reserve(&World::cells_, sizeof(uint2) * nodes, kZero);
         reserve(&World::ordered_, sizeof(uint32_t) * x.pc, kZero);
+        reserve(&World::dead_cnt_, sizeof(uint32_t) * std::max<uint64_t>(x.chunks, 1), kNone);
       }
     } else if (x.deterministic) {
       reserve(&World::cell_slot_, sizeof(uint32_t) * nodes, kOnes);
@@ -4127,7 +4220,10 @@ class World final : public WorldBase {
     if (opts_.block_threads != 128 && opts_.block_threads != 256) opts_.block_threads = 256;
     if (opts_.sort_interval < 1) opts_.sort_interval = 1;
     if (opts_.p2g_variant < kVarTile || opts_.p2g_variant > kVarLanes) opts_.p2g_variant = kVarLanes;
-    if (opts_.block_threads != chunk_threads_) chunks_dirty_ = true;
+    if (opts_.block_threads != chunk_threads_) {
+      chunks_dirty_ = true;
+      if (dead_cnt_) keys_stale_ = true;  // counted per chunk
+    }
     if (chunks_dirty_) {
       chunk_threads_ = opts_.block_threads;
       h_chunks_.clear();
@@ -4220,6 +4316,7 @@ class World final : public WorldBase {
     w.bin_off = bin_off_;
     w.seg_off = seg_ ? seg_ + n_segs_ : nullptr;
     w.cells = cells_;
+    w.dead_cnt = mode_ == AE_MPM_MODE_PHYSICS ? nullptr : dead_cnt_;
     w.acc = acc_;
     w.vel = vel_;
     w.blk_flag = blk_flag_;
@@ -4468,7 +4565,7 @@ class World final : public WorldBase {
     if (sort_first) {
       launch_dependent(scan_and_grid_kernel<T>, n_segs_ + sms * 4, kBinThreads, 0, wg, total_blocks_ * 64, dead_blk_,
                        seg_, counters_ + 5, n_segs_, blk_epoch_, counters_ + 2, touched_count(par ^ 1));
-      launch_dependent(bin_scatter_kernel<T>, unsigned(n_chunks_), unsigned(chunk_threads_), 0, wg, bin_perm_,
+      launch_dependent(bin_scatter_kernel<T, false>, unsigned(n_chunks_), unsigned(chunk_threads_), 0, wg, bin_perm_,
                        uint32_t(total_cap_));
       perm_ = bin_perm_;
       sorted_ = true;
@@ -4515,7 +4612,8 @@ class World final : public WorldBase {
     if (dense_sort_) {
       WorldDev<T> w = dev(false);
       bin_scan_kernel<T><<<n_segs_, kBinThreads, 0, stream_>>>(w, total_blocks_ * 64, dead_blk_, seg_, counters_ + 5);
-      bin_scatter_kernel<T><<<n_chunks_, chunk_threads_, 0, stream_>>>(w, bin_perm_, uint32_t(total_cap_));
+      const auto scatter = w.dead_cnt ? bin_scatter_kernel<T, true> : bin_scatter_kernel<T, false>;
+      scatter<<<n_chunks_, chunk_threads_, 0, stream_>>>(w, bin_perm_, uint32_t(total_cap_));
       // a deterministic substep orders each cell (det_cells_kernel) before anything reads the order
       perm_ = opts_.deterministic ? ordered_ : bin_perm_;
       launches_ += 2;
@@ -4652,6 +4750,7 @@ class World final : public WorldBase {
   bool dense_sort_ = false;  // particles are grouped by counting (bins_), not by the radix sort
   uint32_t *bins_ = nullptr, *bin_off_ = nullptr, *seg_ = nullptr, *bin_perm_ = nullptr;
   uint2* cells_ = nullptr;        // deterministic dense grouping: each cell's places
+  uint32_t* dead_cnt_ = nullptr;  // ... the off-grid particles of each chunk
   uint32_t* ordered_ = nullptr;   // ... and the sorted places in slot order within each cell
   uint32_t n_segs_ = 0;
   const uint32_t* perm_ = nullptr;

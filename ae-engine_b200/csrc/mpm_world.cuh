@@ -72,6 +72,7 @@ struct WorldDev {
   // deterministic worlds with dense grouping, per node: {first sorted place within its scan segment,
   // particles} of the cell based there
   uint2* cells;
+  uint32_t* dead_cnt;  // ... in the reference modes, per chunk: live particles off the grid
   V4* acc;
   V4* vel;
   uint32_t* blk_flag;

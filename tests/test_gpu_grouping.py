@@ -174,3 +174,97 @@ def test_deterministic_world_takes_particles_far_outside_its_grid(ctx, grid):
     for f in ("pos", "vel", "F", "J", "C"):
         assert np.array_equal(getattr(out[0][0], f), getattr(out[1][1], f)), f
     assert rel(out[0][0].pos, out[2][0].pos) <= 1e-6
+
+
+def crowd(n, g, k, seed):
+    # n particles spread over a grid of g nodes per axis, k of them in one cell
+    rng = np.random.default_rng(seed)
+    dx = 1.0 / g
+    x = (4.0 + (g - 8.0) * rng.random((n, 3))) * dx
+    x[rng.choice(n, k, replace=False)] = (6.6 + 0.8 * rng.random((k, 3))) * dx
+    p = S.make_particles(x, (0.2, -0.1, 0.1), 1e-5, 0)
+    p.J[:] = 1.0
+    return M.Scene(n=(g, g, g), dx=dx, dt=1e-5, materials=[S.jelly(E=10.0)], max_particles=n), p
+
+
+@pytest.mark.parametrize("n,k", [(513, 513), (1500, 640), (40000, 5000), (70001, 4097), (70001, 69000)])
+def test_deterministic_sums_over_one_crowded_cell_repeat(ctx, n, k):
+    # slots of one and of two scenes, sorted in two and in three passes of 8 bits
+    sc, p = crowd(n, 24, k, n + k)
+    other, q = crowd(900, 16, 700, 3)
+    ref = p.astype(np.float64)
+    O.run(sc, ref, 3)
+    runs = []
+    for scenes in ([sc], [sc], [other, sc]):
+        w = M.World(ctx, scenes, M.exec_opts(deterministic=1))
+        if len(scenes) == 2:
+            w.upload(0, q)
+        w.upload(len(scenes) - 1, p)
+        w.step(3)
+        w.sync(raise_on_error=False)
+        runs.append(w.download(len(scenes) - 1, n))
+        w.close()
+    assert rel(runs[0].pos, ref.pos) <= 1e-5
+    for r in runs[1:]:
+        for f in ("pos", "vel", "F", "J", "C"):
+            assert np.array_equal(getattr(r, f), getattr(runs[0], f)), f
+
+
+@pytest.mark.parametrize("threads", [128, 256])
+@pytest.mark.parametrize("mode", [M.MODE_REFERENCE, M.MODE_VELOCITY_ONLY])
+@pytest.mark.parametrize("n,share", [(700, 1.0), (5003, 0.5), (40000, 0.9)])
+def test_deterministic_reference_modes_with_many_off_grid_particles_repeat(ctx, mode, n, share, threads):
+    # most of a scene above the grid's top, where the reference lets it fall back in
+    rng = np.random.default_rng(n)
+    g, dx = 20, 0.5
+    p = M.Particles.empty(n)
+    p.pos[:] = (0.5 + (g - 4) * rng.random((n, 3))) * dx
+    above = rng.random(n) < share
+    p.pos[above, 1] = (g + 0.6 + 0.5 * rng.random(int(above.sum()))) * dx
+    p.vel[:] = rng.normal(0, 0.3, (n, 3))
+    p.vel[:, 1] -= 20.0
+    p.mass[:] = 0.01
+    p.J[:] = 1.0
+    sc = M.Scene(n=(g, g, g), dx=dx, dt=0.01, materials=[M.material(young_modulus=1e3, poisson_ratio=0.25)], mode=mode,
+                 gravity=(0, -9.81, 0), max_particles=n + 100)
+    out = []
+    for det in (1, 1, 0):
+        w = M.World(ctx, [sc, sc], M.exec_opts(deterministic=det, block_threads=threads))
+        w.upload(0, p)
+        w.upload(1, p)
+        w.step(5)
+        w.sync(raise_on_error=False)
+        out.append((w.download(0, n), w.download(1, n)))
+        w.close()
+    for f in ("pos", "vel", "F", "J", "C"):
+        assert np.array_equal(getattr(out[0][0], f), getattr(out[1][0], f)), f
+        assert np.array_equal(getattr(out[0][0], f), getattr(out[0][1], f)), f
+    assert rel(out[0][0].pos, out[2][0].pos) <= 2e-5
+
+
+def test_deterministic_substeps_do_not_stall_on_one_crowded_cell(ctx):
+    # 600 particles of 1 M in one cell cost about what 500 cost (walking the scene for them took 40 times
+    # as long), and so do 600 particles above the grid in a reference mode
+    import torch
+
+    def time_us(sc, p):
+        w = M.World(ctx, [sc], M.exec_opts(deterministic=1))
+        w.upload(0, p)
+        w.step(4)
+        st = torch.cuda.ExternalStream(w.stream())
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(st)
+        w.step(6)
+        b.record(st)
+        b.synchronize()
+        w.close()
+        return a.elapsed_time(b) * 1000.0 / 6
+
+    n = 1000000
+    few, many = (time_us(*crowd(n, 96, k, 1)) for k in (500, 600))
+    assert many <= 4.0 * few
+    sc, p = crowd(n, 96, 1, 1)
+    sc.mode, sc.gravity, p.vel[:] = M.MODE_REFERENCE, (0, 0, 0), 0.0
+    few = time_us(sc, p)
+    p.pos[:600, 1] += 1.0
+    assert time_us(sc, p) <= 4.0 * few
