@@ -4632,8 +4632,8 @@ class World final : public WorldBase {
     if (n_chunks_ > 0) {
       mark(0);
       const bool sort_now = phase_ == 0 && !sorted_;
-      // the scan shares its launch with the grid update
-      const bool joined = sort_now && fused() && dense_sort_ && keys_fresh_;
+      // the scan shares its launch with the grid update, except where stages are timed one by one
+      const bool joined = sort_now && fused() && dense_sort_ && keys_fresh_ && !stage_events_;
       if (sort_now && !joined) sort_particles();
       mark(1);
       WorldDev<T> w = dev(sorted_);

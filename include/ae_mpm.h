@@ -307,7 +307,9 @@ int ae_mpm_world_errors(ae_mpm_world* world, uint32_t scene, uint32_t* error_wor
 int ae_mpm_world_launch_count(const ae_mpm_world* world, uint64_t* launches);
 /* Runs n substeps eagerly with CUDA events between the stages on the world's stream and returns
  * the mean device time per substep of each stage in microseconds:
- * out_us = [sort, P2G (deterministic: cell sums + gather), grid update, G2P, whole substep]. */
+ * out_us = [sort, P2G (deterministic: cell sums + gather), grid update, G2P, whole substep].
+ * The stages run as launches of their own here; ae_mpm_world_step lets the sort share one with the
+ * grid update where it can. */
 int ae_mpm_world_stage_times(ae_mpm_world* world, uint32_t n_substeps, double out_us[5]);
 /* The same measurement with a sixth entry: out_us[5] = the G2P kernel alone (in physics mode with
  * the column-lane P2G, the fused G2P + P2G kernel alone), without the snow clamp that out_us[3]

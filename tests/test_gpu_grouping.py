@@ -268,3 +268,18 @@ def test_deterministic_substeps_do_not_stall_on_one_crowded_cell(ctx):
     few = time_us(sc, p)
     p.pos[:600, 1] += 1.0
     assert time_us(sc, p) <= 4.0 * few
+
+
+def test_stage_times_count_the_grouping_as_the_sort(ctx):
+    # every substep groups 1 M particles (scan and placement, some 20 us) or none does: the grid update's
+    # time is the same either way
+    sc, p = crowd(1000000, 96, 1, 2)
+    t = {}
+    for interval in (1, 64):
+        w = M.World(ctx, [sc], M.exec_opts(sort_interval=interval))
+        w.upload(0, p)
+        w.step(4)
+        t[interval] = w.stage_times(20)
+        w.close()
+    assert t[1]["sort"] > 5.0
+    assert t[1]["grid"] <= 1.3 * t[64]["grid"]
