@@ -856,6 +856,10 @@ static int host_sort(ae_mpm_ctx* ctx, const uint32_t* keys, uint64_t n, uint32_t
     cudaError_t e = aemp::sort_scratch_alloc(ctx->sort, n);
     if (e != cudaSuccess) return fail(ctx, AE_MPM_ENOMEM, cudaGetErrorString(e));
   }
+  if (counting) {
+    cudaError_t e = aemp::sort_bins_alloc(ctx->sort);
+    if (e != cudaSuccess) return fail(ctx, AE_MPM_ENOMEM, cudaGetErrorString(e));
+  }
   if (ctx->sort_keys_cap < n) {
     cudaFree(ctx->sort_keys);
     ctx->sort_keys = nullptr;

@@ -353,15 +353,17 @@ cudaError_t sort_scratch_alloc(SortScratch& s, uint64_t n, SortAllocFn alloc, vo
   if ((e = A(&s.keys_alt, sizeof(uint32_t) * m)) != cudaSuccess) return e;
   if ((e = A(&s.vals_a, sizeof(uint32_t) * m)) != cudaSuccess) return e;
   if ((e = A(&s.vals_b, sizeof(uint32_t) * m)) != cudaSuccess) return e;
-  if (n > uint64_t(kSmallSortMax) && (e = A(&s.bins, sizeof(uint32_t) << kCountingSortBits)) != cudaSuccess) return e;
   s.n_cap = n;
   return cudaSuccess;
 }
 
+cudaError_t sort_bins_alloc(SortScratch& s) {
+  return s.bins ? cudaSuccess : cudaMalloc(&s.bins, sizeof(uint32_t) << kCountingSortBits);
+}
+
 uint64_t sort_scratch_bytes(uint64_t n) {
   const uint64_t m = n > 0 ? n : 1, tiles = sort_tiles(m);
-  const uint64_t words[4] = {kMaxRadix * tiles, kMaxRadix * tiles, 4 * kMaxRadix,
-                             n > uint64_t(kSmallSortMax) ? uint64_t(1) << kCountingSortBits : 0};
+  const uint64_t words[3] = {kMaxRadix * tiles, kMaxRadix * tiles, 4 * kMaxRadix};
   uint64_t sum = 0;
   for (uint64_t v : words) sum += (sizeof(uint32_t) * v + 255) & ~uint64_t(255);
   return sum + 3 * ((sizeof(uint32_t) * m + 255) & ~uint64_t(255));

@@ -57,7 +57,7 @@ struct SortScratch {
   uint32_t* keys_alt = nullptr; // [n]
   uint32_t* vals_a = nullptr;   // [n]
   uint32_t* vals_b = nullptr;   // [n]
-  uint32_t* bins = nullptr;     // [1 << kCountingSortBits] (counting sort; allocated for n > kSmallSortMax)
+  uint32_t* bins = nullptr;     // [1 << kCountingSortBits], only after sort_bins_alloc (counting sort)
   uint64_t n_cap = 0;
 };
 
@@ -69,6 +69,7 @@ typedef cudaError_t (*SortAllocFn)(void* user, void** p, size_t bytes);
 typedef void (*SortFreeFn)(void* user, void* p);
 uint64_t sort_scratch_bytes(uint64_t n);  // of such a scratch, each array rounded to 256
 cudaError_t sort_scratch_alloc(SortScratch& s, uint64_t n, SortAllocFn alloc = nullptr, void* user = nullptr);
+cudaError_t sort_bins_alloc(SortScratch& s);  // adds the counting sort's bins (cudaMalloc) if not there yet
 void sort_scratch_free(SortScratch& s, SortFreeFn release = nullptr, void* user = nullptr);
 
 // Sorts keys[0..n) (only bits [0, key_bits) compared).  On return *perm_out points to the
@@ -82,7 +83,8 @@ int radix_sort_pairs(uint32_t* keys, uint64_t n, int key_bits, SortScratch& s, c
 // Groups keys[0..n) by key in one pass (key_bits <= kCountingSortBits): a histogram, one scan
 // over the 2^key_bits bins and a scatter that claims places with atomics.  The keys come out
 // sorted, but equal keys in no defined order (the order atomics give them), so only callers whose
-// results do not depend on that order may use it.  Same outputs and lifetime rules as
+// results do not depend on that order may use it.  Worlds group their particles by counters per grid
+// node instead; this form serves ae_mpm_counting_sort_keys.  Same outputs and lifetime rules as
 // radix_sort_pairs.  n <= kSmallSortMax, wider keys or scratch without bins go to
 // radix_sort_pairs (which clobbers `keys`); the counting pass itself only reads them.  Returns the
 // launch count.
