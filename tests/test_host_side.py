@@ -1,15 +1,18 @@
-"""CPU test of the drop-in calls' error returns, with a CUDA runtime and a world of the test's own."""
+"""CPU tests of the C calls' host side, with a CUDA runtime and a world of the tests' own."""
 import os
 import subprocess
+
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def test_failed_calls_leave_nothing_in_flight(tmp_path):
+@pytest.mark.parametrize("name", ["dropin_errors", "batch_priorities"])
+def test_host_side(tmp_path, name):
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    exe = str(tmp_path / "dropin_errors")
+    exe = str(tmp_path / name)
     subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-fopenmp", "-I" + os.path.join(cuda, "include"),
-                    os.path.join(ROOT, "tests", "cpp", "test_dropin_errors.cpp"), "-o", exe,
+                    os.path.join(ROOT, "tests", "cpp", "test_%s.cpp" % name), "-o", exe,
                     # the library's other parts are not called
                     "-no-pie", "-Wl,--unresolved-symbols=ignore-all"], check=True)
     r = subprocess.run([exe], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=120)
