@@ -283,3 +283,28 @@ def test_stage_times_count_the_grouping_as_the_sort(ctx):
         w.close()
     assert t[1]["sort"] > 5.0
     assert t[1]["grid"] <= 1.3 * t[64]["grid"]
+
+
+@pytest.mark.parametrize("mode,deterministic,interval", [(M.MODE_PHYSICS, 0, 1), (M.MODE_PHYSICS, 0, 3), (M.MODE_PHYSICS, 0, 8),
+                                                         (M.MODE_PHYSICS, 1, 1), (M.MODE_REFERENCE, 0, 4),
+                                                         (M.MODE_REFERENCE, 1, 1)])
+def test_graphs_carry_the_sort_of_their_period(ctx, mode, deterministic, interval):
+    # a run of whole periods consists of graph launches alone
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    sc, p = crowd(20000, 32, 1, 4)
+    sc.mode = mode
+    w = M.World(ctx, [sc], M.exec_opts(sort_interval=interval, deterministic=deterministic))
+    w.upload(0, p)
+    w.step(96)
+    w.step(48)  # periods that start on the other parity are captured by now
+    w.sync(raise_on_error=False)
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        w.step(48)
+        w.sync(raise_on_error=False)
+        torch.cuda.synchronize()
+    w.close()
+    names = [e.name for e in prof.events()]
+    assert sum("GraphLaunch" in n for n in names) == 48 // (interval if interval % 2 == 0 else 2 * interval)
+    assert sum("LaunchKernel" in n for n in names) == 0
