@@ -2208,6 +2208,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) g2p2g_kernel(Worl
 // between 4 and 32, because scattered particles are runs of their own that a warp sums one after
 // another (a short queue took 16 us with 32 entries per warp).  80 registers and 6 CTAs per SM: at 64
 // and 8 the return mapping spills (16.7 against 19.3 us a launch in a batch of snow and other scenes).
+// Launched with those 6 per SM; with 8, the last two waited for a second wave (20 000 quiet particles
+// sorted every substep: 19.3 -> 18.8 us).
 template <class T>
 __global__ void __launch_bounds__(128, 6) snow_clamp_scatter_kernel(WorldDev<T> w, int write_keys) {
   using V4 = typename V4T<T>::type;
@@ -4582,7 +4584,7 @@ class World final : public WorldBase {
     ++launches_;
     mark(5);  // the fused kernel alone ends here
     if (has_snow_) {
-      snow_clamp_scatter_kernel<T><<<sms * 8, 128, fused_smem(128), stream_>>>(wf, write_keys ? 1 : 0);
+      snow_clamp_scatter_kernel<T><<<sms * 6, 128, fused_smem(128), stream_>>>(wf, write_keys ? 1 : 0);
       ++launches_;
     }
     mark(4);
