@@ -3146,22 +3146,38 @@ HostView<double> host_view<double>(const void* host) {
 // leave the later one there; kernels that write both in place would leave a mixture.
 template <class T>
 static bool arrays_overlap(const HostView<T>* views, const uint64_t* counts, uint32_t k) {
-  std::vector<std::pair<uintptr_t, uintptr_t>> used;
-  used.reserve(7 * size_t(k));
-  const uint64_t len[6] = {3, 3, 9, 1, 9, 1};
-  for (uint32_t i = 0; i < k; ++i) {
-    if (counts[i] == 0) continue;
-    for (int q = 0; q < 6; ++q) {
-      const uintptr_t a = reinterpret_cast<uintptr_t>(views[i].f[q]);
-      used.emplace_back(a, a + sizeof(T) * len[q] * counts[i]);
+  typedef std::pair<uintptr_t, uintptr_t> Range;  // begin, end
+  const auto array = [&](uint32_t i, int q) {
+    static const uint64_t bytes[7] = {3 * sizeof(T), 3 * sizeof(T), 9 * sizeof(T), sizeof(T), 9 * sizeof(T), sizeof(T), 2};
+    const uintptr_t a = reinterpret_cast<uintptr_t>(q < 6 ? static_cast<const void*>(views[i].f[q]) : views[i].mat);
+    return Range(a, a + bytes[q] * counts[i]);
+  };
+  const auto apart = [](Range* r, size_t n) {
+    std::sort(r, r + n);
+    for (size_t q = 1; q < n; ++q)
+      if (r[q].first < r[q - 1].second) return false;
+    return true;
+  };
+  // the usual view sets need no sort of all arrays: one buffer per array, its scenes one after another
+  Range span[7] = {};
+  bool in_order = true;
+  for (int q = 0; q < 7 && in_order; ++q) {
+    bool any = false;
+    for (uint32_t i = 0; i < k && in_order; ++i) {
+      if (counts[i] == 0) continue;
+      const Range r = array(i, q);
+      in_order = !any || r.first >= span[q].second;
+      if (!any) span[q].first = r.first;
+      span[q].second = r.second;
+      any = true;
     }
-    const uintptr_t a = reinterpret_cast<uintptr_t>(views[i].mat);
-    used.emplace_back(a, a + sizeof(uint16_t) * counts[i]);
   }
-  std::sort(used.begin(), used.end());
-  for (size_t q = 1; q < used.size(); ++q)
-    if (used[q].first < used[q - 1].second) return true;
-  return false;
+  if (in_order && apart(span, 7)) return false;
+  std::vector<Range> used;
+  used.reserve(7 * size_t(k));
+  for (uint32_t i = 0; i < k; ++i)
+    for (int q = 0; q < 7 && counts[i] > 0; ++q) used.push_back(array(i, q));
+  return !apart(used.data(), used.size());
 }
 
 bool views_overlap(const ae_mpm_particles* views, const uint64_t* counts, uint32_t k) {
@@ -3476,23 +3492,25 @@ class World final : public WorldBase {
   // array is refused by the driver, a kernel would run past it.  Anything else (host, managed or another
   // device's memory, odd addresses, short arrays) travels through the staging area.
   struct DirectViews {
-    uintptr_t lo = 0, hi = 0;  // the allocation the last array lay in
+    struct {
+      uintptr_t lo, hi;
+    } known[8] = {};  // allocations found in this call, the last 8: one per array of the views and one more
+    uint32_t next = 0;
 
     bool array(const void* p, size_t bytes, size_t align) {
       const uintptr_t a = reinterpret_cast<uintptr_t>(p);
       if (a % align != 0) return false;
-      if (a < lo || a >= hi) {
-        int dev = 0;
-        cudaPointerAttributes at{};
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-          cudaGetLastError();
-          return false;
-        }
-        if (at.type != cudaMemoryTypeDevice || at.device != dev || !device_allocation(a, lo, hi)) {
-          lo = hi = 0;
-          return false;
-        }
+      for (const auto& k : known)
+        if (a >= k.lo && a < k.hi) return bytes <= k.hi - a;
+      int dev = 0;
+      cudaPointerAttributes at{};
+      if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
       }
+      uintptr_t lo = 0, hi = 0;
+      if (at.type != cudaMemoryTypeDevice || at.device != dev || !device_allocation(a, lo, hi)) return false;
+      known[next++ % 8] = {lo, hi};
       return a >= lo && a < hi && bytes <= hi - a;
     }
     bool takes(const HostView<T>& hv, uint64_t n) {
