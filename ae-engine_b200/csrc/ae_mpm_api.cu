@@ -388,7 +388,11 @@ int dropin_run(ae_mpm_ctx* ctx, int mode, const ae_mpm_particles* buffer, uint64
   // lists of some length gather on the OpenMP team (reads only; 4 000 particles on one thread made the
   // call 320 us, 10 000 on eight 190); the scatter back is parallel only for
   // ascending (hence distinct) indices, so a repeated index keeps the reference's last-write-wins
-  const int t_host = n >= 1024 ? std::min(8, omp_get_max_threads()) : 1;
+  // (hence on one thread: a gather spread over the cores pays off later there, for a velocity-only call
+  // from 2 048 particles on, for a reference call, which scatters all arrays, from 4 096: 3 000 in random
+  // order 277 us spread, 248 on one thread)
+  const uint64_t spread = ascending ? 1024 : (full ? 4096 : 2048);
+  const int t_host = n >= spread ? std::min(8, omp_get_max_threads()) : 1;
 #pragma omp parallel for num_threads(t_host) schedule(static)
   for (int64_t kk = 0; kk < int64_t(n); ++kk) {
     const uint64_t k = uint64_t(kk);

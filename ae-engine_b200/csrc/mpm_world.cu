@@ -1373,8 +1373,12 @@ __device__ __forceinline__ bool snow_return(const MatDev& md, bool redo, T* F, T
   return fb;
 }
 
-// mpm_substep_serial_active / parallel_with_indices G2P (mpm_solver.rs:914-1053, 1206-1325)
-template <class T>
+// mpm_substep_serial_active / parallel_with_indices G2P (mpm_solver.rs:914-1053, 1206-1325).
+// kAhead: the nine nodes of a plane are loaded before any is used, which hides their latency where the
+// GPU holds few warps; at more registers per thread it has fewer of them where it could hold many (the
+// kernel alone with and without: 20 000 particles 19.4 / 22.5 us, 30 000 19.1 / 21.4, 50 000 26.3 / 24.4,
+// 400 000 99.6 / 78.3).
+template <class T, bool kAhead>
 __device__ __forceinline__ void g2p_reference(const VelTile<T>& vt, const SceneDev<T>& sc, const T* pos, const T* f,
                                               G2POut<T>& o) {
   using V4 = typename V4T<T>::type;
@@ -1388,52 +1392,69 @@ __device__ __forceinline__ void g2p_reference(const VelTile<T>& vt, const SceneD
     g[a] = max(gu, 0);
   }
   T nv[3] = {0, 0, 0}, nc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, gvm[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  T wgt[3][3], dwg[3][3];
+  // one node with mass: velocity, affine matrix and velocity gradient
+  const auto add = [&](const V4& gv, int X, int Y, int Z, T ww, T dwx, T dwy, T dwz) {
+    T g3[3] = {gv.x, gv.y, gv.z};
+    nv[0] += ww * g3[0];
+    nv[1] += ww * g3[1];
+    nv[2] += ww * g3[2];
+    T d3[3] = {(T(X) + T(0.5)) * sc.dx + sc.origin[0] - pos[0], (T(Y) + T(0.5)) * sc.dx + sc.origin[1] - pos[1],
+               (T(Z) + T(0.5)) * sc.dx + sc.origin[2] - pos[2]};
+    T scale = T(4) * sc.inv_dx * sc.inv_dx * ww;
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      wgt[a][k] = b_spline(T(k) - fx[a]);
-      dwg[a][k] = b_spline_deriv(T(k) - fx[a]) * sc.inv_dx;
-    }
-#pragma unroll 1
-  for (int dk = 0; dk < 3; ++dk) {
-    // the plane's nine nodes first, so that their loads overlap (a node outside the grid weighs 0)
-    V4 node[9];
+      for (int c = 0; c < 3; ++c) nc[r * 3 + c] += scale * g3[r] * d3[c];
+    T dw[3] = {dwx, dwy, dwz};
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      const int X = g[0] + q % 3, Y = g[1] + q / 3, Z = g[2] + dk;
-      node[q] = (X < sc.n[0] && Y < sc.n[1] && Z < sc.n[2]) ? vt(sc, X, Y, Z) : mk4(T(0), T(0), T(0), T(0));
-    }
-    const T wz = dk == 0 ? wgt[2][0] : (dk == 1 ? wgt[2][1] : wgt[2][2]);
-    const T dwz = dk == 0 ? dwg[2][0] : (dk == 1 ? dwg[2][1] : dwg[2][2]);
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-    for (int dj = 0; dj < 3; ++dj)
+      for (int c = 0; c < 3; ++c) gvm[r * 3 + c] -= ww * g3[r] * dw[c];
+  };
+  if constexpr (kAhead) {
+    T wgt[3][3], dwg[3][3];
 #pragma unroll
-      for (int di = 0; di < 3; ++di) {
-        T wx = wgt[0][di], wy = wgt[1][dj];
-        T ww = wx * wy * wz;
-        if (ww < T(1e-10)) continue;
-        int X = g[0] + di, Y = g[1] + dj, Z = g[2] + dk;
-        const V4 gv = node[dj * 3 + di];
-        if (gv.w < T(1e-12)) continue;
-        T g3[3] = {gv.x, gv.y, gv.z};
-        nv[0] += ww * g3[0];
-        nv[1] += ww * g3[1];
-        nv[2] += ww * g3[2];
-        T d3[3] = {(T(X) + T(0.5)) * sc.dx + sc.origin[0] - pos[0], (T(Y) + T(0.5)) * sc.dx + sc.origin[1] - pos[1],
-                   (T(Z) + T(0.5)) * sc.dx + sc.origin[2] - pos[2]};
-        T scale = T(4) * sc.inv_dx * sc.inv_dx * ww;
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) nc[r * 3 + c] += scale * g3[r] * d3[c];
-        T dw[3] = {dwg[0][di], dwg[1][dj], dwz};
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) gvm[r * 3 + c] -= ww * g3[r] * dw[c];
+      for (int k = 0; k < 3; ++k) {
+        wgt[a][k] = b_spline(T(k) - fx[a]);
+        dwg[a][k] = b_spline_deriv(T(k) - fx[a]) * sc.inv_dx;
       }
+#pragma unroll 1
+    for (int dk = 0; dk < 3; ++dk) {
+      V4 node[9];  // (a node outside the grid weighs 0)
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const int X = g[0] + q % 3, Y = g[1] + q / 3, Z = g[2] + dk;
+        node[q] = (X < sc.n[0] && Y < sc.n[1] && Z < sc.n[2]) ? vt(sc, X, Y, Z) : mk4(T(0), T(0), T(0), T(0));
+      }
+      const T wz = dk == 0 ? wgt[2][0] : (dk == 1 ? wgt[2][1] : wgt[2][2]);
+      const T dwz = dk == 0 ? dwg[2][0] : (dk == 1 ? dwg[2][1] : dwg[2][2]);
+#pragma unroll
+      for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+        for (int di = 0; di < 3; ++di) {
+          const T ww = wgt[0][di] * wgt[1][dj] * wz;
+          const V4 gv = node[dj * 3 + di];
+          if (ww < T(1e-10) || gv.w < T(1e-12)) continue;
+          add(gv, g[0] + di, g[1] + dj, g[2] + dk, ww, dwg[0][di], dwg[1][dj], dwz);
+        }
+    }
+  } else {
+#pragma unroll 1
+    for (int dk = 0; dk < 3; ++dk)
+#pragma unroll 1
+      for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+        for (int di = 0; di < 3; ++di) {
+          const T ww = b_spline(T(di) - fx[0]) * b_spline(T(dj) - fx[1]) * b_spline(T(dk) - fx[2]);
+          const int X = g[0] + di, Y = g[1] + dj, Z = g[2] + dk;
+          if (ww < T(1e-10) || X >= sc.n[0] || Y >= sc.n[1] || Z >= sc.n[2]) continue;
+          const V4 gv = vt(sc, X, Y, Z);
+          if (gv.w < T(1e-12)) continue;
+          add(gv, X, Y, Z, ww, b_spline_deriv(T(di) - fx[0]) * sc.inv_dx, b_spline_deriv(T(dj) - fx[1]) * sc.inv_dx,
+              b_spline_deriv(T(dk) - fx[2]) * sc.inv_dx);
+        }
   }
   if (!t_finite(nv[0]) || !t_finite(nv[1]) || !t_finite(nv[2])) {
     nv[0] = nv[1] = nv[2] = T(0);
@@ -1590,7 +1611,7 @@ __device__ __forceinline__ void stencil_range(const SceneDev<T>& sc, T x, int a,
   hi = min(g + 2, sc.n[a] - 1);
 }
 
-template <class T, int MODE>
+template <class T, int MODE, bool kAhead>
 __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T) == 4) ? 4 : 1) g2p_kernel(WorldDev<T> w, uint32_t* epoch,
                                                                                                     int write_keys) {
   using V4 = typename V4T<T>::type;
@@ -1696,7 +1717,7 @@ __global__ void __launch_bounds__(256, (MODE == AE_MPM_MODE_PHYSICS && sizeof(T)
       g2p_physics_move<T>(sc, md, x0, pv, F, a3.y, o);
       if (!o.needs_clamp) g2p_physics_affine<T>(sc, md, a0.w, o);
     } else if (MODE == AE_MPM_MODE_REFERENCE) {
-      g2p_reference<T>(vt, sc, x0, F, o);
+      g2p_reference<T, kAhead>(vt, sc, x0, F, o);
     } else {
       const V4 a4 = ld4(w.in[4] + src), a5 = ld4(w.in[5] + src), a6 = ld4(w.in[6] + src);
       g2p_velonly<T>(vt, sc, x0, o);
@@ -4439,7 +4460,10 @@ class World final : public WorldBase {
     }
     mark(3);
     const size_t g2p_smem = sizeof(V4) * ((MODE == AE_MPM_MODE_PHYSICS ? 0 : max_tile_nodes()) + 3 * chunk_threads_);
-    g2p_kernel<T, MODE><<<n_chunks_, chunk_threads_, g2p_smem, stream_>>>(w, counters_ + 2, write_keys ? 1 : 0);
+    // node loads ahead of their use in the reference mode while a CTA of 256 threads per SM holds all slots
+    const bool ahead = MODE == AE_MPM_MODE_REFERENCE && total_cap_ <= uint64_t(sms) * 256;
+    const auto g2p = ahead ? g2p_kernel<T, MODE, MODE == AE_MPM_MODE_REFERENCE> : g2p_kernel<T, MODE, false>;
+    g2p<<<n_chunks_, chunk_threads_, g2p_smem, stream_>>>(w, counters_ + 2, write_keys ? 1 : 0);
     ++launches_;
     mark(5);  // the G2P kernel alone ends here
     if (MODE == AE_MPM_MODE_PHYSICS && has_snow_) {
