@@ -3939,7 +3939,7 @@ class World final : public WorldBase {
         substep_ += period;
         left -= period;
       } else {
-        substep_eager();
+        substep_eager(left == 1);
         --left;
       }
     }
@@ -4668,11 +4668,11 @@ class World final : public WorldBase {
     sorted_ = true;
   }
 
-  void substep_eager() {
+  void substep_eager(bool last = false) {
     // the keys of the next sort are written by the G2P just before it; a sort without them (first
     // substep, changed interval) computes them first.  Only the fused G2P counts cells too.
     const uint32_t next = phase_ + 1 >= sort_interval() ? 0u : phase_ + 1;
-    const bool write_keys = next == 0 && (!dense_sort_ || fused() || opts_.deterministic);
+    const bool write_keys = next == 0 && (!dense_sort_ || fused() || opts_.deterministic || !last);
     if (n_chunks_ > 0) {
       mark(0);
       const bool sort_now = phase_ == 0 && !sorted_;
