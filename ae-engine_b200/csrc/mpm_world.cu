@@ -65,9 +65,11 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
 // A work counter that an earlier kernel wrote and that no thread of this kernel changes, read by
-// every thread: through the read-only cache, so each SM fetches it once.  (A volatile or L2-only
-// load would send every warp of the grid to the same L2 slice before any of them could start.)
-__device__ __forceinline__ uint32_t launch_count(const uint32_t* p) { return __ldg(p); }
+// every thread: an ordinary load, which each SM's L1 serves after the first.  (A volatile or L2-only
+// load would send every warp of the grid to the same L2 slice before any of them could start.  The
+// read-only path is for data that does not change while the kernel runs, and a kernel launched
+// dependently runs before its predecessor has written.)
+__device__ __forceinline__ uint32_t launch_count(const uint32_t* p) { return *p; }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
