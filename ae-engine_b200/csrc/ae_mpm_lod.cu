@@ -19,6 +19,8 @@
 #include <algorithm>
 #include <cmath>
 
+#include "device_util.cuh"
+
 namespace aemp {
 
 namespace {
@@ -31,15 +33,6 @@ __device__ __forceinline__ int64_t as_isize(float v) {  // Rust `f32 as isize`
   if (v >= 9.2233720368547758e18f) return INT64_MAX;
   if (v <= -9.2233720368547758e18f) return INT64_MIN;
   return static_cast<int64_t>(v);
-}
-
-__device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  return x;
 }
 
 // class of particle idx: 0 near, 1 mid, 2 far, 3 skipped (inactive); simulation.rs:499-513
@@ -56,29 +49,37 @@ struct PosClass {
   }
 };
 
-// near candidate k of *n: 0 kept, 1 culled to mid; all kept when they do not exceed the cap
+// near candidate k: 0 kept, 1 culled to mid
 struct KeepClass {
   const uint64_t* near;
-  const uint8_t* keep;
-  const uint32_t* n;
-  uint32_t cap;
+  const uint8_t* keep;  // null: none is kept
   __device__ __forceinline__ int operator()(uint64_t k, uint64_t& item, float& d2) const {
     item = near[k];
     d2 = 0.0f;
-    return *n <= cap || (cap && keep[k]) ? 0 : 1;
+    return keep && keep[k] ? 0 : 1;
   }
 };
 
-// The item count of a partition is `n`, or *n_dev where an earlier kernel found it (CTAs past it
-// leave at once).
-__device__ __forceinline__ uint64_t part_items(uint64_t n, const uint32_t* n_dev) { return n_dev ? *n_dev : n; }
+// The items of a partition: n, or *n_dev where an earlier kernel found it, none of them up to `cap`
+// (the near candidates are where they belong then).  CTAs without items leave at once.
+struct Items {
+  uint64_t n;
+  const uint32_t* n_dev;
+  uint32_t cap;
+  __device__ __forceinline__ uint64_t count() const {
+    if (!n_dev) return n;
+    const uint32_t v = *n_dev;
+    return v > cap ? v : 0u;
+  }
+};
 
 template <class Cls>
-__global__ void __launch_bounds__(kPT) part_count(Cls cls, uint64_t n_items, const uint32_t* n_dev, uint32_t* tile_counts,
-                                                  uint32_t tiles) {
+__global__ void __launch_bounds__(kPT) part_count(Cls cls, Items items, uint32_t* tile_counts, uint32_t tiles) {
   __shared__ uint32_t wc[kPWarps][3];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t n = part_items(n_items, n_dev);
+  let_next_start();
+  dependency_wait();
+  const uint64_t n = items.count();
   if (uint64_t(blockIdx.x) * kPTile >= n) return;
   const uint64_t base = uint64_t(blockIdx.x) * kPTile + uint64_t(w) * (32 * kPItems);
   uint32_t c0 = 0, c1 = 0, c2 = 0;
@@ -112,11 +113,13 @@ __global__ void __launch_bounds__(kPT) part_count(Cls cls, uint64_t n_items, con
 
 // one block: exclusive scan of the three classes' tile counts together, and the class totals
 __global__ void __launch_bounds__(1024) part_scan(const uint32_t* tile_counts, uint32_t* tile_offs, uint32_t tiles,
-                                                  uint64_t n_items, const uint32_t* n_dev, uint32_t* totals) {
+                                                  Items items, uint32_t* totals) {
   __shared__ uint32_t ws[3][32];
   __shared__ uint32_t carry[3];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const uint32_t used = uint32_t((part_items(n_items, n_dev) + kPTile - 1) / kPTile);
+  let_next_start();
+  dependency_wait();
+  const uint32_t used = uint32_t((items.count() + kPTile - 1) / kPTile);
   if (tid < 3) carry[tid] = 0;
   __syncthreads();
   for (uint32_t start = 0; start < used; start += 1024) {
@@ -150,15 +153,16 @@ __global__ void __launch_bounds__(1024) part_scan(const uint32_t* tile_counts, u
 }
 
 // writes each item at its class's tile offset + rank in index order; class 1 lands at *out1_from +
-// position, class 0 optionally also writes its squared distance
+// position, class 0 optionally to a second list too, and its squared distance
 template <class Cls>
-__global__ void __launch_bounds__(kPT) part_scatter(Cls cls, uint64_t n_items, const uint32_t* n_dev,
-                                                    const uint32_t* tile_offs, uint32_t tiles, uint64_t* out0,
-                                                    float* d2_0, uint64_t* out1, const uint32_t* out1_from,
-                                                    uint64_t* out2) {
+__global__ void __launch_bounds__(kPT) part_scatter(Cls cls, Items items, const uint32_t* tile_offs,
+                                                    uint32_t tiles, uint64_t* out0, uint64_t* out0_again, float* d2_0,
+                                                    uint64_t* out1, const uint32_t* out1_from, uint64_t* out2) {
   __shared__ uint32_t wc[kPWarps][3];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t n = part_items(n_items, n_dev);
+  let_next_start();
+  dependency_wait();
+  const uint64_t n = items.count();
   if (uint64_t(blockIdx.x) * kPTile >= n) return;
   const uint64_t out1_base = out1_from ? *out1_from : 0;
   const uint64_t base = uint64_t(blockIdx.x) * kPTile + uint64_t(w) * (32 * kPItems);
@@ -200,6 +204,7 @@ __global__ void __launch_bounds__(kPT) part_scatter(Cls cls, uint64_t n_items, c
     if (k[r] == 0) {
       const uint32_t p = wb[0] + __popc(m0 & lt);
       out0[p] = item[r];
+      if (out0_again) out0_again[p] = item[r];
       if (d2_0) d2_0[p] = d2[r];
     } else if (k[r] == 1) {
       out1[out1_base + wb[1] + __popc(m1 & lt)] = item[r];
@@ -225,6 +230,8 @@ constexpr int kSelectBits = 11, kSelectBins = 1 << kSelectBits;
 __global__ void __launch_bounds__(1024) select_keep(const uint32_t* gkeys, const uint32_t* n_dev, uint32_t k,
                                                     uint8_t* keep) {
   extern __shared__ uint32_t skeys[];  // kSelectSmemKeys keys
+  let_next_start();
+  dependency_wait();
   const uint32_t n = *n_dev;
   if (n <= k) return;
   __shared__ uint32_t hist[kSelectBins];
@@ -593,26 +600,33 @@ cudaError_t LodWork::classify(const float* pos, const uint8_t* active, uint64_t 
   const uint32_t tiles = uint32_t((count + kPTile - 1) / kPTile);
   // squared distances as the reference computes them (simulation.rs:484-485)
   const PosClass pc{pos, active, player[0], player[1], player[2], near_dist * near_dist, mid_dist * mid_dist};
-  part_count<PosClass><<<tiles, kPT, 0, s>>>(pc, count, nullptr, tile_counts_, tiles);
-  part_scan<<<1, 1024, 0, s>>>(tile_counts_, tile_offs_, tiles, count, nullptr, totals_);
-  part_scatter<PosClass><<<tiles, kPT, 0, s>>>(pc, count, nullptr, tile_offs_, tiles, near_tmp_,
-                                               reinterpret_cast<float*>(near_key_), mid_out, nullptr, far_out);
+  // Each kernel after the first is launched dependently and waits for the one before it: the kernels are
+  // short, up to seven in a row.
+  const Items all{count, nullptr, 0u};
+  part_count<PosClass><<<tiles, kPT, 0, s>>>(pc, all, tile_counts_, tiles);
+  LOD_TRY(launch_after(true, part_scan, 1, 1024, 0, s, tile_counts_, tile_offs_, tiles, all, totals_));
+  LOD_TRY(launch_after(true, part_scatter<PosClass>, tiles, kPT, 0, s, pc, all, tile_offs_, tiles, near_out, near_tmp_,
+                       reinterpret_cast<float*>(near_key_), mid_out, nullptr, far_out));
   // cap (simulation.rs:519-530): the max_near smallest squared distances stay near, ties by index.
-  // The number of candidates stays on the device: the host waits once, for the final counts.
+  // The number of candidates stays on the device: the host waits once, for the final counts, and the
+  // kernels of the cap leave at once where the candidates do not exceed it (3 000 particles, 100 near ones
+  // under a cap of 1 000: 37 us, 53 with the kernels launched one after another and working through them).
   const uint32_t cap = uint32_t(std::min<uint64_t>(max_near, 0xffffffffu));
-  if (cap && cap < count) {
+  if (cap < count) {
     if (!select_smem_set_) {
       LOD_TRY(cudaFuncSetAttribute(select_keep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(sizeof(uint32_t) * kSelectSmemKeys)));
       select_smem_set_ = true;
     }
-    select_keep<<<1, 1024, sizeof(uint32_t) * kSelectSmemKeys, s>>>(near_key_, totals_, cap, keep_);
+    if (cap) LOD_TRY(launch_after(true, select_keep, 1, 1024, sizeof(uint32_t) * kSelectSmemKeys, s, near_key_, totals_, cap,
+                                  keep_));
+    const KeepClass kc{near_tmp_, cap ? keep_ : nullptr};
+    const Items near{0, totals_, cap};
+    LOD_TRY(launch_after(true, part_count<KeepClass>, tiles, kPT, 0, s, kc, near, tile_counts_, tiles));
+    LOD_TRY(launch_after(true, part_scan, 1, 1024, 0, s, tile_counts_, tile_offs_, tiles, near, totals_ + 4));
+    LOD_TRY(launch_after(true, part_scatter<KeepClass>, tiles, kPT, 0, s, kc, near, tile_offs_, tiles, near_out, nullptr,
+                         nullptr, mid_out, totals_ + 1, nullptr));
   }
-  const KeepClass kc{near_tmp_, keep_, totals_, cap};
-  part_count<KeepClass><<<tiles, kPT, 0, s>>>(kc, 0, totals_, tile_counts_, tiles);
-  part_scan<<<1, 1024, 0, s>>>(tile_counts_, tile_offs_, tiles, 0, totals_, totals_ + 4);
-  part_scatter<KeepClass><<<tiles, kPT, 0, s>>>(kc, 0, totals_, tile_offs_, tiles, near_out, static_cast<float*>(nullptr),
-                                                mid_out, totals_ + 1, static_cast<uint64_t*>(nullptr));
   LOD_TRY(cudaGetLastError());
   uint32_t tot[3] = {0, 0, 0};
   LOD_TRY(cudaMemcpyAsync(tot, totals_, sizeof(tot), cudaMemcpyDeviceToHost, s));

@@ -20,6 +20,7 @@
 #include <cstring>
 #include <memory>
 
+#include "device_util.cuh"
 #include "mpm_world.cuh"
 
 namespace aemp {
@@ -79,12 +80,6 @@ __device__ __forceinline__ void cp_async_v4(V4* sdst, const V4* gsrc) {
   for (int k = 0; k < int(sizeof(V4) / 16); ++k)
     cp_async16(reinterpret_cast<char*>(sdst) + 16 * k, reinterpret_cast<const char*>(gsrc) + 16 * k);
 }
-
-// Programmatic dependent launch: a kernel launched with launch_dependent may start while the kernel
-// before it drains, and waits here until that one has finished and its writes are visible.  Without
-// the launch attribute both are no-ops.
-__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 template <class T>
 __device__ __forceinline__ int floor_to_int(T v) {
@@ -2298,15 +2293,6 @@ __global__ void discard_scatter_kernel(typename V4T<T>::type* acc, uint32_t* blk
     if (threadIdx.x < 64) acc[uint64_t(gb) * 64u + threadIdx.x] = mk4(T(0), T(0), T(0), T(0));
     if (threadIdx.x == 0) blk_flag[gb] = 0u;
   }
-}
-
-__device__ __forceinline__ uint32_t warp_scan_incl(uint32_t x, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  return x;
 }
 
 // dense grouping (bin_scan_kernel): nodes per scan CTA
@@ -4588,17 +4574,8 @@ class World final : public WorldBase {
   // others: early CTAs crowd on the first free SMs, 9.3 -> 18 us for 128 CTAs.)
   template <class... P, class... A>
   void launch_dependent(void (*kernel)(P...), unsigned ctas, unsigned threads, size_t smem, A&&... args) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(ctas);
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = stream_;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &at;
-    c.numAttrs = total_cap_ <= uint64_t(device_sm_count()) * 1024 ? 1 : 0;
-    cudaLaunchKernelEx(&c, kernel, P(args)...);
+    launch_after(total_cap_ <= uint64_t(device_sm_count()) * 1024, kernel, ctas, threads, smem, stream_,
+                 std::forward<A>(args)...);
     ++launches_;
   }
 
