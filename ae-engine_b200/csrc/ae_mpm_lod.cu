@@ -459,16 +459,17 @@ __device__ __forceinline__ uint8_t phase_hop(uint16_t m, uint8_t cur, float t) {
 // reflecting world bounds (mpss.rs:449-476), temperature clamp (:479-497), phase transitions with
 // up to 3 hops (:500-548), in that order; passes selects them (1, 2, 4).  Each CTA adds its
 // transitions with one atomic: one per warp, 31 000 on one address, took longer
-// than the passes (1 M particles, most of them in transition: 30 -> 14.6 us).
+// than the passes (1 M particles, most of them in transition: 30 -> 14.6 us).  As many CTAs as run at
+// once: with a CTA of its own for every 512 particles the bounds or the clamp alone took 53.7 and 44.7 us
+// for 8 M particles, 37.8 and 31.0 so (all three passes 79.2 -> 67.1).
 __global__ void housekeeping_kernel(float* pos, float* vel, float* temp, uint8_t* phase, const uint16_t* mat,
                                     const uint8_t* active, uint64_t n, float x0, float y0, float z0, float x1, float y1,
                                     float z1, float tmin, float tmax, uint32_t passes, uint32_t* transitions) {
   // a particle's inputs are all loaded before anything is decided, the velocity components once the
   // bounds are known: two memory latencies per particle instead of one per component and pass
   const float lo[3] = {x0, y0, z0}, hi[3] = {x1, y1, z1};
-  const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  bool changed = false;
-  if (i < n) {
+  uint32_t changed = 0;
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
     const bool on = !active || active[i];
     float p[3] = {0.0f, 0.0f, 0.0f}, v[3] = {0.0f, 0.0f, 0.0f}, t = 0.0f;
     uint16_t m = 0;
@@ -514,13 +515,19 @@ __global__ void housekeeping_kernel(float* pos, float* vel, float* temp, uint8_t
         }
         if (next != cur) {
           phase[i] = next;
-          changed = true;
+          ++changed;
         }
       }
     }
   }
-  const int c = __syncthreads_count(changed);
-  if (threadIdx.x == 0 && c) atomicAdd(transitions, uint32_t(c));
+  if (!(passes & 4u)) return;
+  __shared__ uint32_t sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
+  changed = __reduce_add_sync(0xffffffffu, changed);
+  if ((threadIdx.x & 31) == 0 && changed) atomicAdd(&sum, changed);
+  __syncthreads();
+  if (threadIdx.x == 0 && sum) atomicAdd(transitions, sum);
 }
 
 inline unsigned grid_for(uint64_t n, int threads) {
@@ -645,7 +652,7 @@ cudaError_t LodWork::housekeeping(float* pos, float* vel, float* temp, uint8_t* 
   if (n == 0) return cudaSuccess;
   LOD_TRY(grow(1, 0));
   LOD_TRY(cudaMemsetAsync(totals_ + 3, 0, sizeof(uint32_t), s));
-  housekeeping_kernel<<<unsigned((n + 511) / 512), 512, 0, s>>>(pos, vel, temp, phase, material, active, n, bmin[0],
+  housekeeping_kernel<<<std::min(grid_for(n, 256), 148u * 8u), 256, 0, s>>>(pos, vel, temp, phase, material, active, n, bmin[0],
                                                                bmin[1], bmin[2], bmax[0], bmax[1], bmax[2], min_temp,
                                                                max_temp, passes, totals_ + 3);
   LOD_TRY(cudaGetLastError());
