@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(1024) part_scan(const uint32_t* tile_counts, u
 }
 
 // writes each item at its class's tile offset + rank in index order; class 1 lands at *out1_from +
-// position, class 0 optionally to a second list too, and its squared distance
+// position.  The first cap0 items of class 0 go to out0 (nothing is written past them), all of them
+// optionally to a second list, with their squared distances to a third
 template <class Cls>
 __global__ void __launch_bounds__(kPT) part_scatter(Cls cls, Items items, const uint32_t* tile_offs,
-                                                    uint32_t tiles, uint64_t* out0, uint64_t* out0_again, float* d2_0,
+                                                    uint32_t tiles, uint64_t* out0, uint64_t* all0, uint32_t cap0, float* d2_0,
                                                     uint64_t* out1, const uint32_t* out1_from, uint64_t* out2) {
   __shared__ uint32_t wc[kPWarps][3];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -203,8 +204,8 @@ __global__ void __launch_bounds__(kPT) part_scatter(Cls cls, Items items, const 
     const uint32_t m2 = __ballot_sync(0xffffffffu, k[r] == 2);
     if (k[r] == 0) {
       const uint32_t p = wb[0] + __popc(m0 & lt);
-      out0[p] = item[r];
-      if (out0_again) out0_again[p] = item[r];
+      if (p < cap0) out0[p] = item[r];
+      if (all0) all0[p] = item[r];
       if (d2_0) d2_0[p] = d2[r];
     } else if (k[r] == 1) {
       out1[out1_base + wb[1] + __popc(m1 & lt)] = item[r];
@@ -610,15 +611,15 @@ cudaError_t LodWork::classify(const float* pos, const uint8_t* active, uint64_t 
   // Each kernel after the first is launched dependently and waits for the one before it: the kernels are
   // short, up to seven in a row.
   const Items all{count, nullptr, 0u};
+  const uint32_t cap = uint32_t(std::min<uint64_t>(max_near, 0xffffffffu));
   part_count<PosClass><<<tiles, kPT, 0, s>>>(pc, all, tile_counts_, tiles);
   LOD_TRY(launch_after(true, part_scan, 1, 1024, 0, s, tile_counts_, tile_offs_, tiles, all, totals_));
   LOD_TRY(launch_after(true, part_scatter<PosClass>, tiles, kPT, 0, s, pc, all, tile_offs_, tiles, near_out, near_tmp_,
-                       reinterpret_cast<float*>(near_key_), mid_out, nullptr, far_out));
+                       cap, reinterpret_cast<float*>(near_key_), mid_out, nullptr, far_out));
   // cap (simulation.rs:519-530): the max_near smallest squared distances stay near, ties by index.
   // The number of candidates stays on the device: the host waits once, for the final counts, and the
   // kernels of the cap leave at once where the candidates do not exceed it (3 000 particles, 100 near ones
   // under a cap of 1 000: 37 us, 53 with the kernels launched one after another and working through them).
-  const uint32_t cap = uint32_t(std::min<uint64_t>(max_near, 0xffffffffu));
   if (cap < count) {
     if (!select_smem_set_) {
       LOD_TRY(cudaFuncSetAttribute(select_keep, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -632,7 +633,7 @@ cudaError_t LodWork::classify(const float* pos, const uint8_t* active, uint64_t 
     LOD_TRY(launch_after(true, part_count<KeepClass>, tiles, kPT, 0, s, kc, near, tile_counts_, tiles));
     LOD_TRY(launch_after(true, part_scan, 1, 1024, 0, s, tile_counts_, tile_offs_, tiles, near, totals_ + 4));
     LOD_TRY(launch_after(true, part_scatter<KeepClass>, tiles, kPT, 0, s, kc, near, tile_offs_, tiles, near_out, nullptr,
-                         nullptr, mid_out, totals_ + 1, nullptr));
+                         cap, nullptr, mid_out, totals_ + 1, nullptr));
   }
   LOD_TRY(cudaGetLastError());
   uint32_t tot[3] = {0, 0, 0};

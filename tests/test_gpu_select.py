@@ -39,3 +39,30 @@ def test_near_cap_keeps_the_closest_and_ties_by_index(ctx, n, cap, spread):
     assert np.array_equal(gn, keep)
     assert np.array_equal(gm, np.setdiff1d(np.arange(n), keep))
     assert np.array_equal(np.sort(d2[gn]), np.sort(d2[rn])) and gm.size == rm.size
+
+
+@pytest.mark.parametrize("n,near,cap", [(3000, 100, 1000), (3000, 100, 100), (3000, 2500, 100), (5000, 4000, 0),
+                                        (5000, 4000, 5000), (100000, 60000, 59999)])
+def test_lists_in_device_memory_are_written_up_to_their_counts(ctx, n, near, cap):
+    import ctypes as C
+
+    import torch
+
+    rng = np.random.default_rng(n + cap)
+    pos = rng.uniform(200, 300, (n, 3)).astype(f32)
+    pos[rng.choice(n, near, replace=False)] = rng.uniform(-20, 20, (near, 3))
+    player = np.zeros(3, f32)
+    want = O.lod_classify(pos, None, player, 50.0, 400.0, cap)
+    dpos = torch.from_numpy(pos).cuda()
+    lists = [torch.full((n,), -7, dtype=torch.int64, device="cuda") for _ in range(3)]
+    counts = [C.c_uint64() for _ in range(3)]
+    torch.cuda.synchronize()
+    ctx.check(ctx.lib.ae_mpm_lod_classify(ctx.h, dpos.data_ptr(), None, n, player.ctypes.data, 50.0, 400.0, cap,
+                                          lists[0].data_ptr(), C.byref(counts[0]), lists[1].data_ptr(), C.byref(counts[1]),
+                                          lists[2].data_ptr(), C.byref(counts[2])))
+    for k, (got, c) in enumerate(zip(lists, counts)):
+        a = got.cpu().numpy()
+        ref = np.asarray(want[k]).astype(np.int64)
+        assert c.value == ref.size
+        assert np.array_equal(np.sort(a[:c.value]), np.sort(ref)), k  # the oracle's culled tail has its own order
+        assert (a[c.value:] == -7).all(), k
