@@ -308,3 +308,26 @@ def test_graphs_carry_the_sort_of_their_period(ctx, mode, deterministic, interva
     names = [e.name for e in prof.events()]
     assert sum("GraphLaunch" in n for n in names) == 48 // (interval if interval % 2 == 0 else 2 * interval)
     assert sum("LaunchKernel" in n for n in names) == 0
+
+
+@pytest.mark.parametrize("mode", [M.MODE_PHYSICS, M.MODE_REFERENCE])
+def test_deterministic_world_on_a_huge_grid_repeats_and_matches(ctx, mode):
+    # 8.5 M nodes and more for a few thousand particles: the radix-sorted sums, one thread per cell,
+    # with crowded cells and (reference mode) particles off the grid
+    sc, p = crowd(4000, 216, 700, 11)
+    sc.mode, sc.max_particles = mode, p.n + 5
+    if mode == M.MODE_REFERENCE:
+        p.pos[::50, 1] += 1.0
+    runs = []
+    for det in (1, 1, 0):
+        w = M.World(ctx, [sc, sc], M.exec_opts(deterministic=det))
+        w.upload(0, p)
+        w.upload(1, p)
+        w.step(6)
+        w.sync(raise_on_error=False)
+        runs.append((w.download(0, p.n), w.download(1, p.n)))
+        w.close()
+    for f in ("pos", "vel", "F", "J", "C"):
+        assert np.array_equal(getattr(runs[0][0], f), getattr(runs[1][0], f)), f
+        assert np.array_equal(getattr(runs[0][0], f), getattr(runs[0][1], f)), f
+    assert rel(runs[0][0].pos, runs[2][0].pos) <= 1e-6

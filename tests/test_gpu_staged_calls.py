@@ -62,3 +62,22 @@ def test_staged_lists_match_the_oracle_and_leave_the_rest(ctx, full, n, pick):
         assert np.array_equal(getattr(a, f)[rest], getattr(p, f)[rest]), f
         if f in ("mass", "mat") or (not full and f not in ("pos", "vel")):
             assert np.array_equal(getattr(a, f), getattr(p, f)), f
+
+
+@pytest.mark.parametrize("pick", ["sparse", "all"])
+@pytest.mark.parametrize("n", [FULL + 1, 40001, 150001])
+def test_staged_reference_calls_bring_the_affine_matrix_back(ctx, n, pick):
+    # C is one of the two largest arrays on the way back, cut over several pieces.  It is a velocity
+    # gradient: sums of some 30 f32 terms at 4e-6 of the node velocity, times 6 / dx, against a largest
+    # entry of about one node velocity over dx, so 1e-4 of it; a row out of place differs by its size
+    capacity = n if pick == "all" else 2 * n + 77
+    p, grid, cfg = buffer(capacity, n)
+    rng = np.random.default_rng(n + 2)
+    idx = (np.arange(n) if pick == "all" else np.sort(rng.choice(capacity, n, replace=False))).astype(np.uint64)
+    mats = [M.material(young_modulus=1e3, poisson_ratio=0.25, density=1000.0)]
+    a, b = p.copy(), p.copy()
+    ctx.step_parallel_with_grid(a, grid, cfg, mats, [M.NEO_HOOKEAN], 0.004, idx)
+    assert O.step_parallel_with_grid(b, grid, cfg, mats, [M.NEO_HOOKEAN], 0.004, idx) == 0
+    sel = idx.astype(np.int64)
+    assert rel(a.C, b.C) <= 1e-4
+    assert (np.abs(b.C[sel] - p.C[sel]).max(1) > 0).all() and (np.abs(a.C[sel] - p.C[sel]).max(1) > 0).all()
