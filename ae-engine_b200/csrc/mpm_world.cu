@@ -2094,7 +2094,8 @@ __device__ __noinline__ bool snow_return_parked(const MatDev* md, bool redo, T* 
 // Yielding snow particles of a warp from which on the fused kernel maps them back itself.  Where they
 // come in whole warps this saves the clamp kernel's pass over them (512 scenes: fused + clamp 846 + 401 ->
 // 1077 + 25 us; 8.4 M dam break from a yielding start 734 + 134 -> 827 + 23).  The call costs a world with
-// snow 2 % of the kernel while nothing yields (dam break 711 -> 727 us).  The mapping behind the scatter,
+// snow 2 % of the kernel while nothing yields (dam break 711 -> 727 us; 9.4 -> 10.0 us for 2 000 to 20 000
+// particles).  The mapping behind the scatter,
 // as a function or as a second turn of a loop around it, cost more in both states (752 / 837 us).
 constexpr int kInlineClamp = 8;
 
